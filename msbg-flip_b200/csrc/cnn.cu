@@ -3,18 +3,17 @@
 // memory), weight gradients, loss, Adam and the C ABI of include/msbg_cnn.h.
 // No counterpart in the reference.
 //
-// Convolution as an implicit GEMM.  One CTA holds a tile's input (16^3 cells
-// plus a 1-cell halo, 16 channels) in shared memory as two channel halves,
-// each a [z][y][x] array of 18^3 cells x 16 bytes (8 bf16 channels).  An
-// M = 128 block of output cells is 8 consecutive x by the 16 y rows of one z
-// plane; its A operand for kernel tap (kz, ky, kx) is the same array read
-// from a start address shifted by the tap: 8 rows (x) of 16 bytes form a
-// core matrix, the 16 y rows are core-matrix groups 18 cells apart (SBO) and
-// the two channel halves are the two K halves (LBO).  So every tap is one
-// tcgen05.mma of M = 128, N = 16, K = 16 straight from the activations, with
-// no im2col copy; 27 taps accumulate in tensor memory.  While the epilogue
-// of plane z reads its accumulators, the MMAs of plane z+1 run into the
-// other half of a 64-column tensor-memory allocation.
+// Convolution as an implicit GEMM.  A layer's input is up to 18 padded z planes
+// of two channel halves, each an [y][x] array of 18^2 cells x 16 bytes (8 bf16
+// channels), in shared memory.  An M = 128 block of output cells is 8
+// consecutive x by the 16 y rows of one z plane; its A operand for the
+// in-plane tap (ky, kx) is the input plane read from a start address shifted by
+// the tap: 8 rows (x) of 16 bytes form a core matrix, the 16 y rows are
+// core-matrix groups 18 cells apart (SBO) and the two channel halves are the
+// two K halves (LBO).  An input plane contributes to three output planes, one
+// per kz: their accumulators sit side by side in tensor memory, so one
+// tcgen05.mma of M = 128, N = 48 (3 planes x 16 channels), K = 16 serves the
+// three kz of a tap straight from the activations, with no im2col copy.
 //
 // Backward: the data gradient of a "same" convolution is a "same"
 // convolution of the output gradient with the flipped, transposed kernel, so
@@ -31,6 +30,7 @@
 #include <cstring>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cnn.cuh"
@@ -44,16 +44,19 @@ namespace cnn {
 // ---------------------------------------------------------------------------
 // weight images
 // ---------------------------------------------------------------------------
-// Image element (tap, n, k) of the B operand (N x K, K-major, no swizzle):
-// tap*256 + (k>>3)*128 + n*8 + (k&7).  Forward: n = cout, k = cin, W[n][k][tap].
-// Backward-data: n = cin, k = cout, W[k][n][26 - tap].  Unused rows/columns
-// (cin = 4 of layer 1, cout = 1 of layer 4) are zero.
+// One B operand (N x K, K-major, no swizzle) per in-plane tap q = 3 ky + kx: its
+// 48 rows are the 16 channels n of kz = 2, 1, 0 (the order of the output planes
+// an input plane reaches).  Image element (q, kz, n, k):
+// q*768 + (k>>3)*384 + ((2-kz)*16 + n)*8 + (k&7).  Forward: n = cout, k = cin,
+// W[n][k][tap].  Backward-data: n = cin, k = cout, W[k][n][26 - tap].  Unused
+// rows/columns (cin = 4 of layer 1, cout = 1 of layer 4) are zero.
 __global__ void k_pack(const float* __restrict__ w, __nv_bfloat16* __restrict__ fwd,
                        __nv_bfloat16* __restrict__ bwd) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NLAYER * WIMG) return;
   const int l = i / WIMG, e = i % WIMG;
-  const int tap = e / 256, r = e % 256, kh = r / 128, n = (r % 128) / 8, k = kh * 8 + (r % 8);
+  const int r = e % 768, row = (r % 384) / 8, n = row % 16, k = (r / 384) * 8 + (r % 8);
+  const int tap = (2 - row / 16) * 9 + e / 768;
   const int cin = layer_cin(l), cout = layer_cout(l);
   const float* W = w + layer_off(l);
   float f = 0.f, b = 0.f;
@@ -63,125 +66,267 @@ __global__ void k_pack(const float* __restrict__ w, __nv_bfloat16* __restrict__ 
   bwd[i] = __float2bfloat16_rn(b);
 }
 
-// ---------------------------------------------------------------------------
-// layout conversion
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// feat [n][4][NPAD] FP32 planes -> padded bf16 layout (half 0: the 4
-// features and 4 zero channels; half 1: zeros).  One thread per padded cell.
-__global__ void k_feat_pack(int n, const float* __restrict__ feat, uint4* __restrict__ x) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)n * NPAD) return;
-  const int64_t t = i / NPAD;
-  const int c = (int)(i % NPAD);
-  const float* f = feat + t * NFEAT * NPAD;
-  uint4 v;
-  v.x = pack_bf2(f[c], f[NPAD + c]);
-  v.y = pack_bf2(f[2 * NPAD + c], f[3 * NPAD + c]);
-  v.z = 0u;
-  v.w = 0u;
-  x[(t * 2) * NPAD + c] = v;
-  x[(t * 2 + 1) * NPAD + c] = make_uint4(0, 0, 0, 0);
-}
-
 // ---------------------------------------------------------------------------
 // convolution (tcgen05)
 // ---------------------------------------------------------------------------
-// One CTA of 256 threads per SM walks its tiles.  A tile's input (padded
-// layout) arrives by two bulk copies of one channel half each.  Thread 0
-// issues the 54 MMAs of plane z+1 (into the other TMEM column set) before
-// everyone drains plane z: warp w reads TMEM lanes 32*(w%4).. of column half
-// w/4 (the x half of the plane), applies the epilogue and writes the cells.
-// The next tile's copies are issued as soon as the last plane's MMAs are
-// done, so they overlap the last epilogue.  A tcgen05.mma of N = 16 costs
-// about 45 cycles whatever its operands (measured), so 864 MMAs bound a tile
-// to ~20 us per layer.  Every wait is bounded.
-template <int EPI>
-__global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3_tc(ConvArgs a) {
+// A chain of up to 4 layers per tile, one CTA per SM walking its tiles; the
+// activations of the layers in between never leave the SM.
+//   * An input plane is read by MMAs once, for all three output planes that it
+//     reaches, so output plane z takes the place of input plane z in `act` (16
+//     planes, halo cells zero; the zero planes beyond both ends are not multiplied).
+//     The first layer's planes have halos of their own and arrive in a ring.
+//   * Warps 17-20 fill the ring, plane by plane: FP32 features packed to bf16, or
+//     a bf16 gradient.  Channels 8-15 of either are zero: one zero plane stands
+//     for that half of every ring plane.
+//   * Warp 16 issues the MMAs, per plane 10 for each x half (tap 0 in two parts,
+//     since it starts an output plane while it adds to two others), and the copies
+//     of the weight images, one layer ahead.  The accumulators of the 16 output
+//     planes x 2 x halves take the whole tensor memory (512 columns).
+//   * Warps 0-7 drain the even planes z, 8-15 the odd ones, once input plane z + 1
+//     is done: warp w reads TMEM lanes 32*(w%4).. of x half w/4 % 2, applies the
+//     epilogue and writes the cells.  (8 warps for all planes took longer per
+//     plane than its MMAs: 60 us per tile.)
+// A tcgen05.mma of this shape costs about 45 cycles for every N <= 64 (measured; the
+// A operand's 4 KB alone are 32 cycles of shared-memory reads), so the 27 taps cost
+// 10 instead of 27 instructions per plane and x half, with the products added in
+// the same order (kz, ky, kx): the same bits.  That bounds a tile to 30 us for 4
+// layers; measured 56 us.  Forward pass of 4096 tiles on a B200: 3.40 ms with a launch
+// per layer, N = 16 and the activations through global memory, 1.54 ms now.  (An MMA
+// issued by a divergent thread costs over 100 cycles, its operands moving to uniform
+// registers one by one: 2.43 ms.)  Every wait is bounded.
+__global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3_tc(const __grid_constant__ ConvChain a) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  uint8_t* act = sm;
-  uint8_t* wts = sm + 2 * HALF_BYTES;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * HALF_BYTES + WIMG * 2);  // [0,1] MMA, [2] input
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 3);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint8_t* act = sm;                                   // [TS] planes of both halves
+  uint8_t* wts = act + TS * 2 * PLANE_BYTES;           // [2] weight images
+  uint8_t* ring = wts + 2 * WIMG * 2;                  // [CONV_SLOTS] planes of half 0, a zero plane
+  uint64_t* done = reinterpret_cast<uint64_t*>(ring + (CONV_SLOTS + 1) * PLANE_BYTES);
+  // done[PD]: the plane's MMAs are complete (each used one once per pass); stored[TS]:
+  // output plane drained, and in act; full, taken [CONV_SLOTS]: ring; wfull[2]
+  uint64_t* stored = done + PD;
+  uint64_t* full = stored + TS;
+  uint64_t* taken = full + CONV_SLOTS;
+  uint64_t* wfull = taken + CONV_SLOTS;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(wfull + 2);
+  volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform
   const int G = gridDim.x;
   if ((int)blockIdx.x >= a.n) return;
 
-  for (int i = tid; i < WIMG * 2 / 16; i += CONV_THREADS)
-    reinterpret_cast<uint4*>(wts)[i] = reinterpret_cast<const uint4*>(a.wimg)[i];
+  for (int i = tid; i < (int)(TS * 2 * PLANE_BYTES / 16); i += CONV_THREADS)
+    reinterpret_cast<uint4*>(act)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < PLANE; i += CONV_THREADS)
+    reinterpret_cast<uint4*>(ring + CONV_SLOTS * PLANE_BYTES)[i] = make_uint4(0, 0, 0, 0);
   if (tid == 0) {
-    for (int b = 0; b < 3; b++) mbar_init(&bar[b], 1);
+    for (int b = 0; b < PD; b++) mbar_init(&done[b], 1);
+    for (int b = 0; b < TS; b++) mbar_init(&stored[b], 8);
+    for (int b = 0; b < 2 * CONV_SLOTS + 2; b++) mbar_init(&full[b], 1);
     fence_mbar_init();
+    *abort = 0;
   }
   if (warp == 0) {
-    tmem_alloc(tslot, 64);
+    tmem_alloc(tslot, 512);
     tmem_relinquish();
   }
-  fence_proxy_async();  // the weight image (generic writes) -> tensor core
+  fence_proxy_async();  // the zeros (generic writes) -> tensor core
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *tslot;
-  const uint32_t idesc = idesc_bf16_f32(128, 16);
-  const uint64_t a0 = smem_desc(smem_addr(act), HALF_BYTES, PD * 16);
-  const uint64_t b0 = smem_desc(smem_addr(wts), 256, 128);
-  auto load_tile = [&](int t) {
-    mbar_expect_tx(&bar[2], 2 * HALF_BYTES);
-    bulk_g2s(act, a.in + (size_t)t * 2 * NPAD, HALF_BYTES, &bar[2]);
-    bulk_g2s(act + HALF_BYTES, a.in + ((size_t)t * 2 + 1) * NPAD, HALF_BYTES, &bar[2]);
-  };
-  // Descriptors are built once; the start address field (address / 16) is the
-  // low bits: one cell = 16 bytes = +1, and no start reaches 2^14 * 16 bytes.
-  auto issue = [&](int z) {
-    tc_fence_after();
-    const uint32_t cb = tbase + (uint32_t)((z & 1) * 32);
-    const uint64_t az = a0 + (uint64_t)(z * PLANE);
-#pragma unroll
-    for (int tap = 0; tap < 27; tap++)
-#pragma unroll
-      for (int xh = 0; xh < 2; xh++) {
-        const int kz = tap / 9, ky = (tap / 3) % 3, kx = tap % 3;
-        mma_bf16(cb + 16 * xh, az + (uint64_t)((kz * PD + ky) * PD + 8 * xh + kx),
-                 b0 + (uint64_t)(tap * 32), idesc, tap > 0 ? 1u : 0u);
+  const int nTiles = (a.n - (int)blockIdx.x + G - 1) / G;
+  const int passes = nTiles * a.nl;  // pass p: layer p % nl of this CTA's tile p / nl
+
+  if (warp == EPI_WARPS) {
+    // the whole warp runs this loop on uniform values (an MMA takes its operands
+    // from uniform registers); one lane issues
+    const uint32_t zero = smem_addr(ring) + CONV_SLOTS * PLANE_BYTES;
+    const uint64_t a0 = smem_desc(smem_addr(act), PLANE_BYTES, PD * 16);
+    const uint64_t b0 = smem_desc(smem_addr(wts), 768, 128);
+    auto wait = [&](uint64_t* b, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait_abort(b, parity, abort));
+    };
+    auto load_weights = [&](int p, int l) {
+      if (elect_one()) {
+        mbar_expect_tx(&wfull[p & 1], WIMG * 2);
+        bulk_g2s(wts + (p & 1) * (WIMG * 2), a.L[l].wimg, WIMG * 2, &wfull[p & 1]);
       }
-    mma_commit(&bar[z & 1]);
-  };
-  if (tid == 0) load_tile(blockIdx.x);
-  const int xh = warp >> 2, quarter = warp & 3;
-  const int r = 32 * quarter + lane;
-  const int x = 8 * xh + (r & 7), y = r >> 3;
-  bool ok = true;
-  for (int j = 0, t = blockIdx.x; t < a.n && ok; j++, t += G) {
-    if (!__syncthreads_and(mbar_wait(&bar[2], (uint32_t)(j & 1)))) {
-      ok = false;
-      break;
+    };
+    int wl = 0, wlL = 0;  // weight images asked for, the next one's layer
+    for (; wl < 2 && wl < passes; wl++) {
+      load_weights(wl, wlL);
+      wlL = wlL + 1 == a.nl ? 0 : wlL + 1;
     }
-    if (tid == 0) issue(0);
-    const float s = (EPI == EPI_OUT0 && a.outScale) ? a.outScale[t] : 1.f;
-    const int64_t base = (EPI == EPI_OUT0) ? (a.outOff ? a.outOff[t] : (int64_t)t * NCELL) : 0;
-    for (int z = 0; z < TS; z++) {
-      if (tid == 0 && z + 1 < TS) issue(z + 1);
-      if (!__syncthreads_and(mbar_wait(&bar[z & 1], (uint32_t)((z >> 1) & 1)))) {
-        ok = false;
+    int slot = 0;          // ring plane
+    uint32_t slotPar = 0;  // and the parity of its fill
+    // what plane zi of pass p (layer l) waits for: its weights and its input, and
+    // that the last pass has drained the accumulators of the output plane that it
+    // starts (stored implies drained; input plane zi >= 1 of a later layer is
+    // stored[zi - 1], waited for one plane before)
+    auto ready = [&](int p, int l, int zi) -> bool {
+      const uint32_t before = (uint32_t)((p - 1) & 1);
+      bool ok = true;
+      if (zi == (l > 0)) {
+        ok = wait(&wfull[p & 1], (uint32_t)((p >> 1) & 1));
+        if (ok && l > 0) ok = wait(&stored[0], before);
+      }
+      if (ok && p > 0 && zi < TS) ok = wait(&stored[zi], before);
+      if (ok && l == 0) ok = wait(&full[slot], slotPar);
+      return ok;
+    };
+    int p = 0, zi = 0, l = 0;
+    bool ok = ready(0, 0, 0);
+    while (ok) {
+      tc_fence_after();
+      // output planes reached lo..hi, of which nOld started before
+      const int lo = max(zi - 2, 0), hi = min(zi, TS - 1);
+      const int nOld = l > 0 && zi == 1 ? 0 : min(zi, TS) - lo;
+      const int first = lo + nOld;
+      const int row0 = 16 * (lo - (zi - 2));  // first row of B used
+      const uint32_t one = 1u << 18;          // 16 more columns
+      const uint32_t idAll = idesc_bf16_f32(128, 16) + (uint32_t)(hi - lo) * one;
+      const uint32_t idOld = idesc_bf16_f32(128, 16) + (uint32_t)(nOld - 1) * one;
+      const uint32_t idNew = idesc_bf16_f32(128, 16) + (uint32_t)(hi - first) * one;
+      const uint32_t at = smem_addr(ring) + slot * PLANE_BYTES;
+      const uint64_t az = l > 0 ? a0 + (uint64_t)((zi - 1) * (int)(2 * PLANE_BYTES / 16))
+                                : smem_desc(at, zero - at, PD * 16);
+      const uint64_t bz = b0 + (uint64_t)((p & 1) * (WIMG * 2 / 16) + row0);
+      const uint32_t c = tbase + (uint32_t)(16 * lo);
+      // (the x halves alternate: neighbouring MMAs add to different accumulators)
+      auto taps = [&](auto t0, auto t1) {
+#pragma unroll
+        for (int t = decltype(t0)::value; t < decltype(t1)::value; t++)
+#pragma unroll
+          for (int xh = 0; xh < 2; xh++)
+            mma_bf16(c + (uint32_t)(256 * xh), az + (uint64_t)((t / 3) * PD + 8 * xh + t % 3),
+                     bz + (uint64_t)(t * 96), idAll, 1u);
+      };
+      if (elect_one()) {
+#pragma unroll
+        for (int xh = 0; xh < 2; xh++)
+          if (nOld > 0)
+            mma_bf16(c + (uint32_t)(256 * xh), az + (uint64_t)(8 * xh), bz, idOld, 1u);
+#pragma unroll
+        for (int xh = 0; xh < 2; xh++)
+          if (first <= hi)
+            mma_bf16(c + (uint32_t)(256 * xh + 16 * nOld), az + (uint64_t)(8 * xh),
+                     bz + (uint64_t)(16 * nOld), idNew, 0u);
+        taps(std::integral_constant<int, 1>{}, std::integral_constant<int, 5>{});
+      }
+      __syncwarp();
+      // the next plane's waits, while these MMAs run
+      const int pz = zi, pl = l, pslot = slot;
+      if (l == 0 && ++slot == CONV_SLOTS) {
+        slot = 0;
+        slotPar ^= 1u;
+      }
+      // the previous pass is done with its weights: those of the next one
+      if (zi == 6 && p > 0 && wl < passes) {
+        if (!(ok = wait(&done[PD - 1], (uint32_t)((p - 1) & 1)))) break;
+        load_weights(wl++, wlL);
+        wlL = wlL + 1 == a.nl ? 0 : wlL + 1;
+      }
+      if (++zi > (l > 0 ? TS : TS + 1)) {
+        p++;
+        l = l + 1 == a.nl ? 0 : l + 1;
+        zi = l > 0;
+      }
+      const bool more = p < passes;
+      if (more && !(ok = ready(p, l, zi))) break;
+      if (elect_one()) {
+        taps(std::integral_constant<int, 5>{}, std::integral_constant<int, 9>{});
+        if (pz > 1) mma_commit(&done[pz]);  // (no output plane completes before)
+        if (pl > 0 && pz == TS) mma_commit(&done[PD - 1]);  // (its last plane is zero)
+        if (pl == 0) mma_commit(&taken[pslot]);
+      }
+      __syncwarp();
+      if (!more) break;
+    }
+    if (!ok) {
+      // a wait gave up: flag it, give the work in flight one more bounded wait
+      *abort = 1;
+      if (lane == 0) atomicExch(a.err, 1);
+      if (elect_one()) mma_commit(&done[0]);  // (nothing else waits on done[0])
+      __syncwarp();
+      mbar_wait(&done[0], 0);
+      for (int w = p; w < wl; w++)
+        mbar_wait(&wfull[w & 1], (uint32_t)((w >> 1) & 1));
+    }
+  } else if (warp > EPI_WARPS) {
+    // every fourth ring plane: loaded into registers before the slot
+    // is free
+    constexpr int PER = (PLANE + 31) / 32;
+    const int total = nTiles * PD;
+    for (int q = warp - EPI_WARPS - 1; q < total; q += CONV_THREADS / 32 - EPI_WARPS - 1) {
+      const size_t t = blockIdx.x + (size_t)(q / PD) * G;
+      const int zi = q % PD, slot = q % CONV_SLOTS, use = q / CONV_SLOTS;
+      uint4 v[PER];
+      if (a.feat) {
+        const float* f = a.feat + t * NFEAT * NPAD + zi * PLANE;
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+          const int c = min(lane + 32 * i, PLANE - 1);
+          v[i] = make_uint4(pack_bf2(f[c], f[NPAD + c]), pack_bf2(f[2 * NPAD + c], f[3 * NPAD + c]),
+                            0u, 0u);
+        }
+      } else {
+        const uint4* f = a.in + t * 2 * NPAD + zi * PLANE;
+#pragma unroll
+        for (int i = 0; i < PER; i++) v[i] = f[min(lane + 32 * i, PLANE - 1)];
+      }
+      if (use && !mbar_wait_abort(&taken[slot], (uint32_t)((use - 1) & 1), abort)) {
+        *abort = 1;
+        if (lane == 0) atomicExch(a.err, 1);
         break;
       }
-      // the tile's MMAs are all done: its input buffer takes the next tile
-      if (z == TS - 1 && tid == 0 && t + G < a.n) load_tile(t + G);
-      tc_fence_after();
-      float v[16];
-      tmem_ld16(tbase + ((uint32_t)(32 * quarter) << 16) + (uint32_t)((z & 1) * 32 + 16 * xh), v);
-      const int cell = x + TS * (y + TS * z);
-      if (EPI == EPI_OUT0) {
-        a.out0[base + cell] = v[0] * s;
-      } else {
-        const size_t pc = (size_t)pad_index(cell);
-        const size_t o0 = ((size_t)t * 2) * NPAD + pc, o1 = o0 + NPAD;
-        if (EPI == EPI_MASK) {
-          uint4 m2[2] = {a.mask[o0], a.mask[o1]};
+      uint4* d = reinterpret_cast<uint4*>(ring + slot * PLANE_BYTES);
+#pragma unroll
+      for (int i = 0; i < PER; i++)
+        if (lane + 32 * i < PLANE) {
+          d[lane + 32 * i] = v[i];
+          if (a.x0) a.x0[t * 2 * NPAD + zi * PLANE + lane + 32 * i] = v[i];
+        }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[slot]);
+    }
+  } else {
+    const int xh = (warp >> 2) & 1, quarter = warp & 3;
+    const int r = 32 * quarter + lane;
+    const int x = 8 * xh + (r & 7), y = r >> 3;
+    bool ok = true;
+    for (int p = 0; p < passes && ok; p++) {
+      const ConvLayer& Ly = a.L[p % a.nl];
+      const bool last = p % a.nl == a.nl - 1;
+      const size_t t = blockIdx.x + (size_t)(p / a.nl) * G;
+      const int epi = Ly.epi;
+      const float s = epi == EPI_OUT0 && a.outScale ? a.outScale[t] : 1.f;
+      const int64_t base = epi == EPI_OUT0 ? (a.outOff ? a.outOff[t] : (int64_t)t * NCELL) : 0;
+      uint4* out = Ly.out ? Ly.out + t * 2 * NPAD : nullptr;
+      const uint4* mask = epi == EPI_MASK ? Ly.mask + t * 2 * NPAD : nullptr;
+      for (int z = warp >> 3; z < TS; z += EPI_WARPS / 8) {
+        const int cell = x + TS * (y + TS * z), pc = pad_index(cell);
+        uint4 m2[2];
+        if (epi == EPI_MASK) {  // in flight while the MMAs finish
+          m2[0] = mask[pc];
+          m2[1] = mask[NPAD + pc];
+        }
+        if (!(ok = mbar_wait_abort(&done[z + 2], (uint32_t)(p & 1), abort))) break;
+        tc_fence_after();
+        float v[16];
+        tmem_ld16(tbase + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(256 * xh + 16 * z), v);
+        tc_fence_before();
+        if (epi == EPI_OUT0) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&stored[z]);  // drained
+          a.out0[base + cell] = v[0] * s;
+          continue;
+        }
+        if (epi == EPI_MASK) {
           const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(m2);
 #pragma unroll
           for (int c = 0; c < 16; c++)
@@ -199,24 +344,29 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3_tc(ConvArgs a) {
         q1.y = pack_bf2(v[10], v[11]);
         q1.z = pack_bf2(v[12], v[13]);
         q1.w = pack_bf2(v[14], v[15]);
-        a.out[o0] = q0;
-        a.out[o1] = q1;
+        if (!last) {
+          uint4* d = reinterpret_cast<uint4*>(act + z * 2 * PLANE_BYTES) + (x + 1) + PD * (y + 1);
+          d[0] = q0;
+          d[PLANE] = q1;
+          fence_proxy_async();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&stored[z]);
+        if (out) {
+          out[pc] = q0;
+          out[NPAD + pc] = q1;
+        }
       }
-      tc_fence_before();
-      __syncthreads();
     }
-  }
-  if (!ok && tid == 0) {
-    // a wait gave up: flag it, give the work in flight one more bounded wait
-    atomicExch(a.err, 1);
-    mbar_wait(&bar[0], 0);
-    mbar_wait(&bar[1], 0);
-    mbar_wait(&bar[2], 0);
+    if (!ok) {
+      *abort = 1;
+      if (lane == 0) atomicExch(a.err, 1);
+    }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_dealloc(tbase, 64);
+  if (warp == 0) tmem_dealloc(tbase, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -353,8 +503,7 @@ struct msbg_cnn {
   DeviceBuffer err;              // int
   int step = 0;
   int numSMs = 148;
-  // training scratch for `cap` tiles
-  int cap = 0;
+  // activations and gradients of the largest batch so far
   DeviceBuffer x0, a1, a2, a3, y, dy, dz3, dz2, dz1, part, lossPart;  // padded layout
 };
 
@@ -381,49 +530,39 @@ int cnn_error(msbg_cnn* n, int code, const char* fmt, ...) {
 void set_attrs() {
   static bool done = false;
   if (done) return;
-  cudaFuncSetAttribute(k_conv3_tc<EPI_RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
-  cudaFuncSetAttribute(k_conv3_tc<EPI_MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
-  cudaFuncSetAttribute(k_conv3_tc<EPI_OUT0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
+  cudaFuncSetAttribute(k_conv3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
   cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
   done = true;
 }
 
-template <int EPI>
-void conv(msbg_cnn* net, int layer, bool backward, int n, const uint4* in, uint4* out,
-          const uint4* mask, float* out0, const int64_t* outOff, const float* outScale,
-          cudaStream_t st) {
-  ConvArgs a;
+const __nv_bfloat16* image(msbg_cnn* net, int layer, bool backward) {
+  return (backward ? net->imgB : net->imgF).as<__nv_bfloat16>() + (size_t)layer * WIMG;
+}
+
+void conv(msbg_cnn* net, ConvChain& a, int n, cudaStream_t st) {
   a.n = n;
-  a.in = in;
-  a.wimg = (backward ? net->imgB : net->imgF).as<__nv_bfloat16>() + (size_t)layer * WIMG;
-  a.out = out;
-  a.mask = mask;
-  a.out0 = out0;
-  a.outOff = outOff;
-  a.outScale = outScale;
   a.err = net->err.as<int>();
-  const int grid = std::min(n, net->numSMs);
-  k_conv3_tc<EPI><<<grid, CONV_THREADS, CONV_SMEM, st>>>(a);
+  k_conv3_tc<<<std::min(n, net->numSMs), CONV_THREADS, CONV_SMEM, st>>>(a);
 }
 
-void feat_pack(int n, const float* feat, uint4* x0, cudaStream_t st) {
-  const int64_t cnt = (int64_t)n * NPAD;
-  k_feat_pack<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(n, feat, x0);
+// Activations of n tiles, zeroed when allocated (the halos stay zero).
+int ensure_act(msbg_cnn* net, DeviceBuffer& b, int n) {
+  const size_t bytes = (size_t)n * ACT_BYTES;
+  if (b.p && b.bytes >= bytes) return MSBG_OK;
+  CNN_TRY(net, b.ensure(bytes));
+  CNN_TRY(net, cudaMemsetAsync(b.p, 0, bytes, net->stream));
+  return MSBG_OK;
 }
 
-int ensure_cap(msbg_cnn* net, int n) {
-  if (n <= net->cap) return MSBG_OK;
-  const size_t act = (size_t)n * ACT_BYTES;
-  DeviceBuffer* bufs[] = {&net->x0, &net->a1, &net->a2, &net->a3,
-                          &net->dz3, &net->dz2, &net->dz1, &net->dy};
-  for (DeviceBuffer* b : bufs) {
-    CNN_TRY(net, b->ensure(act));
-    CNN_TRY(net, cudaMemsetAsync(b->p, 0, act, net->stream));  // zero halos
+int ensure_train(msbg_cnn* net, int n) {
+  for (DeviceBuffer* b : {&net->x0, &net->a1, &net->a2, &net->a3, &net->dz3, &net->dz2, &net->dz1,
+                          &net->dy}) {
+    int rc = ensure_act(net, *b, n);
+    if (rc) return rc;
   }
   CNN_TRY(net, net->y.ensure((size_t)n * NCELL * sizeof(float)));
   CNN_TRY(net, net->part.ensure((size_t)net->numSMs * NC * NC * 27 * sizeof(float)));
   CNN_TRY(net, net->lossPart.ensure(LOSS_GRID * sizeof(double)));
-  net->cap = n;
   return MSBG_OK;
 }
 
@@ -451,13 +590,17 @@ namespace msbg {
 namespace cnn {
 // Forward pass into out0 (see msbg_cnn_forward); used by the pressure solver.
 int forward(msbg_cnn* net, const float* feat, float* out0, const int64_t* outOff,
-            const float* outScale, int n, cudaStream_t st, uint4* x0, uint4* s1, uint4* s2) {
+            const float* outScale, int n, cudaStream_t st) {
   if (n <= 0) return MSBG_OK;
-  feat_pack(n, feat, x0, st);
-  conv<EPI_RELU>(net, 0, false, n, x0, s1, nullptr, nullptr, nullptr, nullptr, st);
-  conv<EPI_RELU>(net, 1, false, n, s1, s2, nullptr, nullptr, nullptr, nullptr, st);
-  conv<EPI_RELU>(net, 2, false, n, s2, s1, nullptr, nullptr, nullptr, nullptr, st);
-  conv<EPI_OUT0>(net, 3, false, n, s1, nullptr, nullptr, out0, outOff, outScale, st);
+  ConvChain a{};
+  a.nl = NLAYER;
+  a.feat = feat;
+  for (int l = 0; l < NLAYER; l++)
+    a.L[l] = ConvLayer{nullptr, nullptr, image(net, l, false), l < NLAYER - 1 ? EPI_RELU : EPI_OUT0};
+  a.out0 = out0;
+  a.outOff = outOff;
+  a.outScale = outScale;
+  conv(net, a, n, st);
   return cudaGetLastError() == cudaSuccess ? MSBG_OK : MSBG_ERROR;
 }
 
@@ -555,10 +698,7 @@ extern "C" int msbg_cnn_forward(msbg_cnn* net, const float* feat, float* out, in
   if (!net || n < 0 || (n > 0 && (!feat || !out))) return cnn_error(net, MSBG_EINVARG, "bad arguments");
   if (n == 0) return MSBG_OK;
   cudaSetDevice(net->device);
-  int rc = ensure_cap(net, n);
-  if (rc) return rc;
-  rc = forward(net, feat, out, nullptr, nullptr, n, net->stream, net->x0.as<uint4>(),
-               net->a1.as<uint4>(), net->a2.as<uint4>());
+  int rc = forward(net, feat, out, nullptr, nullptr, n, net->stream);
   if (rc) return cnn_error(net, rc, "forward launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   return check_err(net);
 }
@@ -571,7 +711,7 @@ extern "C" int msbg_cnn_loss_grad(msbg_cnn* net, const float* feat, const float*
   if (!net || n <= 0 || !feat || !target || !mask || !(count > 0))
     return cnn_error(net, MSBG_EINVARG, "bad arguments");
   cudaSetDevice(net->device);
-  int rc = ensure_cap(net, n);
+  int rc = ensure_train(net, n);
   if (rc) return rc;
   cudaStream_t st = net->stream;
   uint4* x0 = net->x0.as<uint4>();
@@ -584,18 +724,27 @@ extern "C" int msbg_cnn_loss_grad(msbg_cnn* net, const float* feat, const float*
   uint4* dz1 = net->dz1.as<uint4>();
   float* y = net->y.as<float>();
   // forward, keeping the activations
-  feat_pack(n, feat, x0, st);
-  conv<EPI_RELU>(net, 0, false, n, x0, a1, nullptr, nullptr, nullptr, nullptr, st);
-  conv<EPI_RELU>(net, 1, false, n, a1, a2, nullptr, nullptr, nullptr, nullptr, st);
-  conv<EPI_RELU>(net, 2, false, n, a2, a3, nullptr, nullptr, nullptr, nullptr, st);
-  conv<EPI_OUT0>(net, 3, false, n, a3, nullptr, nullptr, y, nullptr, nullptr, st);
+  ConvChain f{};
+  f.nl = NLAYER;
+  f.feat = feat;
+  f.x0 = x0;
+  f.L[0] = ConvLayer{a1, nullptr, image(net, 0, false), EPI_RELU};
+  f.L[1] = ConvLayer{a2, nullptr, image(net, 1, false), EPI_RELU};
+  f.L[2] = ConvLayer{a3, nullptr, image(net, 2, false), EPI_RELU};
+  f.L[3] = ConvLayer{nullptr, nullptr, image(net, 3, false), EPI_OUT0};
+  f.out0 = y;
+  conv(net, f, n, st);
   // loss and dL/dy
   k_loss<<<LOSS_GRID, 512, 0, st>>>((int64_t)n * NCELL, y, target, mask, (float)(1.0 / count),
                                     reinterpret_cast<__nv_bfloat16*>(dy), net->lossPart.as<double>());
   // backward-data through layers 4, 3, 2 (ReLU masks of their inputs)
-  conv<EPI_MASK>(net, 3, true, n, dy, dz3, a3, nullptr, nullptr, nullptr, st);
-  conv<EPI_MASK>(net, 2, true, n, dz3, dz2, a2, nullptr, nullptr, nullptr, st);
-  conv<EPI_MASK>(net, 1, true, n, dz2, dz1, a1, nullptr, nullptr, nullptr, st);
+  ConvChain d{};
+  d.nl = 3;
+  d.in = dy;
+  d.L[0] = ConvLayer{dz3, a3, image(net, 3, true), EPI_MASK};
+  d.L[1] = ConvLayer{dz2, a2, image(net, 2, true), EPI_MASK};
+  d.L[2] = ConvLayer{dz1, a1, image(net, 1, true), EPI_MASK};
+  conv(net, d, n, st);
   // weight gradients
   const int grid = std::min(n, net->numSMs);
   float* part = net->part.as<float>();

@@ -53,27 +53,42 @@ __host__ __device__ constexpr int pad_index(int cell) {
 
 enum { EPI_RELU = 0, EPI_MASK = 1, EPI_OUT0 = 2 };
 
-struct ConvArgs {
-  int n;                              // tiles
-  const uint4* in;                    // [n][2][NPAD] 16-byte cells (padded layout)
-  const __nv_bfloat16* wimg;          // [27][2][16][8] bf16 image of the layer
-  uint4* out;                         // EPI_RELU / EPI_MASK: padded layout, interior written
-  const uint4* mask;                  // EPI_MASK: padded layout; out = acc where mask > 0
+// One layer of a chain.  out: padded layout in global memory, interior written
+// (null: not kept); mask (EPI_MASK): padded layout, out = acc where mask > 0.
+struct ConvLayer {
+  uint4* out;
+  const uint4* mask;
+  const __nv_bfloat16* wimg;          // [9][2][48][8] bf16 image of the layer
+  int epi;
+};
+struct ConvChain {
+  int n, nl;                          // tiles, layers
+  // the first layer's input: FP32 features [n][4][NPAD] (packed into half 0 of x0
+  // too, if given), or half 0 of a padded layout
+  const float* feat;
+  const uint4* in;
+  uint4* x0;
+  ConvLayer L[NLAYER];
   float* out0;                        // EPI_OUT0: channel 0
   const int64_t* outOff;              // EPI_OUT0: per-tile first cell in out0 (null: t*NCELL)
   const float* outScale;              // EPI_OUT0: per-tile factor (null: 1)
   int* err;                           // set when a bounded wait gives up
 };
 
-// 8 warps: warp w drains TMEM lanes 32*(w%4) of column half w/4.
-constexpr int CONV_THREADS = 256;
-constexpr size_t CONV_SMEM = 2 * (size_t)HALF_BYTES + WIMG * 2 + 256;
+// 16 epilogue warps, one that issues MMAs, 4 that fill the ring.  Shared memory:
+// 16 planes of activations (166 KB), two weight images (28 KB), the ring (36 KB).
+constexpr int EPI_WARPS = 16;
+constexpr int CONV_THREADS = (EPI_WARPS + 5) * 32;
+constexpr int CONV_SLOTS = 6;
+constexpr size_t CONV_SMEM = TS * 2 * (size_t)PLANE_BYTES + 2 * WIMG * 2 +
+                             (CONV_SLOTS + 1) * (size_t)PLANE_BYTES +
+                             (PD + TS + 2 * CONV_SLOTS + 2) * 8 + 16;
+static_assert(CONV_SMEM <= 227 * 1024, "one CTA's shared memory");
 
 // Inference of n tiles on stream st: out0[outOff[t] + cell] = outScale[t] *
-// net(feat[t]) (cnn.cu).  x0, s1, s2: scratch of n * ACT_BYTES each; s1 and
-// s2 must have zero halos (zeroed once when allocated).
+// net(feat[t]) (cnn.cu).
 int forward(msbg_cnn* net, const float* feat, float* out0, const int64_t* outOff,
-            const float* outScale, int n, cudaStream_t st, uint4* x0, uint4* s1, uint4* s2);
+            const float* outScale, int n, cudaStream_t st);
 // Status of the network's bounded waits since the last call (0 = none gave up); clears it.
 int take_error(msbg_cnn* net, cudaStream_t st);
 

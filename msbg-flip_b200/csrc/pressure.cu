@@ -587,10 +587,6 @@ int learned_predict(msbg_gpu_ctx* ctx, Solver& S, msbg_cnn* net, cudaStream_t st
     MSBG_CUDA_TRY(ctx, S.cFeat.ensure(sizeof(float) * CH * cnn::NFEAT * cnn::NPAD));
     MSBG_CUDA_TRY(ctx, S.cScale.ensure(sizeof(float) * CH));
     MSBG_CUDA_TRY(ctx, S.cOff.ensure(sizeof(int64_t) * CH));
-    for (DeviceBuffer* b : {&S.cX0, &S.cS1, &S.cS2}) {
-      MSBG_CUDA_TRY(ctx, b->ensure(cnn::ACT_BYTES * CH));
-      MSBG_CUDA_TRY(ctx, cudaMemsetAsync(b->p, 0, cnn::ACT_BYTES * CH, st));  // zero halos
-    }
     S.cnnChunk = CH;
   }
   for (int c0 = 0; c0 < S.nCnnTiles; c0 += CH) {
@@ -600,9 +596,9 @@ int learned_predict(msbg_gpu_ctx* ctx, Solver& S, msbg_cnn* net, cudaStream_t st
         S.cnnLevel.as<int>() + c0, S.levelNorm, val, nullptr, S.cFeat.as<float>(),
         S.cScale.as<float>(), S.cOff.as<int64_t>(), nullptr, nullptr);
     if (cnn::forward(net, S.cFeat.as<float>(), out, S.cOff.as<int64_t>(), S.cScale.as<float>(),
-                     cnt, st, S.cX0.as<uint4>(), S.cS1.as<uint4>(), S.cS2.as<uint4>()))
+                     cnt, st))
       return set_error(ctx, MSBG_ERROR, "learned network launch failed");
-    launches += 6;
+    launches += 2;
   }
   if (inGraph) return MSBG_OK;  // no host sync inside a capture; checked after the solve
   MSBG_CUDA_TRY(ctx, cudaGetLastError());

@@ -53,7 +53,7 @@ struct Solver {
   int nCnnTiles = 0;
   float levelNorm = 0.f;
   DeviceBuffer cnnTiles, cnnLevel;          // [nCnnTiles] tile id, resolution level
-  DeviceBuffer cFeat, cScale, cOff, cX0, cS1, cS2, guess, cIdx;
+  DeviceBuffer cFeat, cScale, cOff, guess, cIdx;
   std::vector<int> cnnTilesHost, cnnLevelHost;
   int cnnChunk = 0;
   bool haveX64 = false;  // x64 holds the solution of the last refined solve

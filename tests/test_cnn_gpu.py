@@ -93,3 +93,19 @@ def test_forward_is_deterministic():
     b = net.forward(to_dev(feat)).cpu().numpy()
     np.testing.assert_array_equal(a, b)
     net.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 149, 300])
+def test_forward_same_bits_in_any_batch(n):
+    """A tile's result does not depend on its place in a batch: fewer tiles than SMs, and CTAs
+    with 2 and 3 tiles one after the other."""
+    import torch
+    rng = np.random.default_rng(7)
+    net = msbg_gpu.Cnn(0)
+    feat = torch.from_numpy(rng.standard_normal((3, 4 * 18 ** 3)).astype(np.float32)).cuda()
+    alone = torch.cat([net.forward(feat[i:i + 1].contiguous()) for i in range(3)])
+    idx = torch.arange(n, device="cuda") % 3
+    out = net.forward(feat[idx].contiguous())
+    net.close()
+    assert torch.equal(out, alone[idx])
