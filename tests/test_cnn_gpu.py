@@ -109,3 +109,35 @@ def test_forward_same_bits_in_any_batch(n):
     out = net.forward(feat[idx].contiguous())
     net.close()
     assert torch.equal(out, alone[idx])
+
+
+@pytest.mark.parametrize("n", [1, 5, 40])
+def test_batch_gradient_is_the_sum_of_the_tiles(n):
+    """Weight gradients over more and fewer slabs than CTAs: the batch's gradient against the
+    tiles' own at the same count.  Each is an FP32 sum of exact products in at most 16-term
+    steps, so both sides are within 1e-5 of the sum of the tiles' norms."""
+    w, feat, tgt, mask = case(11, n)
+    net = msbg_gpu.Cnn(0)
+    net.set_weights(w)
+    f, t, m = to_dev(feat), to_dev(tgt), to_dev(mask)
+    _, g = net.loss_grad(f, t, m, count=1000.0, want_grad=True)
+    each = [net.loss_grad(f[i:i + 1].contiguous(), t[i:i + 1].contiguous(),
+                          m[i:i + 1].contiguous(), count=1000.0, want_grad=True)[1]
+            for i in range(n)]
+    net.close()
+    ref = np.sum([e.astype(np.float64) for e in each], axis=0)
+    assert np.linalg.norm(g - ref) <= 1e-5 * sum(np.linalg.norm(e) for e in each)
+
+
+def test_a_tile_outside_the_mask_adds_nothing():
+    """Cells with a zero gradient take no part, whatever their features hold."""
+    w, feat, tgt, mask = case(12, 2)
+    feat[0, 0, 3:9] = np.nan
+    mask[0] = 0
+    net = msbg_gpu.Cnn(0)
+    net.set_weights(w)
+    _, g = net.loss_grad(to_dev(feat), to_dev(tgt), to_dev(mask), count=1000.0, want_grad=True)
+    _, e = net.loss_grad(to_dev(feat[1:]), to_dev(tgt[1:]), to_dev(mask[1:]), count=1000.0,
+                         want_grad=True)
+    net.close()
+    assert np.linalg.norm(g - e) <= 1e-5 * np.linalg.norm(e)
