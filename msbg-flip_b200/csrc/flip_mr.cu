@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -33,6 +34,8 @@
 namespace msbg {
 namespace {
 
+#include "particle_bins.cuh"
+
 // The reference's transition width: MultiresSparseGrid::create fixes
 // _dTransRes at 6 whatever it is passed (src/msbg.cpp:198-201, 290).
 constexpr int kDTransRes = 6;
@@ -42,7 +45,9 @@ struct MrState {
   std::vector<int> levels;
   int64_t n = 0;  // packed voxels
   bool distBuilt = false;
-  DeviceBuffer level, off, fc, kind, dist, vel, velOld, parts;
+  DeviceBuffer level, off, fc, kind, dist, parts;
+  DeviceBuffer vel;      // [3n] (vel, velOld) side by side: a gather reads both in one load
+  DeviceBuffer scratch;  // one channel on its way in or out; the visiting order of G2P
   DeviceBuffer dsOffA, dsOffB, dsFlags, dsSrc, dsDst;  // downsampleVelocity
 };
 
@@ -182,7 +187,7 @@ __global__ void __launch_bounds__(256) k_mr_dist(MrGrid g, const int8_t* __restr
 // (src/sbg.h:1386, 2936-2941, 3111-3420) on the distance channel of level
 // lv: cell-centred, the 2x2x2 window clamped to the grid, value blocks read
 // their data, full blocks dTransRes*1024, the others 0; p1*t + p0*(1-t)
-// along x, then y, then z.
+// along x, then y, then z.  A window inside one block asks for its kind once.
 __device__ __forceinline__ float dist_interp(const MrGrid& g, int lv, float px, float py,
                                              float pz) {
   const float x = __fsub_rn(px, 0.5f), y = __fsub_rn(py, 0.5f), z = __fsub_rn(pz, 0.5f);
@@ -190,51 +195,73 @@ __device__ __forceinline__ float dist_interp(const MrGrid& g, int lv, float px, 
   const float u = __fsub_rn(x, (float)ix), v = __fsub_rn(y, (float)iy),
               w = __fsub_rn(z, (float)iz);
   const int nx = g.sx >> lv, ny = g.sy >> lv, nz = g.sz >> lv, sh = g.sh0 - lv;
+  const int m = (1 << sh) - 1;
   const int64_t nb = (int64_t)g.nbx * g.nby * g.nbz;
   const float full = (float)(kDTransRes * 1024);
-  float bz2[2];
+  const int x0 = min(max(ix, 0), nx - 1), x1 = min(max(ix + 1, 0), nx - 1);
+  const int y0 = min(max(iy, 0), ny - 1), y1 = min(max(iy + 1, 0), ny - 1);
+  const int z0 = min(max(iz, 0), nz - 1), z1 = min(max(iz + 1, 0), nz - 1);
+  float c[8];
+  if ((((x0 ^ x1) | (y0 ^ y1) | (z0 ^ z1)) >> sh) == 0) {
+    const int64_t b = (x0 >> sh) + (int64_t)g.nbx * ((y0 >> sh) + (int64_t)g.nby * (z0 >> sh));
+    const int kd = g.kind[(int64_t)lv * nb + b];
+    const float f = kd == 2 ? full : 0.f;
+    const uint16_t* d = kd == 1 && g.level[b] == lv ? g.dist + g.off[b] : nullptr;
 #pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const int zz = min(max(iz + k, 0), nz - 1);
-    float by2[2];
+    for (int k = 0; k < 8; k++)
+      c[k] = d ? (float)d[((k & 1 ? x1 : x0) & m) + (((k & 2 ? y1 : y0) & m) << sh) +
+                          (((k & 4 ? z1 : z0) & m) << (2 * sh))]
+               : f;
+  } else {
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int yy = min(max(iy + j, 0), ny - 1);
-      float bx2[2];
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int xx = min(max(ix + i, 0), nx - 1);
-        const int64_t b = (xx >> sh) + (int64_t)g.nbx * ((yy >> sh) + (int64_t)g.nby * (zz >> sh));
-        const int kd = g.kind[(int64_t)lv * nb + b];
-        bx2[i] = kd == 1 ? (float)g.dist[g.idx(lv, xx, yy, zz)] : kd == 2 ? full : 0.f;
-      }
-      by2[j] = __fadd_rn(__fmul_rn(bx2[1], u), __fmul_rn(bx2[0], __fsub_rn(1.0f, u)));
+    for (int k = 0; k < 8; k++) {
+      const int xx = k & 1 ? x1 : x0, yy = k & 2 ? y1 : y0, zz = k & 4 ? z1 : z0;
+      const int64_t b = (xx >> sh) + (int64_t)g.nbx * ((yy >> sh) + (int64_t)g.nby * (zz >> sh));
+      const int kd = g.kind[(int64_t)lv * nb + b];
+      c[k] = kd == 1 ? (float)g.dist[g.idx(lv, xx, yy, zz)] : kd == 2 ? full : 0.f;
     }
-    bz2[k] = __fadd_rn(__fmul_rn(by2[1], v), __fmul_rn(by2[0], __fsub_rn(1.0f, v)));
   }
-  return __fadd_rn(__fmul_rn(bz2[1], w), __fmul_rn(bz2[0], __fsub_rn(1.0f, w)));
+  const float u1 = __fsub_rn(1.0f, u), v1 = __fsub_rn(1.0f, v), w1 = __fsub_rn(1.0f, w);
+  float e[4], f[2];
+#pragma unroll
+  for (int k = 0; k < 4; k++) e[k] = __fadd_rn(__fmul_rn(c[2 * k + 1], u), __fmul_rn(c[2 * k], u1));
+#pragma unroll
+  for (int k = 0; k < 2; k++) f[k] = __fadd_rn(__fmul_rn(e[2 * k + 1], v), __fmul_rn(e[2 * k], v1));
+  return __fadd_rn(__fmul_rn(f[1], w), __fmul_rn(f[0], w1));
 }
 
 __device__ __constant__ float kMrOff[3][3] = {{0.f, 0.5f, 0.5f}, {0.5f, 0.f, 0.5f},
                                               {0.5f, 0.5f, 0.f}};
 
 // Trilinear sums of component d in both channels at level lv, from the
-// sample origin (ix0, iy0, iz0) and fractions (fx, fy, fz).
-__device__ __forceinline__ void trilinear2(const MrGrid& g, int lv, const float* __restrict__ a,
-                                           const float* __restrict__ b, int d, int ix0, int iy0,
-                                           int iz0, float fx, float fy, float fz, float& sa,
-                                           float& sb) {
+// sample origin (ix0, iy0, iz0) and fractions (fx, fy, fz).  A window inside one
+// block asks for its level and offset once.
+__device__ __forceinline__ void trilinear2(const MrGrid& g, int lv,
+                                           const float2* __restrict__ vel, int d, int ix0, int iy0, int iz0, float fx, float fy, float fz,
+                                           float& sa, float& sb) {
   sa = 0.f;
   sb = 0.f;
+  const int sh = g.sh0 - lv, m = (1 << sh) - 1;
+  const bool in = ix0 >= 0 && iy0 >= 0 && iz0 >= 0 && ix0 < (g.sx >> lv) - 1 &&
+                  iy0 < (g.sy >> lv) - 1 && iz0 < (g.sz >> lv) - 1;
+  const bool one = in && (((ix0 ^ (ix0 + 1)) | (iy0 ^ (iy0 + 1)) | (iz0 ^ (iz0 + 1))) >> sh) == 0;
+  int64_t base = -1;
+  if (one) {
+    const int64_t b = (ix0 >> sh) + (int64_t)g.nbx * ((iy0 >> sh) + (int64_t)g.nby * (iz0 >> sh));
+    // in a block of another level every value reads 0, and so do the sums (+0)
+    if (g.level[b] != lv) return;
+    base = g.off[b] + (ix0 & m) + ((iy0 & m) << sh) + ((iz0 & m) << (2 * sh));
+  }
+  const float gx = __fsub_rn(1.f, fx), gy = __fsub_rn(1.f, fy), gz = __fsub_rn(1.f, fz);
 #pragma unroll
   for (int c = 0; c < 8; c++) {
     const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
-    const int64_t i = g.idx(lv, ix0 + dx, iy0 + dy, iz0 + dz);
-    const float va = i < 0 ? 0.f : a[3 * i + d], vb = i < 0 ? 0.f : b[3 * i + d];
-    const float w = __fmul_rn(__fmul_rn(dx ? fx : __fsub_rn(1.f, fx), dy ? fy : __fsub_rn(1.f, fy)),
-                              dz ? fz : __fsub_rn(1.f, fz));
-    sa = __fadd_rn(sa, __fmul_rn(w, va));
-    sb = __fadd_rn(sb, __fmul_rn(w, vb));
+    const int64_t i =
+        one ? base + dx + (dy << sh) + (dz << (2 * sh)) : g.idx(lv, ix0 + dx, iy0 + dy, iz0 + dz);
+    const float2 v = i < 0 ? make_float2(0.f, 0.f) : vel[3 * i + d];
+    const float w = __fmul_rn(__fmul_rn(dx ? fx : gx, dy ? fy : gy), dz ? fz : gz);
+    sa = __fadd_rn(sa, __fmul_rn(w, v.x));
+    sb = __fadd_rn(sb, __fmul_rn(w, v.y));
   }
 }
 
@@ -242,11 +269,18 @@ __device__ __forceinline__ void trilinear2(const MrGrid& g, int lv, const float*
 // same per component: its shared path, taken when the three staggered
 // samples share a block, computes exactly interpCompMSBG's expressions).
 // la, lb: MtLinstep's bounds as the reference forms them in float.
-__global__ void k_g2p_mr(msbg_flip_particle* __restrict__ p, int64_t np, MrGrid g,
-                         const float* __restrict__ vel, const float* __restrict__ velOld,
-                         float alpha, double la, double lb) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
-       k += (int64_t)gridDim.x * blockDim.x) {
+// Bound by the gather: 16 M particles in no order over 57 M voxels (512^3, 3 levels,
+// B200) took 9.8 ms as they came, every sector a miss; visited block by block, with the
+// channels side by side and one look-up per window inside a block, 3.8 ms, of which the
+// order takes 0.4.  The same bits.
+__global__ void __launch_bounds__(256) k_g2p_mr(msbg_flip_particle* __restrict__ p, int64_t np,
+                                                MrGrid g, const float2* __restrict__ vel,
+                                                BinsOrder order, float alpha, double la,
+                                                double lb) {
+  const int* perm = order.get();
+  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < np;
+       n += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = perm ? perm[n] : n;
     msbg_flip_particle q = p[k];
     const bool finite = isfinite(q.pos[0]) && isfinite(q.pos[1]) && isfinite(q.pos[2]);
 #pragma unroll
@@ -263,7 +297,7 @@ __global__ void k_g2p_mr(msbg_flip_particle* __restrict__ p, int64_t np, MrGrid 
         const int lv = g.level[(cx >> g.sh0) +
                                (int64_t)g.nbx * ((cy >> g.sh0) + (int64_t)g.nby * (cz >> g.sh0))];
         float fa, fb;
-        trilinear2(g, 0, vel, velOld, d, ix0, iy0, iz0, fx, fy, fz, fa, fb);
+        trilinear2(g, 0, vel, d, ix0, iy0, iz0, fx, fy, fz, fa, fb);
         if (lv == 0) {
           pic = fa;
           old = fb;
@@ -275,7 +309,7 @@ __global__ void k_g2p_mr(msbg_flip_particle* __restrict__ p, int64_t np, MrGrid 
           const float cfx = __fsub_rn(cgx, (float)cix0), cfy = __fsub_rn(cgy, (float)ciy0),
                       cfz = __fsub_rn(cgz, (float)ciz0);
           float ca, cb;
-          trilinear2(g, lv, vel, velOld, d, cix0, ciy0, ciz0, cfx, cfy, cfz, ca, cb);
+          trilinear2(g, lv, vel, d, cix0, ciy0, ciz0, cfx, cfy, cfz, ca, cb);
           const float dist = __fmul_rn(dist_interp(g, lv, cgx, cgy, cgz), 1.0f / 1024.0f);
           const double x = (double)dist;
           const float af = x < la ? 0.f : x >= lb ? 1.f : (float)((x - la) / (lb - la));
@@ -367,6 +401,23 @@ __global__ void __launch_bounds__(256)
 
 int grid_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 32); }
 
+// From how many particles on G2P orders them: below, the four launches cost more than
+// a gather out of order does.
+constexpr int64_t MR_BINS_MIN = 1 << 16;
+
+// One of the two interleaved channels: into it (get = 0) or out of it.
+__global__ void __launch_bounds__(256) k_mr_channel(float2* __restrict__ vel, int which,
+                                                    float* __restrict__ data, int64_t n, int get) {
+  float* v = reinterpret_cast<float*>(vel) + which;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    if (get)
+      data[i] = v[2 * i];
+    else
+      v[2 * i] = data[i];
+  }
+}
+
 // The state of a context for its current topology (rebuilt when it changed).
 // The reference asserts that 26-neighbour blocks differ by at most one level
 // (src/msbg.cpp:1718-1719); such a map is rejected here.
@@ -413,12 +464,10 @@ int mr_state(msbg_gpu_ctx* ctx, MrState** out, MrGrid& g) {
     MSBG_CUDA_TRY(ctx, s->fc.ensure(nb));
     MSBG_CUDA_TRY(ctx, s->kind.ensure((size_t)nb * ctx->nLevels));
     MSBG_CUDA_TRY(ctx, s->dist.ensure(2 * (size_t)o));
-    MSBG_CUDA_TRY(ctx, s->vel.ensure(12 * (size_t)o));
-    MSBG_CUDA_TRY(ctx, s->velOld.ensure(12 * (size_t)o));
+    MSBG_CUDA_TRY(ctx, s->vel.ensure(24 * (size_t)o));
     MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(s->level.p, lv8.data(), nb, cudaMemcpyHostToDevice, st));
     MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(s->off.p, off.data(), 8 * nb, cudaMemcpyHostToDevice, st));
     MSBG_CUDA_TRY(ctx, cudaMemsetAsync(s->vel.p, 0, s->vel.bytes, st));
-    MSBG_CUDA_TRY(ctx, cudaMemsetAsync(s->velOld.p, 0, s->velOld.bytes, st));
     // the host vectors are read by the copies above before they go out of scope
     MSBG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     sp = std::move(s);
@@ -491,16 +540,22 @@ extern "C" int msbg_gpu_flip_mr_channel(msbg_gpu_ctx* ctx, int which, float* dat
   MrGrid g;
   int rc = mr_state(ctx, &S, g);
   if (rc) return rc;
-  DeviceBuffer* b = which == MSBG_FLIP_VEL ? &S->vel : which == MSBG_FLIP_VEL_OLD ? &S->velOld
-                                                                                  : nullptr;
-  if (!b) return set_error(ctx, MSBG_EINVARG, "mixed-resolution channel %d unknown", which);
+  if (which != MSBG_FLIP_VEL && which != MSBG_FLIP_VEL_OLD)
+    return set_error(ctx, MSBG_EINVARG, "mixed-resolution channel %d unknown", which);
   if (n != 3 * S->n)
     return set_error(ctx, MSBG_EINVARG, "mixed-resolution channel holds %lld floats, not %lld",
                      (long long)(3 * S->n), (long long)n);
-  MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(get ? (void*)data : b->p, get ? b->p : (const void*)data,
-                                     sizeof(float) * n,
-                                     get ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
-                                     ctx->stream));
+  MSBG_CUDA_TRY(ctx, S->scratch.ensure(sizeof(float) * n));
+  const int w = which == MSBG_FLIP_VEL ? 0 : 1;
+  if (!get)
+    MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(S->scratch.p, data, sizeof(float) * n,
+                                       cudaMemcpyHostToDevice, ctx->stream));
+  k_mr_channel<<<grid_blocks(n), 256, 0, ctx->stream>>>(S->vel.as<float2>(), w,
+                                                        S->scratch.as<float>(), n, get);
+  MSBG_CUDA_TRY(ctx, cudaGetLastError());
+  if (get)
+    MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(data, S->scratch.p, sizeof(float) * n,
+                                       cudaMemcpyDeviceToHost, ctx->stream));
   return msbg_gpu_sync(ctx);
 }
 
@@ -528,8 +583,12 @@ int flip_g2p_mr(msbg_gpu_ctx* ctx, msbg_flip_particle* particles, int64_t np, fl
   // (src/flip_sim.cpp:1514-1521): stenWidth 2, MT_SQRT3F
   const float sqrt3 = 1.73205080756887f;
   const float la = (1.0f * sqrt3) * 1.01f, lb = (0.99f * ((float)kDTransRes + 2.f)) / sqrt3;
-  k_g2p_mr<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, S->vel.as<float>(), S->velOld.as<float>(),
-                                            flipAlpha, (double)la, (double)lb);
+  BinsOrder order;
+  if (np >= MR_BINS_MIN)
+    MSBG_CUDA_TRY(ctx, bins_build(S->scratch, dp, np, BinsGrid{g.sx, g.sy, g.sz, g.sh0, g.nbx, g.nby},
+                                  ctx->nb(), st, order));
+  k_g2p_mr<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, S->vel.as<float2>(), order, flipAlpha,
+                                            (double)la, (double)lb);
   MSBG_CUDA_TRY(ctx, cudaGetLastError());
   if (!onDevice)
     MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(particles, dp, sizeof(msbg_flip_particle) * np,

@@ -209,3 +209,32 @@ def test_downsample_velocity_bit_identical(cfg):
         ctx.close()
         if ref is not None:
             ref.close()
+
+
+@pytest.mark.parametrize("name", list(GRIDS))
+@pytest.mark.parametrize("order", ["blocks", "random"])
+def test_many_particles_in_any_order(name, order):
+    """Enough particles for G2P to order them, in block order and in none, some outside the grid
+    or without a finite position: the bits of batches below that size."""
+    ctx, res, bsx, nl, lev = _ctx(name)
+    try:
+        n = msbg_gpu.packed_voxels(bsx, lev)
+        vel, old = _channels(n, 5)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL, vel)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL_OLD, old)
+        assert np.array_equal(ctx.flip_mr_channel(msbg_gpu.FLIP_VEL), vel)
+        assert np.array_equal(ctx.flip_mr_channel(msbg_gpu.FLIP_VEL_OLD), old)
+        p = particles_for(res, 150001, 9)
+        if order == "blocks":
+            c = np.clip(np.nan_to_num(p["pos"]), 0, res - 1).astype(np.int64) // bsx
+            nb = res // bsx
+            p = p[np.argsort(c[:, 0] + nb * (c[:, 1] + nb * c[:, 2]), kind="stable")]
+        q, r = p.copy(), p.copy()
+        ctx.flip_g2p_mr(q, ALPHA)
+        for i in range(0, len(r), 50000):
+            part = r[i:i + 50000].copy()
+            ctx.flip_g2p_mr(part, ALPHA)
+            r[i:i + 50000] = part
+        assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
+    finally:
+        ctx.close()
