@@ -127,3 +127,46 @@ def test_particles_outside_or_not_finite(setup):
     ctx.flip_g2p(r, 0.95)
     r_o = oracle.flip_g2p(RES, BSX, q, vel, old, 0.95)
     assert np.array_equal(r["vel"], r_o["vel"])
+
+
+@pytest.mark.parametrize("res,bsx", [(32, 8), (64, 16), (64, 32)])
+@pytest.mark.parametrize("order", ["cells", "random"])
+def test_many_particles_in_any_order(res, bsx, order):
+    """Enough particles for the cell-by-cell P2G and the ordered G2P, in cell order and in none,
+    some outside the grid, on its faces or without a finite position.  G2P gives the bits that
+    batches below that size give; P2G is held to the bounds of test_p2g_matches_restatement."""
+    p = msbg_gpu.flip_particles(res, bsx, z_liquid=0.6, ppv=8, air_ppv=2, air_band=6, seed=3)
+    rng = np.random.default_rng(8)
+    extra = np.zeros(4096, msbg_gpu.FLIP_PARTICLE)
+    extra["pos"] = rng.uniform(-1.5, res + 1.5, (4096, 3))
+    extra["pos"][:512] = np.round(extra["pos"][:512] * 2) / 2
+    extra["pos"][512:520, 1] = np.nan
+    extra["pos"][520:524, 0] = np.inf
+    extra["vel"] = rng.standard_normal((4096, 3))
+    p = np.concatenate([p, extra])
+    assert len(p) > 1 << 16
+    if order == "random":
+        p = p[rng.permutation(len(p))]
+    n = res ** 3
+    ctx = msbg_gpu.Context(0)
+    try:
+        ctx.set_topology(res, res, res, bsx)
+        act = ctx.flip_p2g(p)
+        vel = ctx.flip_channel(msbg_gpu.FLIP_VEL, n)
+        beta = ctx.flip_channel(msbg_gpu.FLIP_BETA, n)
+        vel_o, mass_o, beta_o, act_o = oracle.flip_p2g(res, bsx, p)
+        assert np.array_equal(ctx.flip_channel(msbg_gpu.FLIP_MASS, n), mass_o)
+        assert np.array_equal(np.sort(act), np.nonzero(act_o)[0])
+        assert np.abs(vel - vel_o).max() <= 1e-5 * max(1.0, np.abs(vel_o).max())
+        bad = np.abs(beta - beta_o) > 1e-5 * np.maximum(1e-3, np.abs(beta_o))
+        assert bad.mean() <= 1e-4, bad.sum()
+        ctx.flip_gravity(-9.8, 0.02)
+        q, r = p.copy(), p.copy()
+        ctx.flip_g2p(q, 0.95)
+        for i in range(0, len(r), 60000):
+            part = r[i:i + 60000].copy()
+            ctx.flip_g2p(part, 0.95)
+            r[i:i + 60000] = part
+        assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
+    finally:
+        ctx.close()
