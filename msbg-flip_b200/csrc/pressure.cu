@@ -276,7 +276,6 @@ int msbg::ps::pressure_prepare(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
     MSBG_CUDA_TRY(ctx, upload(D->face, L.face, st));
     if (!onDevice) MSBG_CUDA_TRY(ctx, upload(D->ifOff, L.ifOff, st));
     MSBG_CUDA_TRY(ctx, upload(D->toCoarse, L.toCoarse, st));
-    MSBG_CUDA_TRY(ctx, upload(D->passTiles, L.passTiles, st));
     MSBG_CUDA_TRY(ctx, upload(D->groupTiles, L.groupTiles, st));
     if (!onDevice) {
       MSBG_CUDA_TRY(ctx, upload(D->diag, L.diag, st));
@@ -380,7 +379,7 @@ int msbg::ps::pressure_prepare(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
   MSBG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   for (const auto& D : S.dev)
     S.h2dBytes += (int64_t)(D->tileOff.bytes + D->face.bytes + D->ifOff.bytes +
-                            D->toCoarse.bytes + D->passTiles.bytes + D->groupTiles.bytes +
+                            D->toCoarse.bytes + D->groupTiles.bytes +
                             (onDevice ? 0
                                       : D->diag.bytes + D->cx.bytes + D->cy.bytes +
                                             D->cz.bytes + D->ifc.bytes));

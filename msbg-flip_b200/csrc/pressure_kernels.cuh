@@ -47,6 +47,20 @@ __host__ __device__ __forceinline__ int64_t xface_words(int64_t nCells) {
   return (xface_len(nCells) + 3) & ~(int64_t)3;
 }
 
+// Per-tile record: its offset and what its six faces need to gather a halo, resolved
+// (256 bytes: one bulk copy in the pipelined kernels).
+struct FaceRes {
+  int kind, nts, oa, ob, cov, pad;
+  int64_t nOff;   // SAME/COARSER: neighbour tile offset
+  int64_t ifOwn;  // COARSER: our interface-coupling plane
+};
+struct __align__(16) TileRec {
+  int64_t off;
+  int64_t pad;
+  FaceRes f[6];
+};
+static_assert(sizeof(TileRec) == 256, "tile record is one 256-byte bulk copy");
+
 __host__ __device__ __forceinline__ int tidx(int ts, int i, int j, int k) { return i + ts * (j + ts * k); }
 
 // Cell of a tile addressed by its face plane: position along dir = p, face

@@ -315,8 +315,7 @@ void launch_matvec(Solver& S, int m, const float* x, float* q, cudaStream_t st, 
           <<<grid, pipe::NT_APPLY, pipe::SMEM, st>>>(S.views[m], P.start, P.count, x, nullptr, q,
                                                      nullptr, nullptr, nullptr, err, nullptr);
     } else {
-      const int* lst = S.dev[m]->passTiles.as<int>() + P.start;
-      TS_DISPATCH(P.ts, (k_matvec_dot<T, float><<<P.count, T * T, 0, st>>>(S.views[m], lst, x, q,
+      TS_DISPATCH(P.ts, (k_matvec_dot<T, float><<<P.count, TileGeo<T>::NT, 0, st>>>(S.views[m], P.start, x, q,
                                                                             nullptr)));
     }
   }
@@ -475,9 +474,8 @@ extern "C" int msbg_gpu_restrict(msbg_gpu_ctx* ctx, int levelMgCoarse, const flo
                                                      dx.as<float>(), db.as<float>(), nullptr,
                                                      dc.as<float>(), coff, nullptr, err, nullptr);
     } else {
-      const int* lst = S->dev[mf]->passTiles.as<int>() + Pp.start;
-      TS_DISPATCH(Pp.ts, (k_residual_restrict<T, float, float><<<Pp.count, T * T, 0, st>>>(
-                             S->views[mf], lst, dx.as<float>(), db.as<float>(), dc.as<float>(),
+      TS_DISPATCH(Pp.ts, (k_residual_restrict<T, float, float><<<Pp.count, TileGeo<T>::NT, 0, st>>>(
+                             S->views[mf], Pp.start, dx.as<float>(), db.as<float>(), dc.as<float>(),
                              coff)));
     }
   }

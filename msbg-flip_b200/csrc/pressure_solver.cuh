@@ -69,10 +69,6 @@ struct Solver {
 template <typename VT>
 void set_kernel_attrs() {
   const int pipeSmem = (int)pipe::SMEM;
-  cudaFuncSetAttribute(k_smooth<16, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smooth_smem<16>());
-  cudaFuncSetAttribute(k_smooth<8, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smooth_smem<8>());
   cudaFuncSetAttribute(k_smooth_pipe16<VT, pipe::NT_SMOOTH>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pipe::SMEM_SMOOTH);
   cudaFuncSetAttribute(k_apply_pipe16<APPLY_MATVEC, VT, VT, pipe::NT_APPLY>,
@@ -121,7 +117,6 @@ struct Runner {
     return useFaces && usePipe && D.xf.p && S.views[m].cxf ? D.xf.template as<V>() : nullptr;
   }
 
-  const int* passList(int m) { return S.dev[m]->passTiles.template as<int>(); }
   const int* groupList(int m) { return S.dev[m]->groupTiles.template as<int>(); }
 
   // One smoothing sweep of MG level m: the (level, colour) passes in order
@@ -133,15 +128,14 @@ struct Runner {
     for (int pi = 0; pi < np; pi++) {
       const Level::Pass& P = L.passes[post ? np - 1 - pi : pi];
       if (!P.count) continue;
-      const int* lst = passList(m) + P.start;
       if (P.ts == 16 && usePipe) {
         const int grid = std::min(P.count, numSMs);
         // passes are contiguous tile-id ranges (register_tiles sorts by pass)
         k_smooth_pipe16<V, pipe::NT_SMOOTH><<<grid, pipe::NT_SMOOTH, pipe::SMEM_SMOOTH, st>>>(
             S.views[m], P.start, P.count, x, b, inner, post ? 1 : 0, err, xf);
       } else {
-        TS_DISPATCH(P.ts, (k_smooth<T, V><<<P.count, T * T, smooth_smem<T>(), st>>>(
-                               S.views[m], lst, x, b, inner, post ? 1 : 0)));
+        TS_DISPATCH(P.ts, (k_smooth<T, V><<<P.count, TileGeo<T>::NT, 0, st>>>(
+                               S.views[m], P.start, x, b, inner, post ? 1 : 0)));
       }
       launches++;
     }
@@ -155,7 +149,8 @@ struct Runner {
     V* xf = m == last ? nullptr : faces<V>(m);
     if (xf) cudaMemsetAsync(xf, 0, sizeof(V) * xface_len(L.nCells), st);
     if (m == last) {
-      k_coarse_solve<V><<<1, 512, 0, st>>>(S.dCoarseInv.template as<double>(), S.H.nCoarse,
+      k_coarse_solve<V><<<(S.H.nCoarse + COARSE_ROWS - 1) / COARSE_ROWS,
+                          COARSE_ROWS * COARSE_PARTS, 0, st>>>(S.dCoarseInv.template as<double>(), S.H.nCoarse,
                                            S.dCoarseCells.template as<int64_t>(), b, x);
       launches++;
       return;
@@ -191,9 +186,8 @@ struct Runner {
             S.views[0].cxf ? df : nullptr);
         off += grid;
       } else {
-        const int* lst = passList(0) + P.start;
-        TS_DISPATCH(P.ts, (k_matvec_dot<T, VT><<<P.count, T * T, 0, st>>>(S.views[0], lst, d, q,
-                                                                           partial + off)));
+        TS_DISPATCH(P.ts, (k_matvec_dot<T, VT><<<P.count, TileGeo<T>::NT, 0, st>>>(
+                               S.views[0], P.start, d, q, partial + off)));
         off += P.count;
       }
       launches++;
@@ -215,9 +209,8 @@ struct Runner {
         k_apply_pipe16<APPLY_RESIDUAL, V, float, pipe::NT_APPLY><<<grid, pipe::NT_APPLY, pipe::SMEM, st>>>(
             S.views[m], P.start, P.count, x, b, nullptr, bc, coff, nullptr, err, xf);
       } else {
-        const int* lst = passList(m) + P.start;
-        TS_DISPATCH(P.ts, (k_residual_restrict<T, V, float><<<P.count, T * T, 0, st>>>(
-                              S.views[m], lst, x, b, bc, coff)));
+        TS_DISPATCH(P.ts, (k_residual_restrict<T, V, float><<<P.count, TileGeo<T>::NT, 0, st>>>(
+                              S.views[m], P.start, x, b, bc, coff)));
       }
       launches++;
     }

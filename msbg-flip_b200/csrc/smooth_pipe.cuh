@@ -69,19 +69,6 @@ constexpr int TS = 16, N = TS * TS * TS, NT = 512;
 constexpr int NT_SMOOTH = 1024;  // threads of the smoother CTA
 constexpr int NT_APPLY = 1024;   // threads of the operator-application CTA
 
-// Per-face data of a tile needed to gather its halo.
-struct FaceRes {
-  int kind, nts, oa, ob, cov, pad;
-  int64_t nOff;   // SAME/COARSER: neighbour tile offset
-  int64_t ifOwn;  // COARSER: our interface-coupling plane
-};
-struct __align__(16) TileRec {
-  int64_t off;
-  int64_t pad;
-  FaceRes f[6];
-};
-static_assert(sizeof(TileRec) == 256, "tile record is one 256-byte bulk copy");
-
 // A zeroed guard band in front of the first stage keeps the neighbour reads
 // of boundary cells (whose couplings are zero) inside shared memory.
 constexpr int GUARD = TS * TS;
@@ -462,15 +449,15 @@ __global__ void __launch_bounds__(NTH, 1)
 }
 
 // Host side: the 256-byte tile records of one level (offset + resolved faces).
-inline std::vector<pipe::TileRec> build_tile_records(const Level& L) {
-  std::vector<pipe::TileRec> recs(L.tiles.size());
+inline std::vector<TileRec> build_tile_records(const Level& L) {
+  std::vector<TileRec> recs(L.tiles.size());
   for (size_t ti = 0; ti < L.tiles.size(); ti++) {
-    pipe::TileRec& r = recs[ti];
+    TileRec& r = recs[ti];
     std::memset(&r, 0, sizeof(r));
     r.off = L.tiles[ti].off;
     for (int f = 0; f < 6; f++) {
       const int* F = &L.face[(ti * 6 + f) * FACE_INTS];
-      pipe::FaceRes& fr = r.f[f];
+      FaceRes& fr = r.f[f];
       fr.kind = F[F_KIND];
       fr.nts = F[F_NTS];
       fr.oa = F[F_OA];

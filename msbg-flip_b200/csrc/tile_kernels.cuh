@@ -185,111 +185,170 @@ __global__ void __launch_bounds__(VEC_BLOCK) k_convert(VD* __restrict__ y, const
 }
 
 // ---------------------------------------------------------------------------
-// per-tile kernels (any tile size TS <= 16; one CTA per tile, thread (i,j)
-// owns the z column)
+// per-tile kernels (any tile size TS <= 16; one CTA per tile)
 // ---------------------------------------------------------------------------
-
-// In-tile neighbour sum S of cell (i,j,k) from a shared-memory tile, ghosts
-// from gs.  cxv etc. point at the tile's couplings (shared or global).
+// The passes and groups of 8^3 tiles and smaller are short: what they cost is
+// one chain of dependent global loads and a few barriers, so a thread owns one cell
+// (four on 16^3 tiles, where the pipelined kernels of smooth_pipe.cuh take over): all its
+// loads are in flight together, the face data come resolved from the tile's record, and
+// a half sweep is one update per thread.  With a thread per z column of a tile, a
+// smoothing pass of 8^3 / 4^3 tiles took 18 / 14 us and a residual 23 / 14 us (256^3 grid
+// of 16^3 blocks, 3 levels, B200), and the FP16 solve 17.4 ms; now 13.1.
 template <int TS>
-__device__ __forceinline__ float nbr_sum(const float* xs, const float* cxv, const float* cyv,
-                                         const float* czv, const float (*gs)[TS * TS], int i,
-                                         int j, int k) {
-  const int e = tidx(TS, i, j, k);
-  float S = 0.f;
-  S += (i > 0) ? cxv[e] * xs[e - 1] : gs[0][j + TS * k];
-  S += (i < TS - 1) ? cxv[e + 1] * xs[e + 1] : gs[1][j + TS * k];
-  S += (j > 0) ? cyv[e] * xs[e - TS] : gs[2][i + TS * k];
-  S += (j < TS - 1) ? cyv[e + TS] * xs[e + TS] : gs[3][i + TS * k];
-  S += (k > 0) ? czv[e] * xs[e - TS * TS] : gs[4][i + TS * j];
-  S += (k < TS - 1) ? czv[e + TS * TS] * xs[e + TS * TS] : gs[5][i + TS * j];
-  return S;
+struct TileGeo {
+  static constexpr int N = TS * TS * TS;
+  static constexpr int NT = TS == 16 ? 1024 : (N < 32 ? 32 : N);  // threads
+  static constexpr int PER = N > NT ? N / NT : 1;                  // cells per thread
+  static constexpr int P = TS + 2;                                 // padded edge
+  __device__ static constexpr int pad(int i, int j, int k) {
+    return (i + 1) + P * ((j + 1) + P * (k + 1));
+  }
+};
+
+// Coupling times neighbour of face cell (a, b) of face (dir, side), as ghost_sum.
+template <int TS, typename VT>
+__device__ __forceinline__ float halo_term(const LevelView& L, const TileRec& r, int ti,
+                                           const VT* __restrict__ x, int dir, int side, int a,
+                                           int b) {
+  const FaceRes& F = r.f[2 * dir + side];
+  const int kind = F.kind;
+  if (kind == FACE_NONE) return 0.f;
+  const float* cd = dir == 0 ? L.cx : dir == 1 ? L.cy : L.cz;
+  if (kind == FACE_SAME)
+    return cd[(side ? F.nOff : r.off) + plane_idx(TS, dir, 0, a, b)] *
+           to_f(x[F.nOff + plane_idx(TS, dir, side ? 0 : TS - 1, a, b)]);
+  if (kind == FACE_COARSER)
+    return L.ifc[F.ifOwn + a + TS * b] *
+           to_f(x[F.nOff + plane_idx(F.nts, dir, side ? 0 : F.nts - 1, F.oa + (a >> 1),
+                                     F.ob + (b >> 1))]);
+  return ghost_sum(L, x, ti, TS, dir, side, a, b);
 }
 
-// q = A d on the listed tiles, partial d.q per CTA.
+// A tile in shared memory: x inside a padded cube whose face halos hold the halo
+// terms (coupling times neighbour), and per cell of a thread the six couplings, 1
+// towards a halo: the neighbour sum is one multiply-add per face either way.
 template <int TS, typename VT>
-__global__ void __launch_bounds__(TS* TS) k_matvec_dot(LevelView L, const int* __restrict__ tiles,
-                                                       const VT* __restrict__ d,
-                                                       VT* __restrict__ q,
-                                                       double* __restrict__ partial) {
-  constexpr int N = TS * TS * TS, NT = TS * TS;
-  __shared__ float xs[N];
-  __shared__ float gs[6][NT];
-  const int ti = tiles[blockIdx.x];
-  const int64_t off = L.tileOff[ti];
-  const int t = threadIdx.x, i = t % TS, j = t / TS;
-  for (int e = t; e < N; e += NT) xs[e] = to_f(d[off + e]);
+struct TileCells {
+  using G = TileGeo<TS>;
+  float c[G::PER][6];
+  __device__ __forceinline__ void load(const LevelView& L, const TileRec& r, int ti,
+                                       const VT* __restrict__ x, float* xs) {
+    const int t = threadIdx.x;
+    const float* cx = L.cx + r.off;
+    const float* cy = L.cy + r.off;
+    const float* cz = L.cz + r.off;
 #pragma unroll
-  for (int f = 0; f < 6; f++) gs[f][t] = ghost_sum(L, d, ti, TS, f >> 1, f & 1, i, j);
+    for (int q = 0; q < G::PER; q++) {
+      const int e = t + G::NT * q;
+      if (e >= G::N) continue;
+      const int i = e % TS, j = (e / TS) % TS, k = e / (TS * TS);
+      c[q][0] = i > 0 ? cx[e] : 1.f;
+      c[q][1] = i < TS - 1 ? cx[e + 1] : 1.f;
+      c[q][2] = j > 0 ? cy[e] : 1.f;
+      c[q][3] = j < TS - 1 ? cy[e + TS] : 1.f;
+      c[q][4] = k > 0 ? cz[e] : 1.f;
+      c[q][5] = k < TS - 1 ? cz[e + TS * TS] : 1.f;
+      xs[G::pad(i, j, k)] = to_f(x[r.off + e]);
+    }
+    for (int h = t; h < 6 * TS * TS; h += G::NT) {
+      const int f = h / (TS * TS), a = h % TS, b = (h / TS) % TS, dir = f >> 1, side = f & 1;
+      const int p = side ? TS : -1;
+      xs[dir == 0 ? G::pad(p, a, b) : dir == 1 ? G::pad(a, p, b) : G::pad(a, b, p)] =
+          halo_term<TS>(L, r, ti, x, dir, side, a, b);
+    }
+  }
+  // in the order x-, x+, y-, y+, z-, z+
+  __device__ __forceinline__ float sum(const float* at, int q) const {
+    float S = 0.f;
+    S = fmaf(c[q][0], at[-1], S);
+    S = fmaf(c[q][1], at[1], S);
+    S = fmaf(c[q][2], at[-G::P], S);
+    S = fmaf(c[q][3], at[G::P], S);
+    S = fmaf(c[q][4], at[-G::P * G::P], S);
+    S = fmaf(c[q][5], at[G::P * G::P], S);
+    return S;
+  }
+};
+
+// q = A d on tiles tileBase.., partial d.q per CTA.
+template <int TS, typename VT>
+__global__ void __launch_bounds__(TileGeo<TS>::NT) k_matvec_dot(LevelView L, int tileBase,
+                                                                const VT* __restrict__ d,
+                                                                VT* __restrict__ q,
+                                                                double* __restrict__ partial) {
+  using G = TileGeo<TS>;
+  __shared__ float xs[G::P * G::P * G::P];
+  const int ti = tileBase + blockIdx.x, t = threadIdx.x;
+  const TileRec& r = reinterpret_cast<const TileRec*>(L.tileRec)[ti];
+  TileCells<TS, VT> C;
+  C.load(L, r, ti, d, xs);
+  float dg[G::PER];
+#pragma unroll
+  for (int p = 0; p < G::PER; p++) dg[p] = t + G::NT * p < G::N ? L.diag[r.off + t + G::NT * p] : 0.f;
   __syncthreads();
   double acc = 0;
-  const float* cxv = L.cx + off;
-  const float* cyv = L.cy + off;
-  const float* czv = L.cz + off;
-#pragma unroll 4
-  for (int k = 0; k < TS; k++) {
-    const int e = tidx(TS, i, j, k);
-    const float dg = L.diag[off + e];
+#pragma unroll
+  for (int p = 0; p < G::PER; p++) {
+    const int e = t + G::NT * p;
+    if (e >= G::N) continue;
+    const float* at = xs + G::pad(e % TS, (e / TS) % TS, e / (TS * TS));
     float y = 0.f;
-    if (dg > 0.f) y = dg * xs[e] - nbr_sum<TS>(xs, cxv, cyv, czv, gs, i, j, k);
-    q[off + e] = from_f<VT>(y);
-    acc += (double)xs[e] * (double)to_f(from_f<VT>(y));
+    if (dg[p] > 0.f) y = fmaf(dg[p], *at, -C.sum(at, p));
+    q[r.off + e] = from_f<VT>(y);
+    acc += (double)*at * (double)to_f(from_f<VT>(y));
   }
   acc = block_sum(acc);
   if (t == 0 && partial) partial[blockIdx.x] = acc;
 }
 
-// r = b - A x on the listed tiles, restricted (sum over the liquid children,
+// r = b - A x on tiles tileBase.., restricted (sum over the liquid children,
 // P^T) into the coarse right-hand side bc (vectors VT, coarse vectors VC).
 template <int TS, typename VT, typename VC>
-__global__ void __launch_bounds__(TS* TS) k_residual_restrict(LevelView L,
-                                                              const int* __restrict__ tiles,
-                                                              const VT* __restrict__ x,
-                                                              const VT* __restrict__ b,
-                                                              VC* __restrict__ bc,
-                                                              const int64_t* __restrict__ coarseOff) {
-  constexpr int N = TS * TS * TS, NT = TS * TS;
-  __shared__ float xs[N];
-  __shared__ float rs[N];
-  __shared__ float gs[6][NT];
-  const int ti = tiles[blockIdx.x];
-  const int64_t off = L.tileOff[ti];
-  const int t = threadIdx.x, i = t % TS, j = t / TS;
-  for (int e = t; e < N; e += NT) xs[e] = to_f(x[off + e]);
-#pragma unroll
-  for (int f = 0; f < 6; f++) gs[f][t] = ghost_sum(L, x, ti, TS, f >> 1, f & 1, i, j);
-  __syncthreads();
-  const float* cxv = L.cx + off;
-  const float* cyv = L.cy + off;
-  const float* czv = L.cz + off;
-#pragma unroll 4
-  for (int k = 0; k < TS; k++) {
-    const int e = tidx(TS, i, j, k);
-    const float dg = L.diag[off + e];
-    float r = 0.f;
-    if (dg > 0.f)
-      r = to_f(b[off + e]) - (dg * xs[e] - nbr_sum<TS>(xs, cxv, cyv, czv, gs, i, j, k));
-    rs[e] = r;
-  }
-  __syncthreads();
+__global__ void __launch_bounds__(TileGeo<TS>::NT)
+    k_residual_restrict(LevelView L, int tileBase, const VT* __restrict__ x,
+                        const VT* __restrict__ b, VC* __restrict__ bc,
+                        const int64_t* __restrict__ coarseOff) {
+  using G = TileGeo<TS>;
+  __shared__ float xs[G::P * G::P * G::P];
+  __shared__ float rs[G::N];
+  const int ti = tileBase + blockIdx.x, t = threadIdx.x;
+  const TileRec& r = reinterpret_cast<const TileRec*>(L.tileRec)[ti];
+  TileCells<TS, VT> C;
+  C.load(L, r, ti, x, xs);
   const int* tc = L.toCoarse + (size_t)ti * 6;
   const int ct = tc[0], ox = tc[1], oy = tc[2], oz = tc[3], agg = tc[4], cts = tc[5];
-  if (ct < 0) return;
-  VC* dst = bc + coarseOff[ct];
-  if (agg) {
-    constexpr int H = TS / 2;
-    for (int c = t; c < H * H * H; c += NT) {
-      const int ci = c % H, cj = (c / H) % H, ck = c / (H * H);
-      const int e = tidx(TS, 2 * ci, 2 * cj, 2 * ck);
-      const float s = rs[e] + rs[e + 1] + rs[e + TS] + rs[e + TS + 1] + rs[e + TS * TS] +
-                      rs[e + TS * TS + 1] + rs[e + TS * TS + TS] + rs[e + TS * TS + TS + 1];
-      dst[tidx(cts, ox + ci, oy + cj, oz + ck)] = from_f<VC>(s);
-    }
-  } else {
-    for (int e = t; e < N; e += NT) {
-      const int ii = e % TS, jj = (e / TS) % TS, kk = e / (TS * TS);
-      dst[tidx(cts, ox + ii, oy + jj, oz + kk)] = from_f<VC>(rs[e]);
-    }
+  VC* dst = ct >= 0 ? bc + coarseOff[ct] : nullptr;
+  float dg[G::PER], bv[G::PER];
+#pragma unroll
+  for (int p = 0; p < G::PER; p++) {
+    const int e = t + G::NT * p;
+    dg[p] = e < G::N ? L.diag[r.off + e] : 0.f;
+    bv[p] = e < G::N ? to_f(b[r.off + e]) : 0.f;
+  }
+  __syncthreads();
+  if (!dst) return;
+#pragma unroll
+  for (int p = 0; p < G::PER; p++) {
+    const int e = t + G::NT * p;
+    if (e >= G::N) continue;
+    const int i = e % TS, j = (e / TS) % TS, k = e / (TS * TS);
+    const float* at = xs + G::pad(i, j, k);
+    float v = 0.f;
+    if (dg[p] > 0.f) v = bv[p] - fmaf(dg[p], *at, -C.sum(at, p));
+    if (agg)
+      rs[e] = v;
+    else
+      dst[tidx(cts, ox + i, oy + j, oz + k)] = from_f<VC>(v);
+  }
+  if (!agg) return;
+  __syncthreads();
+  constexpr int H = TS / 2;
+  for (int c = t; c < H * H * H; c += G::NT) {
+    const int ci = c % H, cj = (c / H) % H, ck = c / (H * H);
+    const int e = tidx(TS, 2 * ci, 2 * cj, 2 * ck);
+    const float s = rs[e] + rs[e + 1] + rs[e + TS] + rs[e + TS + 1] + rs[e + TS * TS] +
+                    rs[e + TS * TS + 1] + rs[e + TS * TS + TS] + rs[e + TS * TS + TS + 1];
+    dst[tidx(cts, ox + ci, oy + cj, oz + ck)] = from_f<VC>(s);
   }
 }
 
@@ -365,72 +424,72 @@ __global__ void __launch_bounds__(TS* TS) k_prolong(LevelView L, const int* __re
   }
 }
 
-// Red-black Gauss-Seidel inside each listed tile, `inner` iterations, ghosts
+// Red-black Gauss-Seidel inside tiles tileBase.., `inner` iterations, ghosts
 // frozen at their values when the tile is loaded.  reverse=0: red then black;
 // reverse=1: black then red (the adjoint order).
 template <int TS, typename VT>
-__global__ void __launch_bounds__(TS* TS) k_smooth(LevelView L, const int* __restrict__ tiles,
-                                                   VT* __restrict__ x, const VT* __restrict__ b,
-                                                   int inner, int reverse) {
-  constexpr int N = TS * TS * TS, NT = TS * TS;
-  extern __shared__ __align__(128) float sm[];
-  float* xs = sm;
-  float* cxs = sm + N;
-  float* cys = sm + 2 * N;
-  float* czs = sm + 3 * N;
-  float(*gs)[NT] = reinterpret_cast<float(*)[NT]>(sm + 4 * N);
-  const int ti = tiles[blockIdx.x];
-  const int64_t off = L.tileOff[ti];
-  const int t = threadIdx.x, i = t % TS, j = t / TS;
-  for (int e = t; e < N; e += NT) {
-    xs[e] = to_f(x[off + e]);
-    cxs[e] = L.cx[off + e];
-    cys[e] = L.cy[off + e];
-    czs[e] = L.cz[off + e];
-  }
-  float bb[TS], inv[TS];
+__global__ void __launch_bounds__(TileGeo<TS>::NT) k_smooth(LevelView L, int tileBase,
+                                                            VT* __restrict__ x,
+                                                            const VT* __restrict__ b, int inner,
+                                                            int reverse) {
+  using G = TileGeo<TS>;
+  __shared__ float xs[G::P * G::P * G::P];
+  const int ti = tileBase + blockIdx.x, t = threadIdx.x;
+  const TileRec& r = reinterpret_cast<const TileRec*>(L.tileRec)[ti];
+  TileCells<TS, VT> C;
+  C.load(L, r, ti, x, xs);
+  float inv[G::PER], bb[G::PER];
+  int col[G::PER], at[G::PER];
 #pragma unroll
-  for (int k = 0; k < TS; k++) {
-    const int e = tidx(TS, i, j, k);
-    inv[k] = L.invdiag[off + e];
-    bb[k] = to_f(b[off + e]);
+  for (int p = 0; p < G::PER; p++) {
+    const int e = t + G::NT * p;
+    const int i = e % TS, j = (e / TS) % TS, k = e / (TS * TS);
+    inv[p] = e < G::N ? L.invdiag[r.off + e] : 0.f;
+    bb[p] = e < G::N ? to_f(b[r.off + e]) : 0.f;
+    col[p] = (i + j + k) & 1;
+    at[p] = e < G::N ? G::pad(i, j, k) : G::pad(0, 0, 0);
   }
-#pragma unroll
-  for (int f = 0; f < 6; f++) gs[f][t] = ghost_sum(L, x, ti, TS, f >> 1, f & 1, i, j);
   __syncthreads();
   for (int it = 0; it < inner; it++) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int colour = reverse ? 1 - h : h;
 #pragma unroll
-      for (int k = 0; k < TS; k++) {
-        if (((i + j + k) & 1) != colour || inv[k] == 0.f) continue;
-        const float S = nbr_sum<TS>(xs, cxs, cys, czs, gs, i, j, k);
-        xs[tidx(TS, i, j, k)] = (bb[k] + S) * inv[k];
-      }
+      for (int p = 0; p < G::PER; p++)
+        if (col[p] == colour && inv[p] != 0.f)
+          xs[at[p]] = (bb[p] + C.sum(xs + at[p], p)) * inv[p];
       __syncthreads();
     }
   }
-  for (int e = t; e < N; e += NT) x[off + e] = from_f<VT>(xs[e]);
+#pragma unroll
+  for (int p = 0; p < G::PER; p++)
+    if (t + G::NT * p < G::N) x[r.off + t + G::NT * p] = from_f<VT>(xs[at[p]]);
 }
 
-template <int TS>
-size_t smooth_smem() {
-  return sizeof(float) * (4 * TS * TS * TS + 6 * TS * TS);
-}
-
-// Coarsest level: x = A^-1 b with the dense FP64 inverse (symmetric).
+// Coarsest level: x = A^-1 b with the dense FP64 inverse (symmetric).  A CTA has 16
+// rows and 32 parts of the columns, summed part by part in a fixed order.  (One CTA with
+// a thread per row reads up to 2 MB of the inverse alone: 45 us at 500 cells.)
+constexpr int COARSE_ROWS = 16, COARSE_PARTS = 32;
 template <typename VT>
-__global__ void __launch_bounds__(512) k_coarse_solve(const double* __restrict__ Ainv, int n,
-                                                      const int64_t* __restrict__ cells,
-                                                      const VT* __restrict__ b,
-                                                      VT* __restrict__ x) {
+__global__ void __launch_bounds__(COARSE_ROWS* COARSE_PARTS)
+    k_coarse_solve(const double* __restrict__ Ainv, int n, const int64_t* __restrict__ cells,
+                   const VT* __restrict__ b, VT* __restrict__ x) {
   __shared__ double bs[512];
-  const int t = threadIdx.x;
-  if (t < n) bs[t] = to_f(b[cells[t]]);
+  __shared__ double part[COARSE_PARTS][COARSE_ROWS];
+  const int t = threadIdx.x, r = t % COARSE_ROWS, q = t / COARSE_ROWS;
+  const int row = blockIdx.x * COARSE_ROWS + r;
+  for (int i = t; i < n; i += COARSE_ROWS * COARSE_PARTS) bs[i] = to_f(b[cells[i]]);
   __syncthreads();
-  if (t >= n) return;
   double s = 0;
-  for (int j = 0; j < n; j++) s += Ainv[(size_t)j * n + t] * bs[j];
-  x[cells[t]] = from_f<VT>((float)s);
+  if (row < n) {
+#pragma unroll 8
+    for (int j = q; j < n; j += COARSE_PARTS) s += Ainv[(size_t)j * n + row] * bs[j];
+  }
+  part[q][r] = s;
+  __syncthreads();
+  if (t >= COARSE_ROWS || row >= n) return;
+  s = 0;
+#pragma unroll
+  for (int i = 0; i < COARSE_PARTS; i++) s += part[i][t];
+  x[cells[row]] = from_f<VT>((float)s);
 }
