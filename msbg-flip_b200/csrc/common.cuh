@@ -8,11 +8,49 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "msbg_gpu.h"
 
 namespace msbg {
+
+#ifdef __CUDACC__
+// Programmatic dependent launch.  The kernels of a solver iteration, or the colour passes of a
+// smoother, follow each other in one stream, each reading what the last one wrote, and where
+// they are short a launch is mostly latency.  Launched through launch(), a kernel may start while its predecessor still
+// runs (once all CTAs of that one have called pdl_go or ended): it sets itself up and reads
+// what no kernel of the chain writes (an operator, block lists), then calls pdl_wait, which
+// returns when the predecessor has completed and its writes are visible.  Every thread of
+// such a kernel calls pdl_wait before it touches what a predecessor wrote and before it returns, so that its
+// own completion says the same of all kernels before it.  Without the launch attribute both
+// are no-ops.
+__device__ __forceinline__ void pdl_go() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+void launch_if(bool dependent, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+               cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = dependent ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+            A&&... args) {
+  launch_if(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
+}
+#endif
 
 // Neighbour / block-map codes stored in slot tables (slot >= 0 = value block).
 enum : int {

@@ -445,18 +445,19 @@ int run_pcg(msbg_gpu_ctx* ctx, Solver& S, Runner<VT>& R, const VT* bin, double t
     out.status = 0;
     return MSBG_OK;
   }
+  const bool dep = vectors_dependent(n);
   auto iteration = [&]() {
     R.launches += 6;  // finalize x3, axpy_norm, dot, update_d
     int nt = R.matvec_dot(d, q, part, df);
-    k_finalize<<<1, 1024, 0, st>>>(part, nt, sc, FIN_DQ_ALPHA);
-    k_axpy_norm<<<VEC_GRID, VEC_BLOCK, 0, st>>>(x, r, d, q, n, sc, part);
-    k_finalize<<<1, 1024, 0, st>>>(part, VEC_GRID, sc, FIN_RR);
+    launch_if(dep, k_finalize, 1, 1024, 0, st, part, nt, sc, FIN_DQ_ALPHA);
+    launch_if(dep, k_axpy_norm<VT>, VEC_GRID, VEC_BLOCK, 0, st, x, r, d, q, n, sc, part);
+    launch_if(dep, k_finalize, 1, 1024, 0, st, part, VEC_GRID, sc, FIN_RR);
     R.vcycle(0, z, r);
-    k_dot<<<VEC_GRID, VEC_BLOCK, 0, st>>>(r, z, n, part);
-    k_finalize<<<1, 1024, 0, st>>>(part, VEC_GRID, sc, FIN_RHONEW_BETA);
-    k_update_d<<<VEC_GRID, VEC_BLOCK, 0, st>>>(d, z, n, sc);
+    launch_if(dep, k_dot<VT, VT>, VEC_GRID, VEC_BLOCK, 0, st, r, z, n, part);
+    launch_if(dep, k_finalize, 1, 1024, 0, st, part, VEC_GRID, sc, FIN_RHONEW_BETA);
+    launch_if(dep, k_update_d<VT>, VEC_GRID, VEC_BLOCK, 0, st, d, z, n, sc);
     if (df) {
-      k_update_d<<<VEC_GRID, VEC_BLOCK, 0, st>>>(df, zf, nf, sc);
+      launch_if(dep, k_update_d<VT>, VEC_GRID, VEC_BLOCK, 0, st, df, zf, nf, sc);
       R.launches++;
     }
     cudaMemcpyAsync(S.hScal, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
@@ -845,12 +846,13 @@ int solve_reliable(msbg_gpu_ctx* ctx, Solver& S, Runner<float>& R, const msbg_gp
     o.status = 0;
     return MSBG_OK;
   }
+  const bool dep = vectors_dependent(n);
   auto part1 = [&]() {
     R.launches += 3;
     const int nt = R.matvec_dot(d, q, part, df);
-    k_finalize<<<1, 1024, 0, st>>>(part, nt, sc, corr ? FIN_FCG_DQ_ALPHA : FIN_DQ_ALPHA);
-    k_axpy64_norm<<<VEC_GRID, VEC_BLOCK, 0, st>>>(x64, r, d, q, n, sc, part);
-    k_finalize<<<1, 1024, 0, st>>>(part, VEC_GRID, sc, FIN_RR);
+    launch_if(dep, k_finalize, 1, 1024, 0, st, part, nt, sc, corr ? FIN_FCG_DQ_ALPHA : FIN_DQ_ALPHA);
+    launch_if(dep, k_axpy64_norm, VEC_GRID, VEC_BLOCK, 0, st, x64, r, d, q, n, sc, part);
+    launch_if(dep, k_finalize, 1, 1024, 0, st, part, VEC_GRID, sc, FIN_RR);
     cudaMemcpyAsync(S.hScal, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
   };
   int precondRc = MSBG_OK;
@@ -859,20 +861,20 @@ int solve_reliable(msbg_gpu_ctx* ctx, Solver& S, Runner<float>& R, const msbg_gp
     const int e = precond(true);
     if (e) precondRc = e;
     if (!corr) {
-      k_dot<<<VEC_GRID, VEC_BLOCK, 0, st>>>(r, z, n, part);
-      k_finalize<<<1, 1024, 0, st>>>(part, VEC_GRID, sc, FIN_RHONEW_BETA);
-      k_update_d<<<VEC_GRID, VEC_BLOCK, 0, st>>>(d, z, n, sc);
+      launch_if(dep, k_dot<float, float>, VEC_GRID, VEC_BLOCK, 0, st, r, z, n, part);
+      launch_if(dep, k_finalize, 1, 1024, 0, st, part, VEC_GRID, sc, FIN_RHONEW_BETA);
+      launch_if(dep, k_update_d<float>, VEC_GRID, VEC_BLOCK, 0, st, d, z, n, sc);
       if (df) {
-        k_update_d<<<VEC_GRID, VEC_BLOCK, 0, st>>>(df, zf, nf, sc);
+        launch_if(dep, k_update_d<float>, VEC_GRID, VEC_BLOCK, 0, st, df, zf, nf, sc);
         R.launches++;
       }
     } else {
       // beta = -(z.q)/(d.q); d = z + beta d; rho = d.r for the next alpha
-      k_dot<<<VEC_GRID, VEC_BLOCK, 0, st>>>(z, q, n, part);
-      k_finalize<<<1, 1024, 0, st>>>(part, VEC_GRID, sc, FIN_FCG_BETA);
-      k_update_d<<<VEC_GRID, VEC_BLOCK, 0, st>>>(d, z, n, sc);
-      k_dot<<<VEC_GRID, VEC_BLOCK, 0, st>>>(d, r, n, part);
-      k_finalize<<<1, 1024, 0, st>>>(part, VEC_GRID, sc, FIN_RHO);
+      launch_if(dep, k_dot<float, float>, VEC_GRID, VEC_BLOCK, 0, st, z, q, n, part);
+      launch_if(dep, k_finalize, 1, 1024, 0, st, part, VEC_GRID, sc, FIN_FCG_BETA);
+      launch_if(dep, k_update_d<float>, VEC_GRID, VEC_BLOCK, 0, st, d, z, n, sc);
+      launch_if(dep, k_dot<float, float>, VEC_GRID, VEC_BLOCK, 0, st, d, r, n, part);
+      launch_if(dep, k_finalize, 1, 1024, 0, st, part, VEC_GRID, sc, FIN_RHO);
       R.launches += 3;
     }
   };

@@ -16,6 +16,11 @@
 namespace msbg {
 namespace ps {
 
+// What a smoothing sweep from x = 0 may take for granted (zeroStart of the smoothers): the
+// tile's own x (bit 0) and the halos of faces of kind k (bit k: neighbours that the
+// sweep has not reached yet) are 0, whatever the vector's memory holds.
+constexpr int ZERO_OWN = 1;
+
 struct LevelView {
   const int64_t* tileOff;
   const int* face;

@@ -69,7 +69,9 @@ struct Solver {
 template <typename VT>
 void set_kernel_attrs() {
   const int pipeSmem = (int)pipe::SMEM;
-  cudaFuncSetAttribute(k_smooth_pipe16<VT, pipe::NT_SMOOTH>,
+  cudaFuncSetAttribute(k_smooth_pipe16<VT, pipe::NT_SMOOTH, true>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pipe::SMEM_SMOOTH);
+  cudaFuncSetAttribute(k_smooth_pipe16<VT, pipe::NT_SMOOTH, false>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pipe::SMEM_SMOOTH);
   cudaFuncSetAttribute(k_apply_pipe16<APPLY_MATVEC, VT, VT, pipe::NT_APPLY>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, pipeSmem);
@@ -121,21 +123,29 @@ struct Runner {
 
   // One smoothing sweep of MG level m: the (level, colour) passes in order
   // (pre) or in reverse order with the adjoint colour order inside (post).
+  // fromZero: x counts as 0 (its memory, faces included, may hold anything): a pass of a
+  // pre-sweep then reads no more of it than the passes before have written, which are
+  // the other colour of its own level if it is the second, and the finer levels.
   template <typename V>
-  void smooth(int m, V* x, const V* b, bool post, V* xf = nullptr) {
+  void smooth(int m, V* x, const V* b, bool post, V* xf = nullptr, bool fromZero = false) {
     const Level& L = S.H.levels[m];
     const int np = (int)L.passes.size();
     for (int pi = 0; pi < np; pi++) {
       const Level::Pass& P = L.passes[post ? np - 1 - pi : pi];
       if (!P.count) continue;
+      const int zs = !fromZero ? 0
+                               : ZERO_OWN | (1 << FACE_COARSER) |
+                                     (P.colour == 0 ? 1 << FACE_SAME : 0);
       if (P.ts == 16 && usePipe) {
         const int grid = std::min(P.count, numSMs);
         // passes are contiguous tile-id ranges (register_tiles sorts by pass)
-        k_smooth_pipe16<V, pipe::NT_SMOOTH><<<grid, pipe::NT_SMOOTH, pipe::SMEM_SMOOTH, st>>>(
-            S.views[m], P.start, P.count, x, b, inner, post ? 1 : 0, err, xf);
+        launch(fromZero ? k_smooth_pipe16<V, pipe::NT_SMOOTH, true>
+                        : k_smooth_pipe16<V, pipe::NT_SMOOTH, false>,
+               grid, pipe::NT_SMOOTH, pipe::SMEM_SMOOTH, st, S.views[m], P.start, P.count, x, b,
+               inner, post ? 1 : 0, err, xf, zs);
       } else {
-        TS_DISPATCH(P.ts, (k_smooth<T, V><<<P.count, TileGeo<T>::NT, 0, st>>>(
-                               S.views[m], P.start, x, b, inner, post ? 1 : 0)));
+        TS_DISPATCH(P.ts, (launch(k_smooth<T, V>, P.count, TileGeo<T>::NT, 0, st, S.views[m],
+                                   P.start, x, b, inner, post ? 1 : 0, zs)));
       }
       launches++;
     }
@@ -145,26 +155,29 @@ struct Runner {
   void vcycle(int m, V* x, const V* b) {
     const int last = (int)S.H.levels.size() - 1;
     const Level& L = S.H.levels[m];
-    cudaMemsetAsync(x, 0, sizeof(V) * L.nCells, st);
     V* xf = m == last ? nullptr : faces<V>(m);
-    if (xf) cudaMemsetAsync(xf, 0, sizeof(V) * xface_len(L.nCells), st);
+    // the first pre-sweep starts from 0 by itself; the coarsest level's x is 0 off the
+    // cells that the direct solve writes, from prepare on
+    if (m == last ? m == 0 : nPre == 0) {
+      cudaMemsetAsync(x, 0, sizeof(V) * L.nCells, st);
+      if (xf) cudaMemsetAsync(xf, 0, sizeof(V) * xface_len(L.nCells), st);
+    }
     if (m == last) {
-      k_coarse_solve<V><<<(S.H.nCoarse + COARSE_ROWS - 1) / COARSE_ROWS,
-                          COARSE_ROWS * COARSE_PARTS, 0, st>>>(S.dCoarseInv.template as<double>(), S.H.nCoarse,
-                                           S.dCoarseCells.template as<int64_t>(), b, x);
+      launch(k_coarse_solve<V>, (S.H.nCoarse + COARSE_ROWS - 1) / COARSE_ROWS,
+             COARSE_ROWS * COARSE_PARTS, 0, st, S.dCoarseInv.template as<double>(), S.H.nCoarse,
+             S.dCoarseCells.template as<int64_t>(), b, x);
       launches++;
       return;
     }
-    for (int s = 0; s < nPre; s++) smooth(m, x, b, false, xf);
+    for (int s = 0; s < nPre; s++) smooth(m, x, b, false, xf, s == 0);
     LevelDev& C = *S.dev[m + 1];
     residual_restrict(m, x, b, xf);
     float* xc = C.x.template as<float>();
     vcycle<float>(m + 1, xc, C.b.template as<float>());
     for (const auto& g : L.groups) {
       const int* lst = groupList(m) + g.start;
-      TS_DISPATCH(g.ts, (k_prolong<T, V, float><<<g.count, T * T, 0, st>>>(
-                            S.views[m], lst, x, xc, C.tileOff.template as<int64_t>(),
-                            coarseScale, xf)));
+      TS_DISPATCH(g.ts, (launch(k_prolong<T, V, float>, g.count, T * T, 0, st, S.views[m], lst, x, xc,
+                                C.tileOff.template as<int64_t>(), coarseScale, xf)));
       launches++;
     }
     for (int s = 0; s < nPost; s++) smooth(m, x, b, true, xf);
@@ -181,13 +194,13 @@ struct Runner {
       if (!P.count) continue;
       if (P.ts == 16 && usePipe) {
         const int grid = std::min(P.count, numSMs);
-        k_apply_pipe16<APPLY_MATVEC, VT, VT, pipe::NT_APPLY><<<grid, pipe::NT_APPLY, pipe::SMEM, st>>>(
-            S.views[0], P.start, P.count, d, nullptr, q, nullptr, nullptr, partial + off, err,
-            S.views[0].cxf ? df : nullptr);
+        launch(k_apply_pipe16<APPLY_MATVEC, VT, VT, pipe::NT_APPLY>, grid, pipe::NT_APPLY,
+               pipe::SMEM, st, S.views[0], P.start, P.count, d, nullptr, q, nullptr, nullptr,
+               partial + off, err, S.views[0].cxf ? df : nullptr);
         off += grid;
       } else {
-        TS_DISPATCH(P.ts, (k_matvec_dot<T, VT><<<P.count, TileGeo<T>::NT, 0, st>>>(
-                               S.views[0], P.start, d, q, partial + off)));
+        TS_DISPATCH(P.ts, (launch(k_matvec_dot<T, VT>, P.count, TileGeo<T>::NT, 0, st,
+                                   S.views[0], P.start, d, q, partial + off)));
         off += P.count;
       }
       launches++;
@@ -206,11 +219,12 @@ struct Runner {
       if (!P.count) continue;
       if (P.ts == 16 && usePipe) {
         const int grid = std::min(P.count, numSMs);
-        k_apply_pipe16<APPLY_RESIDUAL, V, float, pipe::NT_APPLY><<<grid, pipe::NT_APPLY, pipe::SMEM, st>>>(
-            S.views[m], P.start, P.count, x, b, nullptr, bc, coff, nullptr, err, xf);
+        launch(k_apply_pipe16<APPLY_RESIDUAL, V, float, pipe::NT_APPLY>, grid, pipe::NT_APPLY,
+               pipe::SMEM, st, S.views[m], P.start, P.count, x, b, nullptr, bc, coff, nullptr, err,
+               xf);
       } else {
-        TS_DISPATCH(P.ts, (k_residual_restrict<T, V, float><<<P.count, TileGeo<T>::NT, 0, st>>>(
-                              S.views[m], P.start, x, b, bc, coff)));
+        TS_DISPATCH(P.ts, (launch(k_residual_restrict<T, V, float>, P.count, TileGeo<T>::NT, 0,
+                                   st, S.views[m], P.start, x, b, bc, coff)));
       }
       launches++;
     }

@@ -110,6 +110,8 @@ static __global__ void __launch_bounds__(VEC_BLOCK) k_axpy64_norm(double* __rest
                                                            const float* __restrict__ q, int64_t n,
                                                            const Scalars* __restrict__ s,
                                                            double* __restrict__ partial) {
+  pdl_go();
+  pdl_wait();
   const bool ok = s->status == 0;
   const double alpha = s->alpha;
   const float af = (float)alpha;

@@ -84,11 +84,13 @@ constexpr size_t SMEM = sizeof(float) * ZERO_FLOATS + 3 * sizeof(TileRec) + 3 * 
 template <typename VT>
 __device__ __forceinline__ void halo_load(const LevelView& L, const VT* __restrict__ x,
                                           const VT* __restrict__ xf, const FaceRes& r, int dir,
-                                          int side, int a, int b, VT& xv, float& cv) {
+                                          int side, int a, int b, VT& xv, float& cv,
+                                          int zeroStart = 0) {
   const float* cd = dir == 0 ? L.cx : dir == 1 ? L.cy : L.cz;
   const VT* px = x;
   const float* pc = cd;
-  if (r.kind == FACE_SAME) {
+  const int kind = (zeroStart >> r.kind) & 1 ? FACE_NONE : r.kind;
+  if (kind == FACE_SAME) {
     if (dir == 0 && xf) {
       px = xf + xface_slot(r.nOff, side ? 0 : 1, a, b);
       if (side) pc = L.cxf + (r.nOff >> 4) + a + TS * b;
@@ -96,7 +98,7 @@ __device__ __forceinline__ void halo_load(const LevelView& L, const VT* __restri
       px = x + r.nOff + plane_idx(TS, dir, side ? 0 : TS - 1, a, b);
       if (side) pc = cd + r.nOff + plane_idx(TS, dir, 0, a, b);
     }
-  } else if (r.kind == FACE_COARSER) {
+  } else if (kind == FACE_COARSER) {
     px = x + r.nOff + plane_idx(r.nts, dir, side ? 0 : r.nts - 1, r.oa + (a >> 1), r.ob + (b >> 1));
     pc = L.ifc + r.ifOwn + a + TS * b;
   }
@@ -159,12 +161,15 @@ __device__ __forceinline__ VT* sraw_b(float* st) {
 // thread's own cells, held in registers; 4 of the 6 neighbour values come
 // from shared memory.  The arithmetic per update is that of the reference's
 // order (x-, x+, y-, y+, z-, z+).
-template <typename VT, int NTH>
+// ZERO: the sweep starts from x = 0 (zeroStart, see pressure_kernels.cuh; a variant of its
+// own, since a runtime test in the halo loads costs every sweep 2 %).
+template <typename VT, int NTH, bool ZERO>
 __global__ void __launch_bounds__(NTH, 1)
     k_smooth_pipe16(LevelView L, int tileBase, int count, VT* __restrict__ x,
                     const VT* __restrict__ b, int inner, int reverse, int* __restrict__ err,
-                    VT* __restrict__ xf) {
+                    VT* __restrict__ xf, int zeroFlags) {
   using namespace pipe;
+  const int zeroStart = ZERO ? zeroFlags : 0;
   static_assert(NTH == 1024, "the z-pair thread map covers a 16^3 tile with 1024 threads");
   constexpr int NHALO = 6 * TS * TS;           // halo cells of a tile
   constexpr int HQ = (NHALO + NTH - 1) / NTH;  // halo cells per thread
@@ -179,10 +184,17 @@ __global__ void __launch_bounds__(NTH, 1)
   const int G = gridDim.x;
   int t = blockIdx.x;
   if (t >= count) return;
-  // every float of shared memory holds 0, a value of our (finite) arrays or
-  // two finite 16-bit values (never a float NaN/Inf pattern)
-  for (int q = tid; q < SZERO_FLOATS / 4; q += NTH)
-    reinterpret_cast<float4*>(sm)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+  pdl_go();
+  // a sweep's out-of-tile reads, whose couplings are 0, meet the guard band, the pads of
+  // the x planes or a neighbouring array of the stages: every float there holds 0, a value
+  // of our (finite) arrays or two finite 16-bit values (never a float NaN/Inf pattern)
+  for (int q = tid; q < SGUARD + 2 * TS * 8; q += NTH) {
+    const int w = q - SGUARD;  // pad floats: 8 behind each of a stage's 16 planes
+    if (w < 0)
+      sm[q] = 0.f;
+    else
+      stage(w >> 7)[((w >> 3) & 15) * XP + TS * TS + (w & 7)] = 0.f;
+  }
   // The copies of a stage are issued in parallel, each by lane 0 of its own
   // warp (a bulk copy holds its issuing thread for ~100 cycles): FP32 x
   // plane by plane (warps 0-15) or 16-bit x whole (warp 0), then b, 1/a_ii,
@@ -196,9 +208,11 @@ __global__ void __launch_bounds__(NTH, 1)
     fence_mbar_init();
   }
   __syncthreads();
-  auto issue_arrays = [&](const TileRec& r, float* st, uint64_t* br, int tRec, int slot) {
+  // (vec: x and b; op: the operator and the record)
+  auto issue_arrays = [&](const TileRec& r, float* st, uint64_t* br, int tRec, int slot, bool vec,
+                          bool op) {
     const int w = tid >> 5;
-    if ((tid & 31) != 0 || w >= NISS) return;
+    if ((tid & 31) != 0 || w >= NISS || !(w <= NXC ? vec : op)) return;
     fence_proxy_async();
     const int64_t off = r.off;
     if (w == NISS - 1) {  // the record two tiles ahead, if there is one
@@ -229,6 +243,10 @@ __global__ void __launch_bounds__(NTH, 1)
         default: src = L.cz + off; dst = st + SOFF_C + 2 * N; break;
       }
     }
+    if (w < NXC && (zeroStart & ZERO_OWN)) {
+      mbar_expect_tx(br, 0);
+      return;
+    }
     mbar_expect_tx(br, bytes);
     bulk_g2s(dst, src, bytes, br);
   };
@@ -241,12 +259,16 @@ __global__ void __launch_bounds__(NTH, 1)
     for (int q = 0; q < HQ; q++) {
       const int g = tid + NTH * q, f = g >> 8, c = g & 255;
       if (NHALO % NTH == 0 || g < NHALO)
-        halo_load(L, x, xfr, r.f[f], f >> 1, f & 1, c & 15, c >> 4, hx[q], hc[q]);
+        halo_load(L, x, xfr, r.f[f], f >> 1, f & 1, c & 15, c >> 4, hx[q], hc[q], zeroStart);
     }
   };
   auto halo_combine = [&](const TileRec& r, int ti, int u) {
     float* st = stage(u);
-    if (!WIDE) {
+    if (zeroStart & ZERO_OWN) {
+      // (and, where a 16-bit x would have landed, what the last plane's z + 1 reads meet)
+      for (int e = tid; e < (XS + (WIDE ? 0 : XP)) / 4; e += NTH)
+        reinterpret_cast<float4*>(st)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (!WIDE) {
       const VT* xr = sraw_x<VT>(st);
       for (int e = tid; e < N; e += NTH) st[xpad(e)] = to_f(xr[e]);
     }
@@ -255,7 +277,7 @@ __global__ void __launch_bounds__(NTH, 1)
       const int g = tid + NTH * q, f = g >> 8, c = g & 255;
       if (NHALO % NTH != 0 && g >= NHALO) continue;
       const int dir = f >> 1, side = f & 1, a = c & 15, bb = c >> 4;
-      const int kind = r.f[f].kind;
+      const int kind = (zeroStart >> r.f[f].kind) & 1 ? FACE_NONE : r.f[f].kind;
       float v = 0.f;
       if (kind == FACE_SAME) {
         const float cown = st[SOFF_C + dir * N + plane_idx(TS, dir, 0, a, bb)];
@@ -276,9 +298,12 @@ __global__ void __launch_bounds__(NTH, 1)
   }
   if (!__syncthreads_and(mbar_wait(&bar[2], 0))) {
     if (tid == 0) atomicExch(err, 1);
+    pdl_wait();
     return;
   }
-  issue_arrays(recs[0], stage(0), &bar[0], t + G, 1);
+  issue_arrays(recs[0], stage(0), &bar[0], t + G, 1, false, true);
+  pdl_wait();
+  issue_arrays(recs[0], stage(0), &bar[0], t + G, 1, true, false);
   halo_issue(recs[0]);
   if (!__syncthreads_and(mbar_wait(&bar[0], 0))) {
     if (tid == 0) atomicExch(err, 1);
@@ -302,7 +327,7 @@ __global__ void __launch_bounds__(NTH, 1)
     const TileRec& rn = recs[(n + 1) % 3];
     // 1: prefetch the next tile (arrays + the record two ahead), halo loads
     if (hasNext) {
-      issue_arrays(rn, stage(u), &bar[u], tn + G, (n + 2) % 3);
+      issue_arrays(rn, stage(u), &bar[u], tn + G, (n + 2) % 3, true, true);
       halo_issue(rn);
     }
     // 2: registers: couplings, 1/a_ii, b with the halo sums folded in, and
@@ -505,6 +530,7 @@ __global__ void __launch_bounds__(NTH, 1)
   const int G = gridDim.x;
   int t = blockIdx.x;
   double acc = 0;
+  pdl_go();
   // one issuing thread (lane 0 of its own warp) per copy: x, [b], a_ii,
   // cx, cy, cz, record; the stage barrier counts one arrival each
   constexpr int NISS = NVEC + 5;
@@ -517,9 +543,10 @@ __global__ void __launch_bounds__(NTH, 1)
     }
     __syncthreads();
     // stage arrays: 0 x, 1 b (residual), 2 a_ii, 3..5 couplings
-    auto issue_arrays = [&](const TileRec& r, float* st, uint64_t* br, int tRec, int slot) {
+    auto issue_arrays = [&](const TileRec& r, float* st, uint64_t* br, int tRec, int slot, bool vec,
+                            bool op) {
       const int w = tid >> 5;
-      if ((tid & 31) != 0 || w >= NISS) return;
+      if ((tid & 31) != 0 || w >= NISS || !(w < NVEC ? vec : op)) return;
       fence_proxy_async();
       const int64_t off = r.off;
       if (w == NISS - 1) {
@@ -581,8 +608,10 @@ __global__ void __launch_bounds__(NTH, 1)
       bulk_g2s(&recs[0], grec + t, sizeof(TileRec), &bar[2]);
     }
     bool ok = __syncthreads_and(mbar_wait(&bar[2], 0));
+    if (ok) issue_arrays(recs[0], stage(0), &bar[0], t + G, 1, false, true);
+    pdl_wait();
     if (ok) {
-      issue_arrays(recs[0], stage(0), &bar[0], t + G, 1);
+      issue_arrays(recs[0], stage(0), &bar[0], t + G, 1, true, false);
       halo_issue(recs[0], tileBase + t, 0);
       ok = __syncthreads_and(mbar_wait(&bar[0], 0));
       if (!ok) mbar_wait(&bar[0], 0);
@@ -602,7 +631,7 @@ __global__ void __launch_bounds__(NTH, 1)
       const TileRec& rc = recs[n % 3];
       const TileRec& rn = recs[(n + 1) % 3];
       if (hasNext) {
-        issue_arrays(rn, stage(u), &bar[u], tn + G, (n + 2) % 3);
+        issue_arrays(rn, stage(u), &bar[u], tn + G, (n + 2) % 3, true, true);
         halo_issue(rn, tileBase + tn, u);
       }
       float* X = stage(s);

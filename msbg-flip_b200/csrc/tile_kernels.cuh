@@ -51,6 +51,8 @@ enum {
 // scalar step of PCG that depends on it.
 static __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ partial, int n,
                                                    Scalars* s, int what) {
+  pdl_go();
+  pdl_wait();
   double v = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) v += partial[i];
   v = block_sum(v);
@@ -110,11 +112,18 @@ static __global__ void __launch_bounds__(1024) k_finalize(const double* __restri
 // partial sums are deterministic)
 // ---------------------------------------------------------------------------
 constexpr int VEC_GRID = 148 * 4, VEC_BLOCK = 512;
+// Dependent launches (common.cuh) of the vector kernels and their scalar steps: where they
+// are short.  On long vectors an early start of the next kernel takes from the running one:
+// a solve of 167 M cells took 148.9 ms with them, 145.9 without (B200); one of 64^3, whose
+// kernels take 2-4 us, 1.48 against 1.78 ms.
+inline bool vectors_dependent(int64_t n) { return n <= (8 << 20); }
 
 template <typename VA, typename VB>
 __global__ void __launch_bounds__(VEC_BLOCK) k_dot(const VA* __restrict__ a,
                                                    const VB* __restrict__ b, int64_t n,
                                                    double* __restrict__ partial) {
+  pdl_go();
+  pdl_wait();
   double acc = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n >> 2);
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -132,6 +141,8 @@ __global__ void __launch_bounds__(VEC_BLOCK) k_axpy_norm(VT* __restrict__ x, VT*
                                                          const VT* __restrict__ q, int64_t n,
                                                          const Scalars* __restrict__ s,
                                                          double* __restrict__ partial) {
+  pdl_go();
+  pdl_wait();
   const bool ok = s->status == 0;
   const float alpha = (float)s->alpha;
   double acc = 0;
@@ -160,6 +171,8 @@ template <typename VT>
 __global__ void __launch_bounds__(VEC_BLOCK) k_update_d(VT* __restrict__ d,
                                                         const VT* __restrict__ z, int64_t n,
                                                         const Scalars* __restrict__ s) {
+  pdl_go();
+  pdl_wait();
   if (s->status) return;
   const float beta = (float)s->beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n >> 2);
@@ -209,10 +222,10 @@ struct TileGeo {
 template <int TS, typename VT>
 __device__ __forceinline__ float halo_term(const LevelView& L, const TileRec& r, int ti,
                                            const VT* __restrict__ x, int dir, int side, int a,
-                                           int b) {
+                                           int b, int zeroStart) {
   const FaceRes& F = r.f[2 * dir + side];
   const int kind = F.kind;
-  if (kind == FACE_NONE) return 0.f;
+  if (kind == FACE_NONE || ((zeroStart >> kind) & 1)) return 0.f;
   const float* cd = dir == 0 ? L.cx : dir == 1 ? L.cy : L.cz;
   if (kind == FACE_SAME)
     return cd[(side ? F.nOff : r.off) + plane_idx(TS, dir, 0, a, b)] *
@@ -231,8 +244,8 @@ template <int TS, typename VT>
 struct TileCells {
   using G = TileGeo<TS>;
   float c[G::PER][6];
-  __device__ __forceinline__ void load(const LevelView& L, const TileRec& r, int ti,
-                                       const VT* __restrict__ x, float* xs) {
+  // the couplings; then, once x is there, x and the halo
+  __device__ __forceinline__ void load(const LevelView& L, const TileRec& r) {
     const int t = threadIdx.x;
     const float* cx = L.cx + r.off;
     const float* cy = L.cy + r.off;
@@ -248,13 +261,23 @@ struct TileCells {
       c[q][3] = j < TS - 1 ? cy[e + TS] : 1.f;
       c[q][4] = k > 0 ? cz[e] : 1.f;
       c[q][5] = k < TS - 1 ? cz[e + TS * TS] : 1.f;
-      xs[G::pad(i, j, k)] = to_f(x[r.off + e]);
+    }
+  }
+  __device__ __forceinline__ void load_x(const LevelView& L, const TileRec& r, int ti,
+                                         const VT* __restrict__ x, float* xs, int zeroStart = 0) {
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < G::PER; q++) {
+      const int e = t + G::NT * q;
+      if (e < G::N)
+        xs[G::pad(e % TS, (e / TS) % TS, e / (TS * TS))] =
+            zeroStart & ZERO_OWN ? 0.f : to_f(x[r.off + e]);
     }
     for (int h = t; h < 6 * TS * TS; h += G::NT) {
       const int f = h / (TS * TS), a = h % TS, b = (h / TS) % TS, dir = f >> 1, side = f & 1;
       const int p = side ? TS : -1;
       xs[dir == 0 ? G::pad(p, a, b) : dir == 1 ? G::pad(a, p, b) : G::pad(a, b, p)] =
-          halo_term<TS>(L, r, ti, x, dir, side, a, b);
+          halo_term<TS>(L, r, ti, x, dir, side, a, b, zeroStart);
     }
   }
   // in the order x-, x+, y-, y+, z-, z+
@@ -280,11 +303,14 @@ __global__ void __launch_bounds__(TileGeo<TS>::NT) k_matvec_dot(LevelView L, int
   __shared__ float xs[G::P * G::P * G::P];
   const int ti = tileBase + blockIdx.x, t = threadIdx.x;
   const TileRec& r = reinterpret_cast<const TileRec*>(L.tileRec)[ti];
+  pdl_go();
   TileCells<TS, VT> C;
-  C.load(L, r, ti, d, xs);
+  C.load(L, r);
   float dg[G::PER];
 #pragma unroll
   for (int p = 0; p < G::PER; p++) dg[p] = t + G::NT * p < G::N ? L.diag[r.off + t + G::NT * p] : 0.f;
+  pdl_wait();
+  C.load_x(L, r, ti, d, xs);
   __syncthreads();
   double acc = 0;
 #pragma unroll
@@ -313,8 +339,9 @@ __global__ void __launch_bounds__(TileGeo<TS>::NT)
   __shared__ float rs[G::N];
   const int ti = tileBase + blockIdx.x, t = threadIdx.x;
   const TileRec& r = reinterpret_cast<const TileRec*>(L.tileRec)[ti];
+  pdl_go();
   TileCells<TS, VT> C;
-  C.load(L, r, ti, x, xs);
+  C.load(L, r);
   const int* tc = L.toCoarse + (size_t)ti * 6;
   const int ct = tc[0], ox = tc[1], oy = tc[2], oz = tc[3], agg = tc[4], cts = tc[5];
   VC* dst = ct >= 0 ? bc + coarseOff[ct] : nullptr;
@@ -323,8 +350,12 @@ __global__ void __launch_bounds__(TileGeo<TS>::NT)
   for (int p = 0; p < G::PER; p++) {
     const int e = t + G::NT * p;
     dg[p] = e < G::N ? L.diag[r.off + e] : 0.f;
-    bv[p] = e < G::N ? to_f(b[r.off + e]) : 0.f;
   }
+  pdl_wait();
+#pragma unroll
+  for (int p = 0; p < G::PER; p++)
+    bv[p] = t + G::NT * p < G::N ? to_f(b[r.off + t + G::NT * p]) : 0.f;
+  C.load_x(L, r, ti, x, xs);
   __syncthreads();
   if (!dst) return;
 #pragma unroll
@@ -373,10 +404,12 @@ __global__ void __launch_bounds__(TS* TS) k_prolong(LevelView L, const int* __re
                                                     const int64_t* __restrict__ coarseOff,
                                                     float scale, VT* __restrict__ xf) {
   constexpr int N = TS * TS * TS, NT = TS * TS;
+  pdl_go();
   const int ti = tiles[blockIdx.x];
   const int64_t off = L.tileOff[ti];
   const int* tc = L.toCoarse + (size_t)ti * 6;
   const int ct = tc[0], ox = tc[1], oy = tc[2], oz = tc[3], agg = tc[4], cts = tc[5];
+  pdl_wait();
   if (ct < 0) return;
   const VC* src = xc + coarseOff[ct];
   const int sh = agg ? 1 : 0;
@@ -426,18 +459,19 @@ __global__ void __launch_bounds__(TS* TS) k_prolong(LevelView L, const int* __re
 
 // Red-black Gauss-Seidel inside tiles tileBase.., `inner` iterations, ghosts
 // frozen at their values when the tile is loaded.  reverse=0: red then black;
-// reverse=1: black then red (the adjoint order).
+// reverse=1: black then red (the adjoint order).  zeroStart: see pressure_kernels.cuh.
 template <int TS, typename VT>
 __global__ void __launch_bounds__(TileGeo<TS>::NT) k_smooth(LevelView L, int tileBase,
                                                             VT* __restrict__ x,
                                                             const VT* __restrict__ b, int inner,
-                                                            int reverse) {
+                                                            int reverse, int zeroStart) {
   using G = TileGeo<TS>;
   __shared__ float xs[G::P * G::P * G::P];
   const int ti = tileBase + blockIdx.x, t = threadIdx.x;
   const TileRec& r = reinterpret_cast<const TileRec*>(L.tileRec)[ti];
+  pdl_go();
   TileCells<TS, VT> C;
-  C.load(L, r, ti, x, xs);
+  C.load(L, r);
   float inv[G::PER], bb[G::PER];
   int col[G::PER], at[G::PER];
 #pragma unroll
@@ -445,10 +479,14 @@ __global__ void __launch_bounds__(TileGeo<TS>::NT) k_smooth(LevelView L, int til
     const int e = t + G::NT * p;
     const int i = e % TS, j = (e / TS) % TS, k = e / (TS * TS);
     inv[p] = e < G::N ? L.invdiag[r.off + e] : 0.f;
-    bb[p] = e < G::N ? to_f(b[r.off + e]) : 0.f;
     col[p] = (i + j + k) & 1;
     at[p] = e < G::N ? G::pad(i, j, k) : G::pad(0, 0, 0);
   }
+  pdl_wait();
+#pragma unroll
+  for (int p = 0; p < G::PER; p++)
+    bb[p] = t + G::NT * p < G::N ? to_f(b[r.off + t + G::NT * p]) : 0.f;
+  C.load_x(L, r, ti, x, xs, zeroStart);
   __syncthreads();
   for (int it = 0; it < inner; it++) {
 #pragma unroll
@@ -478,6 +516,8 @@ __global__ void __launch_bounds__(COARSE_ROWS* COARSE_PARTS)
   __shared__ double part[COARSE_PARTS][COARSE_ROWS];
   const int t = threadIdx.x, r = t % COARSE_ROWS, q = t / COARSE_ROWS;
   const int row = blockIdx.x * COARSE_ROWS + r;
+  pdl_go();
+  pdl_wait();
   for (int i = t; i < n; i += COARSE_ROWS * COARSE_PARTS) bs[i] = to_f(b[cells[i]]);
   __syncthreads();
   double s = 0;
