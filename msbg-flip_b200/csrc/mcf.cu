@@ -211,11 +211,17 @@ __device__ __forceinline__ void mcf_fill(float* tile, const T* __restrict__ pool
     }
   }
   // shell voxels with x inside the block (z faces, y faces, x-direction
-  // edges): the ring of (y, z) around the block, one x pair each
-  constexpr int RING = 4 * BSX + 4;
-  for (int q = tid; q < RING * HP; q += NT) {
-    const int r = q / HP, x = 2 * (q % HP);
-    int y, z;
+  // edges): the ring of (y, z) around the block, one x pair each; and with x = -1
+  // or x = BSX (x faces, y- and z-direction edges): (y, z) in [-1, BSX]^2 without
+  // the four corners, one voxel each.  16-bit values are all loaded before any is
+  // stored, so a thread waits for its shell once.
+  constexpr int RING = 4 * BSX + 4, RQ = (RING * HP + NT - 1) / NT;
+  constexpr int SIDE = (BSX + 2) * (BSX + 2), SQ = (2 * SIDE + NT - 1) / NT;
+  uint32_t rv[F32 ? 1 : RQ];
+  T sv[F32 ? 1 : SQ];
+  const auto ring_at = [](int q, int& x, int& y, int& z) {
+    const int r = q / HP;
+    x = 2 * (q % HP);
     if (r < 2 * (BSX + 2)) {  // z = -1 and z = BSX, y in [-1, BSX]
       z = r < BSX + 2 ? -1 : BSX;
       y = (r % (BSX + 2)) - 1;
@@ -224,41 +230,71 @@ __device__ __forceinline__ void mcf_fill(float* tile, const T* __restrict__ pool
       y = r2 < BSX ? -1 : BSX;
       z = r2 % BSX;
     }
-    int ck;
+  };
+  const auto side_at = [](int q, int& x, int& y, int& z) {
+    const int r = q % SIDE;
+    x = q / SIDE ? BSX : -1;
+    y = r % (BSX + 2) - 1;
+    z = r / (BSX + 2) - 1;
+    return !((y < 0 || y >= BSX) && (z < 0 || z >= BSX));  // a corner is not read
+  };
+  uint32_t rc = 0, sc = 0;  // where a const value stands instead: bit 2k empty, 2k + 1 full
+  static_assert(2 * RQ <= 32 && 2 * SQ <= 32, "a bit pair per value");
+#pragma unroll(F32 ? 1 : RQ)
+  for (int k = 0; k < RQ; k++) {
+    const int q = tid + NT * k;
+    if (q >= RING * HP) break;
+    int x, y, z, ck;
+    ring_at(q, x, y, z);
     const T* src = halo_src<BSX, T>(pool, nbSlot, own, x, y, z, ck);
-    float* d = tile + Tl::at(x, y, z);
-    if (src) {
-      if constexpr (F32) {
+    if constexpr (F32) {
+      float* d = tile + Tl::at(x, y, z);
+      if (src)
         cp_async8(d, src);
-      } else {
-        const uint32_t v = *reinterpret_cast<const uint32_t*>(src);
-        d[0] = (float)(v & 0xffffu) * U16_SCALE;
-        d[1] = (float)(v >> 16) * U16_SCALE;
-      }
+      else
+        d[0] = d[1] = ck == 1 ? emptyVal : fullVal;
     } else {
-      const float v = ck == 1 ? emptyVal : fullVal;
-      d[0] = v;
-      d[1] = v;
+      rc |= (uint32_t)ck << (2 * k);
+      if (src) rv[k] = *reinterpret_cast<const uint32_t*>(src);
     }
   }
-  // shell voxels with x = -1 or x = BSX (x faces, y- and z-direction edges):
-  // (y, z) in [-1, BSX]^2 without the four corners, one voxel each
-  constexpr int SIDE = (BSX + 2) * (BSX + 2);
-  for (int q = tid; q < 2 * SIDE; q += NT) {
-    const int side = q / SIDE, r = q % SIDE;
-    const int y = r % (BSX + 2) - 1, z = r / (BSX + 2) - 1;
-    if ((y < 0 || y >= BSX) && (z < 0 || z >= BSX)) continue;  // corner: not read
-    const int x = side ? BSX : -1;
-    int ck;
+#pragma unroll(F32 ? 1 : SQ)
+  for (int k = 0; k < SQ; k++) {
+    const int q = tid + NT * k;
+    int x, y, z, ck;
+    if (q >= 2 * SIDE || !side_at(q, x, y, z)) continue;
     const T* src = xface_src<BSX, T>(pool, xf, nbSlot, x, y, z, ck);
-    float* d = tile + Tl::at(x, y, z);
-    if (src) {
-      if constexpr (F32)
+    if constexpr (F32) {
+      float* d = tile + Tl::at(x, y, z);
+      if (src)
         cp_async4(d, src);
       else
-        *d = (float)(*src) * U16_SCALE;
+        *d = ck == 1 ? emptyVal : fullVal;
     } else {
-      *d = ck == 1 ? emptyVal : fullVal;
+      sc |= (uint32_t)ck << (2 * k);
+      if (src) sv[k] = *src;
+    }
+  }
+  if constexpr (!F32) {
+#pragma unroll
+    for (int k = 0; k < RQ; k++) {
+      const int q = tid + NT * k;
+      if (q >= RING * HP) break;
+      int x, y, z;
+      ring_at(q, x, y, z);
+      const uint32_t ck = (rc >> (2 * k)) & 3;
+      const float cv = ck == 1 ? emptyVal : fullVal;
+      float* d = tile + Tl::at(x, y, z);
+      d[0] = ck ? cv : (float)(rv[k] & 0xffffu) * U16_SCALE;
+      d[1] = ck ? cv : (float)(rv[k] >> 16) * U16_SCALE;
+    }
+#pragma unroll
+    for (int k = 0; k < SQ; k++) {
+      const int q = tid + NT * k;
+      int x, y, z;
+      if (q >= 2 * SIDE || !side_at(q, x, y, z)) continue;
+      const uint32_t ck = (sc >> (2 * k)) & 3;
+      tile[Tl::at(x, y, z)] = ck ? (ck == 1 ? emptyVal : fullVal) : (float)sv[k] * U16_SCALE;
     }
   }
 }
@@ -403,8 +439,10 @@ __global__ void __launch_bounds__(BSX* BSX, mcf_ctas_per_sm<BSX>())
       mcf_fill<BSX, T>(tiles + s * TILE, pool, xf, nbSlot[s], emptyVal, fullVal, tid);
     cp_async_commit();
   };
-  neighbours(k, 0);
+  pdl_go();
+  neighbours(k, 0);  // (the block list and slots are not written by a pass)
   __syncthreads();
+  pdl_wait();
   fill(0);
   for (int it = 0; k < n; it++, k += G) {
     const int s = ST == 2 ? (it & 1) : 0;
@@ -648,9 +686,11 @@ __global__ void __launch_bounds__(256, 3)
     cp_async_commit();
     halo_load(h, pool, xf, nbSlot[s], emptyVal, fullVal, tid);
   };
+  pdl_go();
   __syncthreads();  // barriers initialised
-  neighbours(k, 0);
+  neighbours(k, 0);  // (the block list and slots are not written by a pass)
   __syncthreads();
+  pdl_wait();
   issue(0);
   for (int it = 0; k < n; it++, k += G) {
     const int s = it & 1;
@@ -689,6 +729,7 @@ template <int BSX, typename T>
 __global__ void __launch_bounds__(256) k_mcf_xfaces(const T* __restrict__ pool, int64_t nSlots,
                                                     T* __restrict__ xf) {
   constexpr int F = BSX * BSX;
+  pdl_go();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nSlots * 2 * F;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t sl = i / (2 * F);
@@ -772,21 +813,25 @@ cudaError_t launch_mcf_t(T* pool, T* xf, int64_t nSlots, const int* slotOf,
         for (int c = 0; c < 8; c++) {
           const int n = colourStart[c + 1] - colourStart[c];
           if (n <= 0) continue;
-          mcf_colour_kernel_tma<<<std::min(n, maxGrid), tma::Tl::NT, tma::SMEM, stream>>>(
-              map, pool, xf, slotOf, colourList + colourStart[c], n, nbx, nby, nbz, emptyVal,
-              fullVal, dt, clamp01, errFlag);
+          launch(mcf_colour_kernel_tma, std::min(n, maxGrid), tma::Tl::NT, tma::SMEM, stream, map,
+                 pool, xf, slotOf, colourList + colourStart[c], n, nbx, nby, nbz, emptyVal,
+                 fullVal, dt, clamp01, errFlag);
         }
       return cudaGetLastError();
     }
   }
+  // (the caller's own kernels may write the pool, the slots and the list: the first pass
+  // waits for them before it starts)
+  bool dependent = xf && nSlots > 0;
   for (int it = 0; it < nIter; it++)
     for (int c = 0; c < 8; c++) {
       int n = colourStart[c + 1] - colourStart[c];
       if (n <= 0) continue;
       const int grid = mcf_stages<BSX>() == 2 ? std::min(n, maxGrid) : n;
-      mcf_colour_kernel<BSX, T><<<grid, Tl::NT, Tl::SMEM * mcf_stages<BSX>(), stream>>>(
-          pool, xf, slotOf, colourList + colourStart[c], n, nbx, nby, nbz, emptyVal, fullVal, dt,
-          clamp01, errFlag);
+      launch_if(dependent, mcf_colour_kernel<BSX, T>, grid, Tl::NT, Tl::SMEM * mcf_stages<BSX>(), stream, pool,
+             xf, slotOf, colourList + colourStart[c], n, nbx, nby, nbz, emptyVal, fullVal, dt,
+             clamp01, errFlag);
+      dependent = true;
     }
   return cudaGetLastError();
 }
