@@ -175,3 +175,30 @@ def test_splat_then_smoother_matches_reference_pipeline():
     d = np.abs(got.astype(np.int64) - ref.astype(np.int64))
     assert (ref != g["final"]).any()
     assert d.max() <= 2 and (d > 0).mean() <= 2e-3, (int(d.max()), float((d > 0).mean()))
+
+
+@pytest.mark.parametrize("bsx", [8, 16, 32])
+@pytest.mark.parametrize("r_particle,nb_dist", [(2.0, 2.0), (1.25, 0.7), (2.6, 2.1)])
+def test_gpu_dense_clumps_and_reaches(bsx, r_particle, nb_dist):
+    """Dense clumps (several chunks of particles around a block, and blocks with a few) across
+    block borders and the domain's edges, for reaches up to and above 4 voxels, with kinds that
+    stop some scans."""
+    res3 = (96, 64, 128)
+    rng = np.random.default_rng(17)
+    ctr = rng.uniform(0, 1, (6, 3)) * np.array(res3)
+    ctr[0] = [0.5, 0.5, 0.5]
+    ctr[1] = [95.5, 31.9, 64.1]
+    pos = np.concatenate([c + rng.normal(0, 2.5, (4000, 3)) for c in ctr] +
+                         [rng.uniform(0, 1, (500, 3)) * np.array(res3)])
+    pos[:200] = np.round(pos[:200] * 2) / 2
+    pos = np.clip(pos, 0.0, np.array(res3) - 1e-3).astype(np.float32)
+    kw = dict(r_particle=r_particle, nb_dist=nb_dist)
+    k, fin = gpu_splat(res3, bsx, pos, **kw)
+    act = oracle.splat_mark(res3, bsx, pos, r_particle, nb_dist)
+    assert np.array_equal(k == 1, act == 1)
+    assert np.array_equal(fin, oracle.splat(res3, bsx, act, pos, r_particle, nb_dist))
+    kind = np.where(act == 1, 1, 2).astype(np.int8)
+    drop = np.nonzero(act == 1)[0]
+    kind[rng.choice(drop, len(drop) // 5, replace=False)] = 2
+    _, fin = gpu_splat(res3, bsx, pos, kind=kind, **kw)
+    assert np.array_equal(fin, oracle.splat(res3, bsx, kind, pos, r_particle, nb_dist))
