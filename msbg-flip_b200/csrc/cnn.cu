@@ -205,6 +205,23 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3_tc(const __grid_const
             mma_bf16(c + (uint32_t)(256 * xh), az + (uint64_t)((t / 3) * PD + 8 * xh + t % 3),
                      bz + (uint64_t)(t * 96), idAll, 1u);
       };
+      // the next plane, and a first look at its barriers: the answer comes while the
+      // MMAs below are issued
+      const int pz = zi, pl = l, pslot = slot;
+      if (l == 0 && ++slot == CONV_SLOTS) {
+        slot = 0;
+        slotPar ^= 1u;
+      }
+      int np = p, nl = l, nz = zi + 1;
+      if (nz > (l > 0 ? TS : TS + 1)) {
+        np++;
+        nl = l + 1 == a.nl ? 0 : l + 1;
+        nz = nl > 0;
+      }
+      const bool more = np < passes, inside = np == p;
+      bool seen = inside;
+      if (inside && p > 0 && nz < TS) seen = mbar_test(&stored[nz], (uint32_t)((p - 1) & 1));
+      if (inside && l == 0) seen = mbar_test(&full[slot], slotPar) && seen;
       if (elect_one()) {
 #pragma unroll
         for (int xh = 0; xh < 2; xh++)
@@ -218,25 +235,16 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3_tc(const __grid_const
         taps(std::integral_constant<int, 1>{}, std::integral_constant<int, 5>{});
       }
       __syncwarp();
-      // the next plane's waits, while these MMAs run
-      const int pz = zi, pl = l, pslot = slot;
-      if (l == 0 && ++slot == CONV_SLOTS) {
-        slot = 0;
-        slotPar ^= 1u;
-      }
       // the previous pass is done with its weights: those of the next one
-      if (zi == 6 && p > 0 && wl < passes) {
+      if (pz == 6 && p > 0 && wl < passes) {
         if (!(ok = wait(&done[PD - 1], (uint32_t)((p - 1) & 1)))) break;
         load_weights(wl++, wlL);
         wlL = wlL + 1 == a.nl ? 0 : wlL + 1;
       }
-      if (++zi > (l > 0 ? TS : TS + 1)) {
-        p++;
-        l = l + 1 == a.nl ? 0 : l + 1;
-        zi = l > 0;
-      }
-      const bool more = p < passes;
-      if (more && !(ok = ready(p, l, zi))) break;
+      p = np;
+      l = nl;
+      zi = nz;
+      if (!__all_sync(0xffffffffu, seen) && more && !(ok = ready(p, l, zi))) break;
       if (elect_one()) {
         taps(std::integral_constant<int, 5>{}, std::integral_constant<int, 9>{});
         if (pz > 1) mma_commit(&done[pz]);  // (no output plane completes before)
