@@ -66,24 +66,89 @@ enum : int {
   MCF_ERR_NOT_VALUE = 2   // a listed block is not a value block; it was skipped
 };
 
+// Device blocks on their way from one owner to the next.  While a PoolScope is open on a
+// thread, buffers that it releases there go to the scope's pool, and buffers that need memory
+// look there first (a block of at most 1/4 more than asked for); what is left is freed when
+// the scope closes, or before an allocation fails.  For work on one stream: a block may still
+// be read by what its last owner has issued there.
+class DevicePool {
+ public:
+  ~DevicePool() { clear(); }
+  void clear() {
+    for (auto& b : blocks_) cudaFree(b.second);
+    blocks_.clear();
+  }
+  void give(void* p, size_t cap) { blocks_.emplace(cap, p); }
+  void* take(size_t n, size_t& cap) {
+    auto it = blocks_.lower_bound(n);
+    if (it == blocks_.end() || it->first > n + n / 4 + 4096) return nullptr;
+    void* p = it->second;
+    cap = it->first;
+    blocks_.erase(it);
+    return p;
+  }
+  static DevicePool*& current() {
+    static thread_local DevicePool* c = nullptr;
+    return c;
+  }
+
+ private:
+  std::multimap<size_t, void*> blocks_;
+};
+class PoolScope {
+ public:
+  PoolScope() : before_(DevicePool::current()) { DevicePool::current() = &pool_; }
+  ~PoolScope() { DevicePool::current() = before_; }
+  PoolScope(const PoolScope&) = delete;
+  PoolScope& operator=(const PoolScope&) = delete;
+
+ private:
+  DevicePool* before_;
+  DevicePool pool_;
+};
+
 struct DeviceBuffer {
   void* p = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0;  // asked for
+  size_t cap = 0;    // of the block
   DeviceBuffer() = default;
   DeviceBuffer(const DeviceBuffer&) = delete;
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
   ~DeviceBuffer() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p) {
+      if (DevicePool* pool = DevicePool::current())
+        pool->give(p, cap);
+      else
+        cudaFree(p);
+    }
     p = nullptr;
-    bytes = 0;
+    bytes = cap = 0;
   }
   cudaError_t ensure(size_t n) {
-    if (n <= bytes && p) return cudaSuccess;
+    if (n <= cap && p) {
+      if (n > bytes) bytes = n;
+      return cudaSuccess;
+    }
     release();
-    cudaError_t e = cudaMalloc(&p, n ? n : 16);
-    if (e == cudaSuccess) bytes = n;
-    return e;
+    const size_t want = n ? n : 16;
+    DevicePool* pool = DevicePool::current();
+    if (pool) p = pool->take(want, cap);
+    if (!p) {
+      cudaError_t e = cudaMalloc(&p, want);
+      if (e != cudaSuccess && pool) {  // what the last owner left makes room
+        cudaGetLastError();
+        pool->clear();
+        e = cudaMalloc(&p, want);
+      }
+      if (e != cudaSuccess) {
+        p = nullptr;
+        return e;
+      }
+      cap = want;
+    }
+    bytes = n;
+    return cudaSuccess;
   }
   template <typename T>
   T* as() const { return reinterpret_cast<T*>(p); }
@@ -93,8 +158,9 @@ struct DeviceBuffer {
     release();
     p = o.p;
     bytes = o.bytes;
+    cap = o.cap;
     o.p = nullptr;
-    o.bytes = 0;
+    o.bytes = o.cap = 0;
   }
 };
 

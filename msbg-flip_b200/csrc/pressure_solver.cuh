@@ -31,6 +31,12 @@ namespace ps {
 // solver state
 // ---------------------------------------------------------------------------
 struct Solver {
+  Solver() = default;
+  Solver(const Solver&) = delete;
+  Solver& operator=(const Solver&) = delete;
+  ~Solver() {
+    if (hScal) cudaFreeHost(hScal);
+  }
   Hierarchy H;
   int64_t h2dBytes = 0;
   int numSMs = 148;
