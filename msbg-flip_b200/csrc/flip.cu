@@ -53,17 +53,19 @@ struct GridF {
   __device__ __forceinline__ int64_t idx(int x, int y, int z) const {
     if (x < 0 || y < 0 || z < 0 || x >= sx || y >= sy || z >= sz) return -1;
     const int m = (1 << sh) - 1;
-    const int64_t bid = (x >> sh) + (int64_t)nbx * ((y >> sh) + (int64_t)nby * (z >> sh));
-    return (bid << (3 * sh)) + (x & m) + ((int64_t)(y & m) << sh) + ((int64_t)(z & m) << (2 * sh));
+    // (block ids are ints: 64 bits only for the voxel)
+    const int bid = (x >> sh) + nbx * ((y >> sh) + nby * (z >> sh));
+    return ((int64_t)bid << (3 * sh)) + ((x & m) + ((y & m) << sh) + ((z & m) << (2 * sh)));
   }
   // voxel coordinates of block-layout index i
   __device__ __forceinline__ void coords(int64_t i, int& x, int& y, int& z) const {
     const int m = (1 << sh) - 1;
-    const int64_t bid = i >> (3 * sh);
+    const unsigned bid = (unsigned)(i >> (3 * sh));
     const int v = (int)(i & ((1 << (3 * sh)) - 1));
-    x = (int)(bid % nbx) * (1 << sh) + (v & m);
-    y = (int)((bid / nbx) % nby) * (1 << sh) + ((v >> sh) & m);
-    z = (int)(bid / ((int64_t)nbx * nby)) * (1 << sh) + (v >> (2 * sh));
+    const unsigned row = bid / (unsigned)nbx, bz = row / (unsigned)nby;
+    x = (int)(bid - row * nbx) * (1 << sh) + (v & m);
+    y = (int)(row - bz * nby) * (1 << sh) + ((v >> sh) & m);
+    z = (int)bz * (1 << sh) + (v >> (2 * sh));
   }
 };
 

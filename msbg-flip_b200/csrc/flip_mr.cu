@@ -68,9 +68,9 @@ struct MrGrid {
     if (x < 0 || y < 0 || z < 0 || x >= (sx >> lv) || y >= (sy >> lv) || z >= (sz >> lv))
       return -1;
     const int sh = sh0 - lv, m = (1 << sh) - 1;
-    const int64_t b = (x >> sh) + (int64_t)nbx * ((y >> sh) + (int64_t)nby * (z >> sh));
+    const int b = (x >> sh) + nbx * ((y >> sh) + nby * (z >> sh));
     if (level[b] != lv) return -1;
-    return off[b] + (x & m) + ((int64_t)(y & m) << sh) + ((int64_t)(z & m) << (2 * sh));
+    return off[b] + ((x & m) + ((y & m) << sh) + ((z & m) << (2 * sh)));
   }
 };
 
