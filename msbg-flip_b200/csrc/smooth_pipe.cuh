@@ -159,8 +159,10 @@ __device__ __forceinline__ VT* sraw_b(float* st) {
 // z = 2kp + {0,1} of row jj: per colour one cell of each z plane, and for
 // each of them the x- and the z-neighbour of the other colour are the
 // thread's own cells, held in registers; 4 of the 6 neighbour values come
-// from shared memory.  The arithmetic per update is that of the reference's
-// order (x-, x+, y-, y+, z-, z+).
+// from shared memory.  A cell's terms are added own x, other x, y-, y+, own z, other z (own:
+// the neighbour inside the thread's block), which needs no select: the sweeps are bound by
+// instructions issued, and with the order x-, x+, y-, y+, z-, z+ a quarter of them were
+// selects by the cell's place in its pair (1.091 -> 1.021 ms a sweep of 167 M cells, B200).
 // ZERO: the sweep starts from x = 0 (zeroStart, see pressure_kernels.cuh; a variant of its
 // own, since a runtime test in the halo loads costs every sweep 2 %).
 template <typename VT, int NTH, bool ZERO>
@@ -401,33 +403,33 @@ __global__ void __launch_bounds__(NTH, 1)
         }
       }
     }
-    // 3: red-black sweeps (colour compile-time so the arrays stay in registers)
+    // 3: red-black sweeps (colour compile-time so the arrays stay in registers).  The cell
+    // of colour c in plane s is the x pair's cell q where c == s, else the other one.
+    if (q) {
+      const float cz = Czp[0];
+      Czp[0] = Czp[1];
+      Czp[1] = cz;
+    }
+    const int eq[2] = {eb + q, eb + 1 - q};        // by c != s
+    const int xo_[2] = {q ? 1 : -1, q ? -1 : 1};  // and where the x neighbour beyond lies
     auto half = [&](auto cc) {
       constexpr int c = decltype(cc)::value;
 #pragma unroll
       for (int sl = 0; sl < 2; sl++) {
-        const int dx = dxof(c, sl);
-        const int e = eb + dx + XP * sl;
+        constexpr int A = c;
+        const int w = A == sl ? 0 : 1;
+        const int e = eq[w] + XP * sl;
         // the x-neighbour of the other colour inside the pair is ours; the
         // one beyond is read (out-of-tile reads have zero coupling and stay
-        // inside shared memory: guard band, pads, adjacent arrays)
-        const float xo = X[dx ? e + 1 : e - 1], xs = xv[1 - c][sl];
-        // z: plane 2kp reads z-1 and owns z+1; plane 2kp+1 the reverse
-        const float zo = X[sl ? e + XP : e - XP], zs = xv[1 - c][1 - sl];
-        const float czs = dx ? Czp[1] : Czp[0];
-        // terms in the order x-, x+, y-, y+, z-, z+
+        // inside shared memory: guard band, pads, adjacent arrays); plane 2kp reads z-1
+        // and owns z+1, plane 2kp+1 the reverse
         float S = R[c][sl];
-        S = fmaf(dx ? Cxp[sl] : Cxo[c][sl], dx ? xs : xo, S);
-        S = fmaf(dx ? Cxo[c][sl] : Cxp[sl], dx ? xo : xs, S);
+        S = fmaf(Cxp[sl], xv[1 - c][sl], S);
+        S = fmaf(Cxo[c][sl], X[e + xo_[w]], S);
         S = fmaf(Cym[c][sl], X[e - TS], S);
         S = fmaf(Cyp[c][sl], X[e + TS], S);
-        if (sl) {
-          S = fmaf(czs, zs, S);
-          S = fmaf(Czo[c][sl], zo, S);
-        } else {
-          S = fmaf(Czo[c][sl], zo, S);
-          S = fmaf(czs, zs, S);
-        }
+        S = fmaf(Czp[w], xv[1 - c][1 - sl], S);
+        S = fmaf(Czo[c][sl], X[sl ? e + XP : e - XP], S);
         xv[c][sl] = S * I[c][sl];
         X[e] = xv[c][sl];
       }
