@@ -399,24 +399,28 @@ __global__ void __launch_bounds__(256, 4) k_splat_blocks(SplatGeom g, const int*
 // eighth of a 32^3 block).  The particles of the 27 bins that reach the cube come in chunks
 // of up to CHUNK; a chunk is sorted by cell in shared memory (a cell: a voxel's unit cube;
 // W^3 of them, the cube and 4 around it), and every voxel searches the cells around it for
-// a particle nearer than its best: plane by plane and row by row outwards, skipping planes,
-// rows and cells that are empty or whose nearest point is no nearer.  All cells of a row
-// within reach are one run of the sorted chunk.
+// a particle nearer than its best: plane by plane and row by row outwards, skipping what is
+// empty or no nearer.  All cells of a row within reach are one run of the sorted chunk (cell by
+// cell outwards the loop costs more than the particles it saves).  In the case below 3 of 4
+// voxels have no particle in reach and the others meet 57, but a voxel visits 61 rows:
+// bit masks of the rows, planes and voxels with particles in reach make those one test.
 // The distances are those of k_splat_blocks: a particle of cell c has |x - p| >= |c - x| - 1/2
 // exactly (both differences are exact), so nothing that could lower the minimum is skipped.
 // The scan box and a scan that stops early matter only at the edge of the reach and for marked
 // particles; those look the particle up again.
 // The demo's 4096 x 4096 particles at 1024^3 (B200): 28.4 ms a call with particles visiting
-// voxels everywhere, 14.2 with this kernel.  (Chunks of 4096 spill registers: 17.2 ms.)
+// voxels everywhere, 13.1 with this kernel but masks of the occupied rows alone, 10.4 now
+// that only the voxels with a cell in reach are searched.
 constexpr int CUBE_T = 512, CHUNK = 2048;
 
 template <int CUBE>
 struct SplatCube {
   static constexpr int R = 4, W = CUBE + 2 * R, CELLS = W * W * W;
   static constexpr int PER = (CELLS + CUBE_T - 1) / CUBE_T;  // cells per thread of the scan
-  static constexpr int VOX = CUBE * CUBE * CUBE / CUBE_T;    // voxels per thread
-  static constexpr size_t SMEM =
-      sizeof(float4) * CHUNK + sizeof(uint32_t) * (W * W + W) + sizeof(uint16_t) * (CELLS + 2);
+  static constexpr int VOX = CUBE * CUBE * CUBE;             // voxels
+  static constexpr size_t SMEM = sizeof(float4) * CHUNK + sizeof(float) * VOX +
+                                 sizeof(uint32_t) * (W * W + W * CUBE + CUBE * CUBE) +
+                                 sizeof(uint16_t) * (CELLS + 2 + VOX);
 };
 
 // The exact conditions of the scan for voxel v: inside the particle's scan box, and before
@@ -444,13 +448,18 @@ __global__ void __launch_bounds__(CUBE_T, 2)
   constexpr int W = C::W, SUBS = BSX / CUBE, NV = BSX * BSX * BSX;
   extern __shared__ __align__(16) unsigned char smem[];
   float4* buf = reinterpret_cast<float4*>(smem);                   // p - 1/2, index of the particle
-  uint32_t* rowMask = reinterpret_cast<uint32_t*>(buf + CHUNK);    // [z][y] cells with particles
-  uint32_t* planeMask = rowMask + W * W;                           // [z] rows with particles
-  uint16_t* first = reinterpret_cast<uint16_t*>(planeMask + W);    // [CELLS + 1]
+  float* best = reinterpret_cast<float*>(buf + CHUNK);             // [VOX] each its thread's own
+  // bit x: particles within reach of a voxel's x in cell row (y, z); in the rows within
+  // reach of its y; in the planes within reach of its z
+  uint32_t* inRow = reinterpret_cast<uint32_t*>(best + C::VOX);    // [W z][W y]
+  uint32_t* inPlane = inRow + W * W;                               // [W z][CUBE y]
+  uint32_t* inReach = inPlane + W * CUBE;                          // [CUBE z][CUBE y]
+  uint16_t* first = reinterpret_cast<uint16_t*>(inReach + CUBE * CUBE);  // [CELLS + 1]
+  uint16_t* reached = first + C::CELLS + 2;                        // [VOX] voxels with particles in reach
   uint32_t* cnt = reinterpret_cast<uint32_t*>(first);              // counts, two to a word
   __shared__ int64_t binFirst[27];
   __shared__ int binEnd[27];
-  __shared__ int total, nBuf, warpSum[CUBE_T / 32];
+  __shared__ int total, nBuf, nReached, warpSum[CUBE_T / 32];
   const int s = blockIdx.x / (SUBS * SUBS * SUBS), sub = blockIdx.x % (SUBS * SUBS * SUBS);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int bid = vbid[s];
@@ -485,22 +494,16 @@ __global__ void __launch_bounds__(CUBE_T, 2)
   }
   __syncthreads();
   if (total < 0) return;  // k_splat_blocks has it
-  // this thread's voxels: x, y and z0, z0 + step, ...
-  const int vx = CUBE == 16 ? lane & 15 : lane & 7;
-  const int vy = CUBE == 16 ? (lane >> 4) + 2 * (w & 7) : (lane >> 3) + 4 * (w & 1);
-  const int vz0 = CUBE == 16 ? w >> 3 : w >> 1;
-  constexpr int VSTEP = 2;
   const float none = __uint_as_float(__float_as_uint(g.distSqMax) + 1u);
   // nearer than this a voxel is inside the scan box whatever the rounding of its bounds
   const float in = fmaxf(g.rScan - (1e-4f + 2e-6f * (float)max(g.s[0], max(g.s[1], g.s[2]))), 0.f);
   const float edge = in * in;
-  float best[C::VOX];
-#pragma unroll
-  for (int q = 0; q < C::VOX; q++) best[q] = none;
+  for (int v = tid; v < C::VOX; v += CUBE_T) best[v] = none;
 
   auto flush = [&](int n) {
     for (int i = tid; i < (C::CELLS + 2) / 2; i += CUBE_T) cnt[i] = 0u;
-    for (int i = tid; i < W * W + W; i += CUBE_T) rowMask[i] = 0u;
+    for (int i = tid; i < W * W; i += CUBE_T) inRow[i] = 0u;
+    if (tid == 0) nReached = 0;
     __syncthreads();
     float4 P[CHUNK / CUBE_T];
     int cell[CHUNK / CUBE_T], rank[CHUNK / CUBE_T];
@@ -515,10 +518,13 @@ __global__ void __launch_bounds__(CUBE_T, 2)
       cell[k] = cx + W * (cy + W * cz);
       rank[k] = (atomicAdd(&cnt[cell[k] >> 1], 1u << (16 * (cell[k] & 1))) >> (16 * (cell[k] & 1))) &
                 0xffff;
-      atomicOr(&rowMask[cz * W + cy], 1u << cx);
-      atomicOr(&planeMask[cz], 1u << cy);
+      atomicOr(&inRow[cz * W + cy], 1u << cx);
     }
     __syncthreads();
+    for (int i = tid; i < W * W; i += CUBE_T) {  // cells x .. x + 2R of the region's row
+      const uint32_t m = inRow[i], m2 = m | m >> 1, m4 = m2 | m2 >> 2;
+      inRow[i] = m4 | m4 >> 4 | m >> 8;
+    }
     {  // counts to first entries
       int sum = 0;
 #pragma unroll 3
@@ -534,6 +540,12 @@ __global__ void __launch_bounds__(CUBE_T, 2)
       }
       if (lane == 31) warpSum[w] = x;
       __syncthreads();
+      for (int i = tid; i < W * CUBE; i += CUBE_T) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int k = 0; k < 2 * C::R + 1; k++) m |= inRow[i / CUBE * W + i % CUBE + k];
+        inPlane[i] = m;
+      }
       int run = x - sum;
       for (int i = 0; i < w; i++) run += warpSum[i];
 #pragma unroll 3
@@ -553,29 +565,47 @@ __global__ void __launch_bounds__(CUBE_T, 2)
         buf[first[cell[k]] + rank[k]] =
             make_float4(__fsub_rn(P[k].x, 0.5f), __fsub_rn(P[k].y, 0.5f),
                         __fsub_rn(P[k].z, 0.5f), P[k].w);
-    __syncthreads();
-    const float fx = (float)(C0[0] + vx), fy = (float)(C0[1] + vy);
+    for (int i = tid; i < CUBE * CUBE; i += CUBE_T) {
+      uint32_t m = 0;
 #pragma unroll
-    for (int q = 0; q < C::VOX; q++) {
-      const int vz = vz0 + VSTEP * q;
-      const float fz = (float)(C0[2] + vz);
-      float b = best[q];
+      for (int k = 0; k < 2 * C::R + 1; k++) m |= inPlane[i + k * CUBE];
+      inReach[i] = m;
+    }
+    __syncthreads();
+    // the voxels to search, one behind the other: the threads share them evenly wherever in
+    // the cube the particles lie
+    for (int v = tid; v < C::VOX; v += CUBE_T) {
+      const bool on = (inReach[v / CUBE] >> (v % CUBE)) & 1u;
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      int at = 0;
+      if (lane == 0 && m) at = atomicAdd(&nReached, __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1));
+      if (on) reached[at] = (uint16_t)v;
+    }
+    __syncthreads();
+    const int nv = nReached;
+    // (one body for all voxels of a thread: unrolled over them, with the best in registers,
+    // it no longer fits the instruction cache)
+#pragma unroll 1
+    for (int q = tid; q < nv; q += CUBE_T) {
+      const int v = reached[q];
+      const int vx = v % CUBE, vy = v / CUBE % CUBE, vz = v / (CUBE * CUBE);
+      const float fx = (float)(C0[0] + vx), fy = (float)(C0[1] + vy), fz = (float)(C0[2] + vz);
+      float b = best[v];
       for (int kz = 0; kz < 2 * C::R + 1; kz++) {  // planes 0, -1, 1, -2, 2, ...
         const int az = (kz + 1) >> 1, oz = kz & 1 ? -az : az;
         const float mz = fmaxf((float)az - 0.5f, 0.f), mz2 = mz * mz;
         if (mz2 >= b) break;
-        const uint32_t rows = planeMask[vz + C::R + oz] >> vy;  // bit R + oy: row vy + oy
-        if (!(rows & ((2u << (2 * C::R)) - 1))) continue;
+        if (!((inPlane[(vz + C::R + oz) * CUBE + vy] >> vx) & 1u)) continue;
         for (int ky = 0; ky < 2 * C::R + 1; ky++) {
           const int ay = (ky + 1) >> 1, oy = ky & 1 ? -ay : ay;
           const float my = fmaxf((float)ay - 0.5f, 0.f), r = fmaf(my, my, mz2);
           if (r >= b) break;
-          if (!((rows >> (C::R + oy)) & 1u)) continue;
           const int row = (vz + C::R + oz) * W + vy + C::R + oy;
+          if (!((inRow[row] >> vx) & 1u)) continue;
           // cells vx - h .. vx + h: those with (h - 1/2)^2 + r < b
           const float left = b - r;
           const int h = (left > 0.25f) + (left > 2.25f) + (left > 6.25f) + (left > 12.25f);
-          if (!((rowMask[row] >> (vx + C::R - h)) & ((2u << (2 * h)) - 1))) continue;
           int i = first[row * W + vx + C::R - h];
           const int e = first[row * W + vx + C::R + h + 1];
           for (; i < e; i++) {
@@ -591,7 +621,7 @@ __global__ void __launch_bounds__(CUBE_T, 2)
           }
         }
       }
-      best[q] = b;
+      best[v] = b;
     }
     __syncthreads();  // the chunk is read
   };
@@ -632,11 +662,10 @@ __global__ void __launch_bounds__(CUBE_T, 2)
     }
   }
   uint16_t* out = pool + (int64_t)s * NV;
-#pragma unroll
-  for (int q = 0; q < C::VOX; q++) {
-    const uint32_t a = best[q] == none ? 65535u : splat_quantise(g, best[q]);
-    const int z = O[2] + vz0 + VSTEP * q;
-    out[O[0] + vx + BSX * (O[1] + vy + BSX * z)] = raw ? (uint16_t)a : splat_finalise(g, a);
+  for (int v = tid; v < C::VOX; v += CUBE_T) {
+    const int x = O[0] + v % CUBE, y = O[1] + v / CUBE % CUBE, z = O[2] + v / (CUBE * CUBE);
+    const uint32_t a = best[v] == none ? 65535u : splat_quantise(g, best[v]);
+    out[x + BSX * (y + BSX * z)] = raw ? (uint16_t)a : splat_finalise(g, a);
   }
 }
 
