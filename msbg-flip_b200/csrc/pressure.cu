@@ -534,7 +534,7 @@ int absmax(msbg_gpu_ctx* ctx, Solver& S, Runner<VT>& R, const V* v, int64_t n, d
   cudaStream_t st = R.st;
   Scalars* sc = S.scal.as<Scalars>();
   k_absmax<<<VEC_GRID, VEC_BLOCK, 0, st>>>(v, n, S.partial.as<double>());
-  k_finalize_max<<<1, 32, 0, st>>>(S.partial.as<double>(), VEC_GRID, sc);
+  k_finalize_max<<<1, 1024, 0, st>>>(S.partial.as<double>(), VEC_GRID, sc);
   cudaMemcpyAsync(S.hScal, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
   R.launches += 2;
   MSBG_CUDA_TRY(ctx, cudaStreamSynchronize(st));

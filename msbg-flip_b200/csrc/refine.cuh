@@ -93,13 +93,23 @@ __global__ void __launch_bounds__(VEC_BLOCK) k_absmax(const VT* __restrict__ v, 
   }
 }
 
-// Max of the partials into s->amax.
-static __global__ void __launch_bounds__(32) k_finalize_max(const double* __restrict__ partial, int n,
-                                                     Scalars* s) {
-  if (threadIdx.x != 0) return;
+// Max of the partials into s->amax (not a number if one of them is not).
+static __global__ void __launch_bounds__(1024) k_finalize_max(const double* __restrict__ partial,
+                                                              int n, Scalars* s) {
+  __shared__ double ws[32];
   double m = 0;
-  for (int i = 0; i < n; i++) m = (partial[i] != partial[i] || m != m) ? NAN : fmax(m, partial[i]);
-  s->amax = m;
+  bool nan = false;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    nan = nan || partial[i] != partial[i];
+    m = fmax(m, partial[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = m;
+  nan = __syncthreads_or(nan);
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmax(m, ws[w]);
+  s->amax = nan ? NAN : m;
 }
 
 // x64 += alpha d (FP64 accumulation of the FP32 direction); r -= alpha q;
