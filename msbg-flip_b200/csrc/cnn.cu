@@ -95,8 +95,8 @@ __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
 // A operand's 4 KB alone are 32 cycles of shared-memory reads), so the 27 taps cost
 // 10 instead of 27 instructions per plane and x half, with the products added in
 // the same order (kz, ky, kx): the same bits.  That bounds a tile to 30 us for 4
-// layers; measured 56 us.  Forward pass of 4096 tiles on a B200: 3.40 ms with a launch
-// per layer, N = 16 and the activations through global memory, 1.54 ms now.  (An MMA
+// layers; measured 50 us.  Forward pass of 4096 tiles on a B200: 3.40 ms with a launch
+// per layer, N = 16 and the activations through global memory, 1.39 ms now.  (An MMA
 // issued by a divergent thread costs over 100 cycles, its operands moving to uniform
 // registers one by one: 2.43 ms.)  Every wait is bounded.
 __global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3_tc(const __grid_constant__ ConvChain a) {

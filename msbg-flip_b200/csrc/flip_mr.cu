@@ -271,7 +271,7 @@ __device__ __forceinline__ void trilinear2(const MrGrid& g, int lv,
 // la, lb: MtLinstep's bounds as the reference forms them in float.
 // Bound by the gather: 16 M particles in no order over 57 M voxels (512^3, 3 levels,
 // B200) took 9.8 ms as they came, every sector a miss; visited block by block, with the
-// channels side by side and one look-up per window inside a block, 3.8 ms, of which the
+// channels side by side and one look-up per window inside a block, 3.5 ms, of which the
 // order takes 0.4.  The same bits.
 __global__ void __launch_bounds__(256) k_g2p_mr(msbg_flip_particle* __restrict__ p, int64_t np,
                                                 MrGrid g, const float2* __restrict__ vel,

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) k_convert(VD* __restrict__ y, const
 // loads are in flight together, the face data come resolved from the tile's record, and
 // a half sweep is one update per thread.  With a thread per z column of a tile, a
 // smoothing pass of 8^3 / 4^3 tiles took 18 / 14 us and a residual 23 / 14 us (256^3 grid
-// of 16^3 blocks, 3 levels, B200), and the FP16 solve 17.4 ms; now 13.1.
+// of 16^3 blocks, 3 levels, B200), and the FP16 solve 17.4 ms; with these kernels 13.1.
 template <int TS>
 struct TileGeo {
   static constexpr int N = TS * TS * TS;
