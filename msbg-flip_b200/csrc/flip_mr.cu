@@ -40,12 +40,14 @@ namespace {
 // _dTransRes at 6 whatever it is passed (src/msbg.cpp:198-201, 290).
 constexpr int kDTransRes = 6;
 
+constexpr int MR_LEVELS = 4;  // resolution levels at most
+
 struct MrState {
   int sx = 0, sy = 0, sz = 0, bsx0 = 0, nLevels = 0;
   std::vector<int> levels;
   int64_t n = 0;  // packed voxels
   bool distBuilt = false;
-  DeviceBuffer level, off, fc, kind, dist, parts;
+  DeviceBuffer level, off, fc, kind, key, dist, parts;
   DeviceBuffer vel;      // [3n] (vel, velOld) side by side: a gather reads both in one load
   DeviceBuffer scratch;  // one channel on its way in or out; the visiting order of G2P
   DeviceBuffer dsOffA, dsOffB, dsFlags, dsSrc, dsDst;  // downsampleVelocity
@@ -62,6 +64,7 @@ struct MrGrid {
   const int64_t* __restrict__ off;
   const int8_t* __restrict__ kind;  // [nl][nb]: 0 empty, 1 value, 2 full
   const uint16_t* __restrict__ dist;
+  const uint64_t* __restrict__ key;  // level, kinds and offset of a block
   // packed index of voxel (x, y, z) of level lv, or -1 (outside the level's
   // grid, or in a block of another level)
   __device__ __forceinline__ int64_t idx(int lv, int x, int y, int z) const {
@@ -183,48 +186,86 @@ __global__ void __launch_bounds__(256) k_mr_dist(MrGrid g, const int8_t* __restr
   }
 }
 
+// What a gather asks of a block, in one load: its level, its kinds in the distance channels
+// and its offset.
+constexpr int KEY_KIND = 4, KEY_OFF = KEY_KIND + 2 * MR_LEVELS;
+__device__ __forceinline__ int key_level(uint64_t k) { return (int)(k & 15); }
+__device__ __forceinline__ int key_kind(uint64_t k, int lv) {
+  return (int)(k >> (KEY_KIND + 2 * lv)) & 3;
+}
+
+__global__ void __launch_bounds__(256) k_mr_key(MrGrid g, uint64_t* __restrict__ key) {
+  const int64_t nb = (int64_t)g.nbx * g.nby * g.nbz;
+  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nb;
+       b += (int64_t)gridDim.x * blockDim.x) {
+    uint64_t k = (uint64_t)g.off[b] << KEY_OFF | (uint64_t)g.level[b];
+    for (int l = 0; l < g.nl; l++) k |= (uint64_t)g.kind[l * nb + b] << (KEY_KIND + 2 * l);
+    key[b] = k;
+  }
+}
+
+// The gathers are shared by a pair of lanes, of which one (side 0) loads the values at x and
+// the other those at x + 1: the two are next to each other in memory, so a pair asks for
+// one line per row of its window.  The pair then trades what the other needs.
+__device__ __forceinline__ float pair_trade(float v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+
+// A lane's half of a 2x2x2 window at level lv: column x, rows y[0..1], planes z[0..1] (in the
+// grid), by shares of the block index and of the voxel's place in its block.
+struct MrWindow {
+  int sh, bx, lx, by[2], ly[2], bz[2], lz[2];
+  __device__ __forceinline__ MrWindow(const MrGrid& g, int lv, int x, int y0, int y1, int z0, int z1)
+      : sh(g.sh0 - lv) {
+    const int m = (1 << sh) - 1;
+    bx = x >> sh;
+    lx = x & m;
+    by[0] = (y0 >> sh) * g.nbx;
+    by[1] = (y1 >> sh) * g.nbx;
+    ly[0] = (y0 & m) << sh;
+    ly[1] = (y1 & m) << sh;
+    bz[0] = (z0 >> sh) * (g.nbx * g.nby);
+    bz[1] = (z1 >> sh) * (g.nbx * g.nby);
+    lz[0] = (z0 & m) << (2 * sh);
+    lz[1] = (z1 & m) << (2 * sh);
+  }
+  __device__ __forceinline__ int block(int c) const { return bx + by[c & 1] + bz[c >> 1]; }
+  __device__ __forceinline__ int voxel(int c) const { return lx + ly[c & 1] + lz[c >> 1]; }
+};
+
 // SparseGrid<uint16_t>::interpolateToFloat<IP_LINEAR> with OPT_IPBC_NEUMAN
 // (src/sbg.h:1386, 2936-2941, 3111-3420) on the distance channel of level
 // lv: cell-centred, the 2x2x2 window clamped to the grid, value blocks read
 // their data, full blocks dTransRes*1024, the others 0; p1*t + p0*(1-t)
-// along x, then y, then z.  A window inside one block asks for its kind once.
-__device__ __forceinline__ float dist_interp(const MrGrid& g, int lv, float px, float py,
-                                             float pz) {
+// along x, then y, then z.
+// All lanes of a warp call it; `on` is the same in both lanes of a pair.
+__device__ __forceinline__ float dist_interp(const MrGrid& g, int lv, bool on, int side, float px,
+                                             float py, float pz) {
   const float x = __fsub_rn(px, 0.5f), y = __fsub_rn(py, 0.5f), z = __fsub_rn(pz, 0.5f);
   const int ix = (int)floorf(x), iy = (int)floorf(y), iz = (int)floorf(z);
   const float u = __fsub_rn(x, (float)ix), v = __fsub_rn(y, (float)iy),
               w = __fsub_rn(z, (float)iz);
-  const int nx = g.sx >> lv, ny = g.sy >> lv, nz = g.sz >> lv, sh = g.sh0 - lv;
-  const int m = (1 << sh) - 1;
-  const int64_t nb = (int64_t)g.nbx * g.nby * g.nbz;
-  const float full = (float)(kDTransRes * 1024);
-  const int x0 = min(max(ix, 0), nx - 1), x1 = min(max(ix + 1, 0), nx - 1);
-  const int y0 = min(max(iy, 0), ny - 1), y1 = min(max(iy + 1, 0), ny - 1);
-  const int z0 = min(max(iz, 0), nz - 1), z1 = min(max(iz + 1, 0), nz - 1);
-  float c[8];
-  if ((((x0 ^ x1) | (y0 ^ y1) | (z0 ^ z1)) >> sh) == 0) {
-    const int64_t b = (x0 >> sh) + (int64_t)g.nbx * ((y0 >> sh) + (int64_t)g.nby * (z0 >> sh));
-    const int kd = g.kind[(int64_t)lv * nb + b];
-    const float f = kd == 2 ? full : 0.f;
-    const uint16_t* d = kd == 1 && g.level[b] == lv ? g.dist + g.off[b] : nullptr;
+  float c[4] = {0.f, 0.f, 0.f, 0.f};
+  if (on) {
+    const int nx = g.sx >> lv, ny = g.sy >> lv, nz = g.sz >> lv;
+    const MrWindow win(g, lv, min(max(ix + side, 0), nx - 1), min(max(iy, 0), ny - 1),
+                       min(max(iy + 1, 0), ny - 1), min(max(iz, 0), nz - 1),
+                       min(max(iz + 1, 0), nz - 1));
+    uint64_t key[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++)
-      c[k] = d ? (float)d[((k & 1 ? x1 : x0) & m) + (((k & 2 ? y1 : y0) & m) << sh) +
-                          (((k & 4 ? z1 : z0) & m) << (2 * sh))]
-               : f;
-  } else {
+    for (int k = 0; k < 4; k++) key[k] = g.key[win.block(k)];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int xx = k & 1 ? x1 : x0, yy = k & 2 ? y1 : y0, zz = k & 4 ? z1 : z0;
-      const int64_t b = (xx >> sh) + (int64_t)g.nbx * ((yy >> sh) + (int64_t)g.nby * (zz >> sh));
-      const int kd = g.kind[(int64_t)lv * nb + b];
-      c[k] = kd == 1 ? (float)g.dist[g.idx(lv, xx, yy, zz)] : kd == 2 ? full : 0.f;
+    for (int k = 0; k < 4; k++) {
+      const int kd = key_kind(key[k], lv);
+      if (kd == 1) c[k] = (float)g.dist[(int64_t)(key[k] >> KEY_OFF) + win.voxel(k)];
+      if (kd == 2) c[k] = (float)(kDTransRes * 1024);
     }
   }
   const float u1 = __fsub_rn(1.0f, u), v1 = __fsub_rn(1.0f, v), w1 = __fsub_rn(1.0f, w);
   float e[4], f[2];
 #pragma unroll
-  for (int k = 0; k < 4; k++) e[k] = __fadd_rn(__fmul_rn(c[2 * k + 1], u), __fmul_rn(c[2 * k], u1));
+  for (int k = 0; k < 4; k++) {
+    const float mine = __fmul_rn(c[k], side ? u : u1), other = pair_trade(mine);
+    e[k] = __fadd_rn(mine, other);  // the same in either order
+  }
 #pragma unroll
   for (int k = 0; k < 2; k++) f[k] = __fadd_rn(__fmul_rn(e[2 * k + 1], v), __fmul_rn(e[2 * k], v1));
   return __fadd_rn(__fmul_rn(f[1], w), __fmul_rn(f[0], w1));
@@ -233,36 +274,42 @@ __device__ __forceinline__ float dist_interp(const MrGrid& g, int lv, float px, 
 __device__ __constant__ float kMrOff[3][3] = {{0.f, 0.5f, 0.5f}, {0.5f, 0.f, 0.5f},
                                               {0.5f, 0.5f, 0.f}};
 
-// Trilinear sums of component d in both channels at level lv, from the
-// sample origin (ix0, iy0, iz0) and fractions (fx, fy, fz).  A window inside one
-// block asks for its level and offset once.
-__device__ __forceinline__ void trilinear2(const MrGrid& g, int lv,
-                                           const float2* __restrict__ vel, int d, int ix0, int iy0, int iz0, float fx, float fy, float fz,
-                                           float& sa, float& sb) {
-  sa = 0.f;
-  sb = 0.f;
-  const int sh = g.sh0 - lv, m = (1 << sh) - 1;
-  const bool in = ix0 >= 0 && iy0 >= 0 && iz0 >= 0 && ix0 < (g.sx >> lv) - 1 &&
-                  iy0 < (g.sy >> lv) - 1 && iz0 < (g.sz >> lv) - 1;
-  const bool one = in && (((ix0 ^ (ix0 + 1)) | (iy0 ^ (iy0 + 1)) | (iz0 ^ (iz0 + 1))) >> sh) == 0;
-  int64_t base = -1;
-  if (one) {
-    const int64_t b = (ix0 >> sh) + (int64_t)g.nbx * ((iy0 >> sh) + (int64_t)g.nby * (iz0 >> sh));
-    // in a block of another level every value reads 0, and so do the sums (+0)
-    if (g.level[b] != lv) return;
-    base = g.off[b] + (ix0 & m) + ((iy0 & m) << sh) + ((iz0 & m) << (2 * sh));
-  }
-  const float gx = __fsub_rn(1.f, fx), gy = __fsub_rn(1.f, fy), gz = __fsub_rn(1.f, fz);
+// Trilinear sum of component d at level lv, from the sample origin (ix0, iy0, iz0) and
+// fractions (fx, fy, fz): that of vel in side 0, that of velOld in side 1.  Outside the
+// grid, and in a block of another level, every value reads 0.  All lanes of a warp call
+// it; `on` is the same in both lanes of a pair.
+__device__ __forceinline__ float trilinear_pair(const MrGrid& g, int lv, bool on, int side,
+                                                const float2* __restrict__ vel, int d, int ix0,
+                                                int iy0, int iz0, float fx, float fy, float fz) {
+  float2 v[4];
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
-    const int64_t i =
-        one ? base + dx + (dy << sh) + (dz << (2 * sh)) : g.idx(lv, ix0 + dx, iy0 + dy, iz0 + dz);
-    const float2 v = i < 0 ? make_float2(0.f, 0.f) : vel[3 * i + d];
-    const float w = __fmul_rn(__fmul_rn(dx ? fx : gx, dy ? fy : gy), dz ? fz : gz);
-    sa = __fadd_rn(sa, __fmul_rn(w, v.x));
-    sb = __fadd_rn(sb, __fmul_rn(w, v.y));
+  for (int c = 0; c < 4; c++) v[c] = make_float2(0.f, 0.f);
+  const int x = ix0 + side, nx = g.sx >> lv, ny = g.sy >> lv, nz = g.sz >> lv;
+  if (on && (unsigned)x < (unsigned)nx) {
+    const MrWindow win(g, lv, x, iy0, iy0 + 1, iz0, iz0 + 1);
+    bool in[4];
+    uint64_t key[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      in[c] = (unsigned)(iy0 + (c & 1)) < (unsigned)ny && (unsigned)(iz0 + (c >> 1)) < (unsigned)nz;
+      key[c] = in[c] ? g.key[win.block(c)] : 15;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      if (key_level(key[c]) == lv)
+        v[c] = vel[3 * ((int64_t)(key[c] >> KEY_OFF) + win.voxel(c)) + d];
   }
+  const float wx = side ? fx : __fsub_rn(1.f, fx), gy = __fsub_rn(1.f, fy), gz = __fsub_rn(1.f, fz);
+  float s = 0.f;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const float w = __fmul_rn(__fmul_rn(wx, c & 1 ? fy : gy), c >> 1 ? fz : gz);
+    const float a = __fmul_rn(w, v[c].x), b = __fmul_rn(w, v[c].y);
+    const float mine = side ? b : a, other = pair_trade(side ? a : b);
+    s = __fadd_rn(s, side ? other : mine);  // x, then x + 1
+    s = __fadd_rn(s, side ? mine : other);
+  }
+  return s;
 }
 
 // gridToParticle with interpCompMSBG per component (interpVec3MSBG yields the
@@ -271,59 +318,69 @@ __device__ __forceinline__ void trilinear2(const MrGrid& g, int lv,
 // la, lb: MtLinstep's bounds as the reference forms them in float.
 // Bound by the gather: 16 M particles in no order over 57 M voxels (512^3, 3 levels,
 // B200) took 9.8 ms as they came, every sector a miss; visited block by block, with the
-// channels side by side and one look-up per window inside a block, 3.5 ms, of which the
-// order takes 0.4.  The same bits.
+// channels side by side, 3.5 ms, of which the order takes 0.4.  That was 2000
+// instructions for 16 particles, most for windows that cross blocks, of which every warp
+// has some: with a pair of lanes per particle 3.26 ms, and with one look-up of a block's key
+// per corner, the same for all windows, 1.94 ms.  The same bits.
 __global__ void __launch_bounds__(256) k_g2p_mr(msbg_flip_particle* __restrict__ p, int64_t np,
                                                 MrGrid g, const float2* __restrict__ vel,
                                                 BinsOrder order, float alpha, double la,
                                                 double lb) {
   const int* perm = order.get();
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < np;
-       n += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = perm ? perm[n] : n;
-    msbg_flip_particle q = p[k];
-    const bool finite = isfinite(q.pos[0]) && isfinite(q.pos[1]) && isfinite(q.pos[2]);
+  const int side = threadIdx.x & 1;
+  const int64_t n0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 1;
+  const int lane2 = (threadIdx.x & 31) >> 1;
+  // the bound is the warp's: its lanes stay together for the trades
+  for (int64_t n = n0; n - lane2 < np; n += ((int64_t)gridDim.x * blockDim.x) >> 1) {
+    const bool valid = n < np;
+    const int64_t k = valid ? (perm ? perm[n] : n) : 0;
+    const msbg_flip_particle q = p[k];
+    const bool finite = valid && isfinite(q.pos[0]) && isfinite(q.pos[1]) && isfinite(q.pos[2]);
+    float out[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      float pic = 0.f, old = 0.f;  // no cell for a particle without a finite position
+      const float gx = __fsub_rn(q.pos[0], kMrOff[d][0]), gy = __fsub_rn(q.pos[1], kMrOff[d][1]),
+                  gz = __fsub_rn(q.pos[2], kMrOff[d][2]);
+      const int ix0 = (int)floorf(gx), iy0 = (int)floorf(gy), iz0 = (int)floorf(gz);
+      const float fx = __fsub_rn(gx, (float)ix0), fy = __fsub_rn(gy, (float)iy0),
+                  fz = __fsub_rn(gz, (float)iz0);
+      int lv = 0;
       if (finite) {
-        const float gx = __fsub_rn(q.pos[0], kMrOff[d][0]), gy = __fsub_rn(q.pos[1], kMrOff[d][1]),
-                    gz = __fsub_rn(q.pos[2], kMrOff[d][2]);
-        const int ix0 = (int)floorf(gx), iy0 = (int)floorf(gy), iz0 = (int)floorf(gz);
-        const float fx = __fsub_rn(gx, (float)ix0), fy = __fsub_rn(gy, (float)iy0),
-                    fz = __fsub_rn(gz, (float)iz0);
         const int cx = min(max(ix0, 0), g.sx - 1), cy = min(max(iy0, 0), g.sy - 1),
                   cz = min(max(iz0, 0), g.sz - 1);
-        const int lv = g.level[(cx >> g.sh0) +
-                               (int64_t)g.nbx * ((cy >> g.sh0) + (int64_t)g.nby * (cz >> g.sh0))];
-        float fa, fb;
-        trilinear2(g, 0, vel, d, ix0, iy0, iz0, fx, fy, fz, fa, fb);
-        if (lv == 0) {
-          pic = fa;
-          old = fb;
-        } else {
-          const float scale = 1.f / (float)(1 << lv);  // a power of two: exact
-          const float cgx = __fmul_rn(gx, scale), cgy = __fmul_rn(gy, scale),
-                      cgz = __fmul_rn(gz, scale);
-          const int cix0 = (int)floorf(cgx), ciy0 = (int)floorf(cgy), ciz0 = (int)floorf(cgz);
-          const float cfx = __fsub_rn(cgx, (float)cix0), cfy = __fsub_rn(cgy, (float)ciy0),
-                      cfz = __fsub_rn(cgz, (float)ciz0);
-          float ca, cb;
-          trilinear2(g, lv, vel, d, cix0, ciy0, ciz0, cfx, cfy, cfz, ca, cb);
-          const float dist = __fmul_rn(dist_interp(g, lv, cgx, cgy, cgz), 1.0f / 1024.0f);
+        lv = key_level(g.key[(cx >> g.sh0) + g.nbx * ((cy >> g.sh0) + g.nby * (cz >> g.sh0))]);
+      }
+      // pic in side 0, the old value in side 1
+      float s = trilinear_pair(g, 0, finite, side, vel, d, ix0, iy0, iz0, fx, fy, fz);
+      if (__any_sync(0xffffffffu, lv > 0)) {
+        const bool on = lv > 0;
+        const float scale = 1.f / (float)(1 << lv);  // a power of two: exact
+        const float cgx = __fmul_rn(gx, scale), cgy = __fmul_rn(gy, scale),
+                    cgz = __fmul_rn(gz, scale);
+        const int cix0 = (int)floorf(cgx), ciy0 = (int)floorf(cgy), ciz0 = (int)floorf(cgz);
+        const float c = trilinear_pair(g, lv, on, side, vel, d, cix0, ciy0, ciz0,
+                                       __fsub_rn(cgx, (float)cix0), __fsub_rn(cgy, (float)ciy0),
+                                       __fsub_rn(cgz, (float)ciz0));
+        const float dist =
+            __fmul_rn(dist_interp(g, lv, on, side, cgx, cgy, cgz), 1.0f / 1024.0f);
+        if (on) {
           const double x = (double)dist;
           const float af = x < la ? 0.f : x >= lb ? 1.f : (float)((x - la) / (lb - la));
-          const float bf = __fsub_rn(1.f, af);
-          pic = __fadd_rn(__fmul_rn(af, fa), __fmul_rn(bf, ca));
-          old = __fadd_rn(__fmul_rn(af, fb), __fmul_rn(bf, cb));
+          s = __fadd_rn(__fmul_rn(af, s), __fmul_rn(__fsub_rn(1.f, af), c));
         }
       }
-      q.vel[d] = __fadd_rn(__fmul_rn(__fsub_rn(1.f, alpha), pic),
-                           __fmul_rn(alpha, __fadd_rn(q.vel[d], __fsub_rn(pic, old))));
+      if (!finite) s = 0.f;  // no cell for a particle without a finite position
+      const float t = pair_trade(s), pic = side ? t : s, old = side ? s : t;
+      out[d] = __fadd_rn(__fmul_rn(__fsub_rn(1.f, alpha), pic),
+                         __fmul_rn(alpha, __fadd_rn(q.vel[d], __fsub_rn(pic, old))));
     }
-    p[k].vel[0] = q.vel[0];
-    p[k].vel[1] = q.vel[1];
-    p[k].vel[2] = q.vel[2];
+    if (!valid) continue;
+    if (side) {
+      p[k].vel[2] = out[2];
+    } else {
+      p[k].vel[0] = out[0];
+      p[k].vel[1] = out[1];
+    }
   }
 }
 
@@ -463,6 +520,7 @@ int mr_state(msbg_gpu_ctx* ctx, MrState** out, MrGrid& g) {
     MSBG_CUDA_TRY(ctx, s->off.ensure(8 * nb));
     MSBG_CUDA_TRY(ctx, s->fc.ensure(nb));
     MSBG_CUDA_TRY(ctx, s->kind.ensure((size_t)nb * ctx->nLevels));
+    MSBG_CUDA_TRY(ctx, s->key.ensure(8 * nb));
     MSBG_CUDA_TRY(ctx, s->dist.ensure(2 * (size_t)o));
     MSBG_CUDA_TRY(ctx, s->vel.ensure(24 * (size_t)o));
     MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(s->level.p, lv8.data(), nb, cudaMemcpyHostToDevice, st));
@@ -477,7 +535,7 @@ int mr_state(msbg_gpu_ctx* ctx, MrState** out, MrGrid& g) {
   while ((1 << sh) < ctx->bsx0) sh++;
   g = MrGrid{S.sx, S.sy, S.sz, sh, ctx->nbx, ctx->nby, ctx->nbz, S.nLevels,
              S.level.as<int8_t>(), S.off.as<int64_t>(), S.kind.as<int8_t>(),
-             S.dist.as<uint16_t>()};
+             S.dist.as<uint16_t>(), S.key.as<uint64_t>()};
   *out = sp.get();
   return MSBG_OK;
 }
@@ -494,6 +552,7 @@ int mr_build_dist(msbg_gpu_ctx* ctx, MrState* S, const MrGrid& g) {
                                                            S->kind.as<int8_t>());
   k_mr_dist<<<(int)std::min<int64_t>(nb, 148 * 16), 256, 0, st>>>(g, S->fc.as<int8_t>(),
                                                                    S->dist.as<uint16_t>());
+  k_mr_key<<<grid_blocks(nb), 256, 0, st>>>(g, S->key.as<uint64_t>());
   MSBG_CUDA_TRY(ctx, cudaGetLastError());
   S->distBuilt = true;
   return MSBG_OK;
@@ -587,7 +646,7 @@ int flip_g2p_mr(msbg_gpu_ctx* ctx, msbg_flip_particle* particles, int64_t np, fl
   if (np >= MR_BINS_MIN)
     MSBG_CUDA_TRY(ctx, bins_build(S->scratch, dp, np, BinsGrid{g.sx, g.sy, g.sz, g.sh0, g.nbx, g.nby},
                                   ctx->nb(), st, order));
-  k_g2p_mr<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, S->vel.as<float2>(), order, flipAlpha,
+  k_g2p_mr<<<grid_blocks(2 * np), 256, 0, st>>>(dp, np, g, S->vel.as<float2>(), order, flipAlpha,
                                             (double)la, (double)lb);
   MSBG_CUDA_TRY(ctx, cudaGetLastError());
   if (!onDevice)

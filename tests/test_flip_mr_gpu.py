@@ -238,3 +238,22 @@ def test_many_particles_in_any_order(name, order):
         assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("count", [1, 2, 15, 16, 17, 31, 129])
+def test_few_particles_and_a_ragged_last_warp(count):
+    """Two lanes share a particle and the last warp is not full: every particle has the bits that
+    it has in a larger batch, whichever lanes it falls to."""
+    name = list(GRIDS)[-1]
+    ctx, res, bsx, nl, lev = _ctx(name)
+    try:
+        vel, old = _channels(msbg_gpu.packed_voxels(bsx, lev), 6)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL, vel)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL_OLD, old)
+        p = particles_for(res, 400, 13)
+        q, r = p.copy(), p[-count:].copy()
+        ctx.flip_g2p_mr(q, ALPHA)
+        ctx.flip_g2p_mr(r, ALPHA)
+        assert np.array_equal(q["vel"][-count:].view(np.uint32), r["vel"].view(np.uint32))
+    finally:
+        ctx.close()
