@@ -123,17 +123,17 @@ __global__ void k_p2g_scatter(const msbg_flip_particle* __restrict__ p, int64_t 
 // Many particles: cell by cell.  Scattering them one by one costs 72 float atomics each,
 // at 400 G atomics/s the bound of the pass (13.3 M particles on 160^3 cells, B200: 2.2 of
 // P2G's 2.5 ms).  Here
-//   k_p2g_count  gives each particle its rank in its cell, and counts the cells'
-//                particles and liquid ones;
+//   k_p2g_count  gives each particle its cell and its rank there, and counts the cells'
+//                particles and liquid ones; a particle with a finite position outside the
+//                grid reaches its boundary faces alone, and does so here;
 //   k_p2g_start, k_p2g_place  list the particles cell by cell (indices; the particles
 //                stay where they are);
-//   k_p2g_cells  a CTA per 8^3 cells, a thread per cell: a cell's particles reach 2 x 3 x
+//   k_p2g_cells  a CTA per 8 x 8 x 4 cells, a thread per cell: a cell's particles reach 2 x 3 x
 //                3 faces per direction, whose three sums the thread keeps in registers;
-//                they go to the CTA's 9 x 10 x 10 faces in shared memory one neighbour
+//                they go to the CTA's faces in shared memory one neighbour
 //                offset at a time, in which no two threads meet, and from there to the
 //                grid with one float atomic per face and sum.
-// A particle with a finite position outside the grid reaches its boundary faces alone,
-// through k_p2g_outside.  0.92 ms for the five kernels.
+// 0.73 ms for the four kernels.
 
 // The cell of a particle with a finite position; -1 outside the grid.
 __device__ __forceinline__ int64_t cell_of(const msbg_flip_particle& q, const GridF& g) {
@@ -141,15 +141,21 @@ __device__ __forceinline__ int64_t cell_of(const msbg_flip_particle& q, const Gr
 }
 
 __global__ void __launch_bounds__(256) k_p2g_count(const msbg_flip_particle* __restrict__ p,
-                                                   int64_t np, GridF g,
+                                                   int64_t np, GridF g, int64_t n, float rhoL,
+                                                   float rhoG,
                                                    unsigned long long* __restrict__ cnt,
-                                                   int* __restrict__ rank) {
+                                                   int2* __restrict__ place,
+                                                   float* __restrict__ acc) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
        k += (int64_t)gridDim.x * blockDim.x) {
     const msbg_flip_particle& q = p[k];
-    const int64_t ci = finite_pos(q) ? cell_of(q, g) : -1;
+    const bool finite = finite_pos(q);
+    const int64_t ci = finite ? cell_of(q, g) : -1;
+    int2 at = make_int2((int)ci, 0);
     // low word particles, high word liquid ones
-    if (ci >= 0) rank[k] = (int)atomicAdd(&cnt[ci], q.phase == 0 ? (1ull << 32) + 1 : 1ull);
+    if (ci >= 0) at.y = (int)atomicAdd(&cnt[ci], q.phase == 0 ? (1ull << 32) + 1 : 1ull);
+    place[k] = at;
+    if (finite && ci < 0) scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
   }
 }
 
@@ -190,32 +196,21 @@ __global__ void __launch_bounds__(1024) k_p2g_start(int64_t n,
   liq[c] = (int)(u >> 32);
 }
 
-__global__ void __launch_bounds__(256) k_p2g_place(const msbg_flip_particle* __restrict__ p,
-                                                   int64_t np, GridF g,
-                                                   const int* __restrict__ rank,
+__global__ void __launch_bounds__(256) k_p2g_place(int64_t np, const int2* __restrict__ place,
                                                    const int* __restrict__ start,
                                                    int* __restrict__ perm) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
        k += (int64_t)gridDim.x * blockDim.x) {
-    const msbg_flip_particle& q = p[k];
-    const int64_t ci = finite_pos(q) ? cell_of(q, g) : -1;
-    if (ci >= 0) perm[start[ci] + rank[k]] = (int)k;
+    const int2 at = place[k];
+    if (at.x >= 0) perm[start[at.x] + at.y] = (int)k;
   }
 }
 
-__global__ void __launch_bounds__(256) k_p2g_outside(const msbg_flip_particle* __restrict__ p,
-                                                     int64_t np, GridF g, int64_t n, float rhoL,
-                                                     float rhoG, float* __restrict__ acc) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const msbg_flip_particle& q = p[k];
-    if (finite_pos(q) && cell_of(q, g) < 0)
-      scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
-  }
-}
-
-constexpr int SUB = 8;                         // cells per edge of a CTA's cube
-constexpr int FACE_ROW = SUB + 2, FACES = FACE_ROW * FACE_ROW * FACE_ROW;
+// Cells of a CTA along x and y, and along z.  A thread needs 54 sums and so close to 80
+// registers: three CTAs of this size share an SM, of 8^3 cells it holds one, which waits out
+// its loads and barriers alone (0.66 ms; 0.56 this way).
+constexpr int SUB = 8, SUB_Z = 4, SUB_T = SUB * SUB * SUB_Z;
+constexpr int FACE_ROW = SUB + 2, FACES = FACE_ROW * FACE_ROW * (SUB_Z + 2);
 
 // Direction D: faces of cell (x, y, z) at offset 0, 1 along D and -1, 0, 1 along the others.
 template <int D>
@@ -278,7 +273,7 @@ __device__ __forceinline__ void p2g_direction(const msbg_flip_particle* __restri
       }
 }
 
-__global__ void __launch_bounds__(SUB* SUB* SUB) k_p2g_cells(
+__global__ void __launch_bounds__(SUB_T, 3) k_p2g_cells(
     const msbg_flip_particle* __restrict__ p, GridF g, int64_t n, float rhoL, float rhoG,
     const unsigned long long* __restrict__ cnt, const int* __restrict__ start,
     const int* __restrict__ perm, float* __restrict__ acc) {
@@ -286,7 +281,7 @@ __global__ void __launch_bounds__(SUB* SUB* SUB) k_p2g_cells(
   const int t = threadIdx.x;
   const int nsx = g.sx / SUB, nsy = g.sy / SUB;
   const int bx = blockIdx.x % nsx * SUB, by = blockIdx.x / nsx % nsy * SUB,
-            bz = blockIdx.x / (nsx * nsy) * SUB;
+            bz = blockIdx.x / (nsx * nsy) * SUB_Z;
   const int lx = t % SUB, ly = t / SUB % SUB, lz = t / (SUB * SUB);
   const int x = bx + lx, y = by + ly, z = bz + lz;
   const int64_t ci = g.idx(x, y, z);
@@ -296,10 +291,10 @@ __global__ void __launch_bounds__(SUB* SUB* SUB) k_p2g_cells(
   const int at = (lx + 1) + FACE_ROW * ((ly + 1) + FACE_ROW * (lz + 1));
   auto direction = [&](auto dd) {
     constexpr int D = decltype(dd)::value;
-    for (int i = t; i < 3 * FACES; i += SUB * SUB * SUB) sums[i / FACES][i % FACES] = 0.f;
+    for (int i = t; i < 3 * FACES; i += SUB_T) sums[i / FACES][i % FACES] = 0.f;
     __syncthreads();
     p2g_direction<D>(p, list, m, x, y, z, at, rhoL, rhoG, sums);
-    for (int i = t; i < FACES; i += SUB * SUB * SUB) {
+    for (int i = t; i < FACES; i += SUB_T) {
       const float w = sums[1][i];
       const float v = sums[0][i], r = sums[2][i];
       if (w == 0.f && v == 0.f && r == 0.f) continue;
@@ -578,7 +573,8 @@ int flip_p2g(msbg_gpu_ctx* ctx, const msbg_flip_particle* particles, int64_t np,
   }
   bool cells = np >= FLIP_MANY && np <= INT_MAX && n <= INT_MAX;
   if (cells && (S->cells.ensure(12 * (size_t)n + 8) != cudaSuccess ||
-                S->lists.ensure(bins_bytes(np, ctx->nb())) != cudaSuccess)) {
+                S->lists.ensure(std::max<size_t>(12 * (size_t)np, bins_bytes(np, ctx->nb()))) !=
+                    cudaSuccess)) {
     cudaGetLastError();  // no room for the lists: particle by particle
     cells = false;
   }
@@ -586,17 +582,16 @@ int flip_p2g(msbg_gpu_ctx* ctx, const msbg_flip_particle* particles, int64_t np,
     auto* cnt = S->cells.as<unsigned long long>();  // [n], the cursor, then the starts [n]
     int* cursor = reinterpret_cast<int*>(cnt + n);
     int* start = cursor + 2;
-    int* rank = S->lists.as<int>();
-    int* perm = rank + np;
+    int2* place = S->lists.as<int2>();  // cell (-1: none) and rank in it of a particle
+    int* perm = reinterpret_cast<int*>(place + np);
     MSBG_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, 8 * (size_t)(n + 1), st));
-    k_p2g_count<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, cnt, rank);
+    k_p2g_count<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, n, prm->rhoL, prm->rhoG, cnt, place,
+                                                 S->acc.as<float>());
     k_p2g_start<<<(unsigned)((n + 1023) / 1024), 1024, 0, st>>>(
         n, cnt, start, S->mass.as<float>(), S->liq.as<int>(), cursor);
-    k_p2g_place<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, rank, start, perm);
-    k_p2g_cells<<<(unsigned)(n / (SUB * SUB * SUB)), SUB * SUB * SUB, 0, st>>>(
+    k_p2g_place<<<grid_blocks(np), 256, 0, st>>>(np, place, start, perm);
+    k_p2g_cells<<<(unsigned)(n / SUB_T), SUB_T, 0, st>>>(
         dp, g, n, prm->rhoL, prm->rhoG, cnt, start, perm, S->acc.as<float>());
-    k_p2g_outside<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, n, prm->rhoL, prm->rhoG,
-                                                   S->acc.as<float>());
   } else {
     MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S->mass.p, 0, 4 * (size_t)n, st));
     MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S->liq.p, 0, 4 * (size_t)n, st));
