@@ -511,11 +511,13 @@ int residual64(msbg_gpu_ctx* ctx, Solver& S, Runner<VT>& R, const float* b, floa
   cudaStream_t st = R.st;
   const Level& L = S.H.levels[0];
   double* part = S.partial.as<double>();
+  cudaFuncSetAttribute(k_residual64_16, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)RES16_SMEM);
   int off = 0;
   for (const auto& g : L.groups) {
     const int* lst = S.dev[0]->groupTiles.as<int>() + g.start;
-    TS_DISPATCH(g.ts, (k_residual64<T><<<g.count, T * T * res64_split<T>(), 0, st>>>(
-                          S.views[0], lst, S.x64.as<double>(), b, r32, part + off)));
+    TS_DISPATCH(g.ts, (launch_residual64<T>(S.views[0], lst, g.count, S.x64.as<double>(), b, r32,
+                                            part + off, st)));
     off += g.count;
     R.launches++;
   }

@@ -7,25 +7,21 @@
 // correction to x in FP64.  This is what lets the true residual reach 1e-6
 // where an FP32 iterate cannot represent it.
 
-// r32 = b - A x64 on MG level 0 (one CTA per tile; thread (i,j,h) owns the
-// h-th part of the z column (i,j): 16^3 tiles in two halves, so a CTA has
-// 512 threads and more loads in flight), per-CTA partial |r|^2 in FP64.
+// r32 = b - A x64 on MG level 0 (one CTA per tile; thread (i, j) owns the z column (i, j)),
+// per-CTA partial |r|^2 in FP64.
 template <int TS>
-__host__ __device__ constexpr int res64_split() { return TS == 16 ? 2 : 1; }
-template <int TS>
-__global__ void __launch_bounds__(TS* TS* res64_split<TS>())
+__global__ void __launch_bounds__(TS* TS)
     k_residual64(LevelView L, const int* __restrict__ tiles, const double* __restrict__ x,
                  const float* __restrict__ b, float* __restrict__ r,
                  double* __restrict__ partial) {
-  constexpr int N = TS * TS * TS, NF = TS * TS, SPLIT = res64_split<TS>(), NT = NF * SPLIT;
-  constexpr int ZC = TS / SPLIT;  // cells of a thread's z column part
+  constexpr int N = TS * TS * TS, NF = TS * TS;
   __shared__ double xs[N];
   __shared__ double gs[6][NF];
   const int ti = tiles[blockIdx.x];
   const int64_t off = L.tileOff[ti];
-  const int t = threadIdx.x, i = t % TS, j = (t / TS) % TS, h = t / NF;
-  for (int e = t; e < N; e += NT) xs[e] = x[off + e];
-  for (int q = t; q < 6 * NF; q += NT) {
+  const int t = threadIdx.x, i = t % TS, j = t / TS;
+  for (int e = t; e < N; e += NF) xs[e] = x[off + e];
+  for (int q = t; q < 6 * NF; q += NF) {
     const int f = q / NF, c = q % NF;
     gs[f][c] = ghost_sum<double, double>(L, x, ti, TS, f >> 1, f & 1, c % TS, c / TS);
   }
@@ -34,7 +30,7 @@ __global__ void __launch_bounds__(TS* TS* res64_split<TS>())
   const float* cy = L.cy + off;
   const float* cz = L.cz + off;
   double acc = 0;
-  for (int k = h * ZC; k < (h + 1) * ZC; k++) {
+  for (int k = 0; k < TS; k++) {
     const int e = tidx(TS, i, j, k);
     const double dg = L.diag[off + e];
     double rv = 0;
@@ -53,6 +49,113 @@ __global__ void __launch_bounds__(TS* TS* res64_split<TS>())
   }
   acc = block_sum(acc);
   if (t == 0) partial[blockIdx.x] = acc;
+}
+
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+// The same on 16^3 tiles, which hold nearly all cells of a large grid.  Bound by memory: 32
+// bytes a cell (x 8, five floats in, one out).  All of a tile's loads are issued at once: x and the
+// couplings by asynchronous copies into shared memory, a_ii and b into registers, the
+// neighbours' x of faces to tiles of the same size.  Two CTAs of 92 KB share an SM.  With x
+// alone in shared memory and the rest loaded cell by cell behind a test of a_ii a
+// call took 1.86 ms (173 M cells, B200); 1.27 now.
+// Thread (i, j, h) owns half h of the z column (i, j).
+constexpr int RES16_NT = 512;
+constexpr size_t RES16_SMEM = 8 * 4096 + 3 * 4 * 4096 + 8 * 6 * 256;
+static __global__ void __launch_bounds__(RES16_NT, 2)
+    k_residual64_16(LevelView L, const int* __restrict__ tiles, const double* __restrict__ x,
+                    const float* __restrict__ b, float* __restrict__ r,
+                    double* __restrict__ partial) {
+  constexpr int TS = 16, N = TS * TS * TS, NF = TS * TS, ZC = N / RES16_NT, NQ = 6 * NF / RES16_NT;
+  extern __shared__ __align__(128) unsigned char smem[];
+  double* xs = reinterpret_cast<double*>(smem);
+  float* cs = reinterpret_cast<float*>(smem + 8 * N);  // cx, cy, cz
+  double* gs = reinterpret_cast<double*>(smem + 8 * N + 12 * N);
+  const int ti = tiles[blockIdx.x];
+  const int64_t off = L.tileOff[ti];
+  const int t = threadIdx.x, i = t % TS, j = (t / TS) % TS, h = t / NF;
+  // (a tile's arrays start on a multiple of 64 entries)
+#pragma unroll
+  for (int q = 0; q < N / 2 / RES16_NT; q++) {
+    const int e = 2 * (t + RES16_NT * q);
+    copy16_async(xs + e, x + off + e);
+  }
+#pragma unroll
+  for (int q = 0; q < 3 * N / 4 / RES16_NT; q++) {
+    const int d = q / (N / 4 / RES16_NT), e = 4 * (t + RES16_NT * (q % (N / 4 / RES16_NT)));
+    copy16_async(cs + d * N + e, (d == 0 ? L.cx : d == 1 ? L.cy : L.cz) + off + e);
+  }
+  float dg[ZC], bb[ZC];
+#pragma unroll
+  for (int k = 0; k < ZC; k++) dg[k] = L.diag[off + t % NF + NF * (h * ZC + k)];
+#pragma unroll
+  for (int k = 0; k < ZC; k++) bb[k] = b[off + t % NF + NF * (h * ZC + k)];
+  int kind[NQ];
+  int64_t no[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+    const int* F = L.face + ((size_t)ti * 6 + (t + RES16_NT * q) / NF) * FACE_INTS;
+    kind[q] = F[F_KIND];
+    no[q] = kind[q] == FACE_SAME ? L.tileOff[F[F_T0]] : 0;
+  }
+  double xn[NQ];
+  float cn[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+    const int g = t + RES16_NT * q, f = g / NF, dir = f >> 1, side = f & 1, a = g % TS,
+              c = (g / TS) % TS;
+    xn[q] = 0;
+    cn[q] = 0.f;
+    if (kind[q] == FACE_SAME) {
+      xn[q] = x[no[q] + plane_idx(TS, dir, side ? 0 : TS - 1, a, c)];
+      cn[q] = (dir == 0 ? L.cx : dir == 1 ? L.cy : L.cz)[(side ? no[q] : off) +
+                                                         plane_idx(TS, dir, 0, a, c)];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+    const int g = t + RES16_NT * q, f = g / NF;
+    gs[g] = kind[q] == FACE_SAME || kind[q] == FACE_NONE
+                ? (double)cn[q] * xn[q]
+                : ghost_sum<double, double>(L, x, ti, TS, f >> 1, f & 1, g % TS, (g / TS) % TS);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  const float *cx = cs, *cy = cs + N, *cz = cs + 2 * N;
+  double acc = 0;
+#pragma unroll
+  for (int m = 0; m < ZC; m++) {
+    const int k = h * ZC + m, e = tidx(TS, i, j, k);
+    double rv = 0;
+    if (dg[m] > 0) {
+      double S = 0;
+      S += (i > 0) ? (double)cx[e] * xs[e - 1] : gs[j + TS * k];
+      S += (i < TS - 1) ? (double)cx[e + 1] * xs[e + 1] : gs[NF + j + TS * k];
+      S += (j > 0) ? (double)cy[e] * xs[e - TS] : gs[2 * NF + i + TS * k];
+      S += (j < TS - 1) ? (double)cy[e + TS] * xs[e + TS] : gs[3 * NF + i + TS * k];
+      S += (k > 0) ? (double)cz[e] * xs[e - TS * TS] : gs[4 * NF + i + TS * j];
+      S += (k < TS - 1) ? (double)cz[e + TS * TS] * xs[e + TS * TS] : gs[5 * NF + i + TS * j];
+      rv = (double)bb[m] - ((double)dg[m] * xs[e] - S);
+    }
+    r[off + e] = (float)rv;
+    acc += rv * rv;
+  }
+  acc = block_sum(acc);
+  if (t == 0) partial[blockIdx.x] = acc;
+}
+
+template <int TS>
+void launch_residual64(const LevelView& L, const int* tiles, int count, const double* x,
+                       const float* b, float* r, double* partial, cudaStream_t st) {
+  if constexpr (TS == 16)
+    k_residual64_16<<<count, RES16_NT, RES16_SMEM, st>>>(L, tiles, x, b, r, partial);
+  else
+    k_residual64<TS><<<count, TS * TS, 0, st>>>(L, tiles, x, b, r, partial);
 }
 
 // x64 += e * unscale (all cells; e is 0 off the liquid)
