@@ -189,3 +189,46 @@ def test_packed_faces_change_no_bit(bsx0, nl, monkeypatch):
     for (ia, sa, pa), (ib, sb, pb) in zip(*out):
         assert sa == 0 and sb == 0 and ia == ib
         assert np.array_equal(pa, pb)
+
+
+@pytest.mark.parametrize("bsx0,nl", [(8, 2), (16, 3), (32, 2)])
+@pytest.mark.parametrize("n_pre,n_post", [(0, 2), (1, 1), (2, 2), (3, 1)])
+def test_vcycle_reads_nothing_of_an_earlier_one(bsx0, nl, n_pre, n_post):
+    """The first sweep of a level starts from x = 0 without x having been cleared: after other
+    V-cycles the result has the bits of a new context's first one."""
+    s = msbg_gpu.PressureScene(128, bsx0, nl, band=4.0, seed=3)
+    out = []
+    for earlier in (0, 2):
+        ctx = msbg_gpu.Context(0)
+        try:
+            ctx.pressure_prepare(s)
+            n = ctx.level_size(0)
+            rng = np.random.default_rng(17)
+            r = (rng.standard_normal(n) * (ctx.diagonal(0) > 0)).astype(np.float32)
+            for _ in range(earlier):
+                ctx.vcycle(1e3 * r[::-1].copy() * (ctx.diagonal(0) > 0), n_pre, n_post)
+            out.append(ctx.vcycle(r, n_pre, n_post))
+        finally:
+            ctx.close()
+    assert np.abs(out[0]).max() > 0
+    assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("first,second", [((128, 16, 3), (64, 16, 2)), ((64, 16, 2), (128, 8, 2)),
+                                          ((128, 32, 2), (128, 16, 2))])
+def test_prepare_over_another_problem(first, second):
+    """A problem's buffers take over those of the problem before it, of another size and other
+    blocks: the solution has the bits of a new context's."""
+    out = []
+    for problems in ((second,), (first, second), (second, first, second)):
+        ctx = msbg_gpu.Context(0)
+        try:
+            for res, bsx0, nl in problems:
+                ctx.pressure_prepare(msbg_gpu.PressureScene(res, bsx0, nl, band=4.0, seed=5))
+                info = ctx.pressure_solve(tol=1e-6, maxRefine=30)
+            out.append((info.status, info.iterations, ctx.pressure_download()))
+        finally:
+            ctx.close()
+    assert out[0][0] == 0
+    for o in out[1:]:
+        assert o[:2] == out[0][:2] and np.array_equal(o[2], out[0][2])
