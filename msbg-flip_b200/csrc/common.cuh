@@ -25,6 +25,11 @@ namespace msbg {
 // such a kernel calls pdl_wait before it touches what a predecessor wrote and before it returns, so that its
 // own completion says the same of all kernels before it.  Without the launch attribute both
 // are no-ops.
+// What a kernel of the chain writes changes while the next one is resident already.  So in a
+// kernel that calls pdl_wait no pointer to it is __restrict__ and no load of it is __ldg: both
+// say that nothing else writes there while the kernel runs, and let the compiler take the
+// non-coherent path or move the load above the wait.  Block lists, tile offsets and the
+// operator, which no kernel of a chain writes, may have either.
 __device__ __forceinline__ void pdl_go() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

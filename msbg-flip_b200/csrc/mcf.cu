@@ -188,9 +188,9 @@ __device__ __forceinline__ const T* xface_src(const T* pool, const T* xf, const 
 }
 
 template <int BSX, typename T>
-__device__ __forceinline__ void mcf_fill(float* tile, const T* __restrict__ pool,
-                                         const T* __restrict__ xf, const int* nbSlot,
-                                         float emptyVal, float fullVal, int tid) {
+__device__ __forceinline__ void mcf_fill(float* tile, const T* pool, const T* xf,
+                                         const int* nbSlot, float emptyVal, float fullVal,
+                                         int tid) {
   using Tl = McfTile<BSX>;
   constexpr int NV = Tl::NV, NT = Tl::NT, HP = Tl::HP;
   constexpr bool F32 = std::is_same<T, float>::value;
@@ -301,8 +301,8 @@ __device__ __forceinline__ void mcf_fill(float* tile, const T* __restrict__ pool
 
 // The 19-point update of one block from its tile, stored in place.
 template <int BSX, typename T, int XOFF = 2>
-__device__ __forceinline__ void mcf_compute(const float* tile, T* __restrict__ block,
-                                            T* __restrict__ xfOwn, float dt, int clamp01,
+__device__ __forceinline__ void mcf_compute(const float* tile, T* block,
+                                            T* xfOwn, float dt, int clamp01,
                                             int tid) {
   using Tl = McfTile<BSX, XOFF>;
   constexpr int RP = Tl::RP, PP = Tl::PP, HP = Tl::HP;
@@ -405,7 +405,7 @@ __host__ __device__ constexpr int mcf_ctas_per_sm() { return BSX == 8 ? 12 : BSX
 // before block k is computed.
 template <int BSX, typename T>
 __global__ void __launch_bounds__(BSX* BSX, mcf_ctas_per_sm<BSX>())
-    mcf_colour_kernel(T* __restrict__ pool, T* __restrict__ xf, const int* __restrict__ slotOf,
+    mcf_colour_kernel(T* pool, T* xf, const int* __restrict__ slotOf,
                       const int* __restrict__ list, int n, int nbx, int nby, int nbz,
                       float emptyVal, float fullVal, float dt, int clamp01,
                       int* __restrict__ errFlag) {
@@ -544,9 +544,9 @@ __device__ __forceinline__ float const_val(int ck, float emptyVal, float fullVal
   return ck == 1 ? emptyVal : fullVal;
 }
 
-__device__ __forceinline__ void halo_load(Halo& h, const float* __restrict__ pool,
-                                          const float* __restrict__ xf, const int* nbSlot,
-                                          float emptyVal, float fullVal, int tid) {
+__device__ __forceinline__ void halo_load(Halo& h, const float* pool, const float* xf,
+                                          const int* nbSlot, float emptyVal, float fullVal,
+                                          int tid) {
   const float* own = pool + (size_t)nbSlot[13] * Tl::NV;
   {  // y faces: y = -1 / 16, z in [0, 16), one x pair
     const int side = tid >> 7, r = tid & 127, z = r >> 3, x = 2 * (r & 7);
@@ -596,9 +596,8 @@ __device__ __forceinline__ void halo_store(const Halo& h, float* tile, int tid) 
 
 // The z = -1 and z = 16 planes: faces (x pairs, y in [-1, 16]) and the edges
 // along y (x = -1 / 16, y in [0, 16)), by asynchronous copies.
-__device__ __forceinline__ void zplanes_fill(float* tile, const float* __restrict__ pool,
-                                             const float* __restrict__ xf, const int* nbSlot,
-                                             float emptyVal, float fullVal, int tid) {
+__device__ __forceinline__ void zplanes_fill(float* tile, const float* pool, const float* xf,
+                                             const int* nbSlot, float emptyVal, float fullVal, int tid) {
   const float* own = pool + (size_t)nbSlot[13] * Tl::NV;
   constexpr int ROWS = BS + 2, PAIRS = 2 * ROWS * (BS / 2);  // 288
   for (int q = tid; q < PAIRS; q += Tl::NT) {
@@ -631,10 +630,9 @@ __device__ __forceinline__ void zplanes_fill(float* tile, const float* __restric
 }  // namespace tma
 
 __global__ void __launch_bounds__(256, 3)
-    mcf_colour_kernel_tma(const __grid_constant__ CUtensorMap map, float* __restrict__ pool,
-                          float* __restrict__ xf, const int* __restrict__ slotOf,
-                          const int* __restrict__ list, int n, int nbx, int nby, int nbz,
-                          float emptyVal, float fullVal, float dt, int clamp01,
+    mcf_colour_kernel_tma(const __grid_constant__ CUtensorMap map, float* pool, float* xf,
+                          const int* __restrict__ slotOf, const int* __restrict__ list, int n,
+                          int nbx, int nby, int nbz, float emptyVal, float fullVal, float dt, int clamp01,
                           int* __restrict__ errFlag) {
   using namespace tma;
   extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -77,7 +77,7 @@ __host__ __device__ __forceinline__ int plane_idx(int ts, int dir, int p, int a,
 // Sum over the neighbours across face (dir, side) of face cell (a,b) of tile
 // ti: coupling * x(neighbour), accumulated in AT.  x = vector of this level.
 template <typename XT, typename AT = float>
-__host__ __device__ __forceinline__ AT ghost_sum(const LevelView& L, const XT* __restrict__ x,
+__host__ __device__ __forceinline__ AT ghost_sum(const LevelView& L, const XT* x,
                                                  int ti, int ts, int dir, int side, int a,
                                                  int b) {
   const int* F = L.face + ((size_t)ti * 6 + dir * 2 + side) * FACE_INTS;

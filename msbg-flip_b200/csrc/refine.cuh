@@ -217,12 +217,12 @@ static __global__ void __launch_bounds__(1024) k_finalize_max(const double* __re
 
 // x64 += alpha d (FP64 accumulation of the FP32 direction); r -= alpha q;
 // partial |r|^2.  Skipped (norm only) after a breakdown.
-static __global__ void __launch_bounds__(VEC_BLOCK) k_axpy64_norm(double* __restrict__ x,
-                                                           float* __restrict__ r,
-                                                           const float* __restrict__ d,
-                                                           const float* __restrict__ q, int64_t n,
-                                                           const Scalars* __restrict__ s,
-                                                           double* __restrict__ partial) {
+static __global__ void __launch_bounds__(VEC_BLOCK) k_axpy64_norm(double* x,
+                                                           float* r,
+                                                           const float* d,
+                                                           const float* q, int64_t n,
+                                                           const Scalars* s,
+                                                           double* partial) {
   pdl_go();
   pdl_wait();
   const bool ok = s->status == 0;

@@ -82,10 +82,9 @@ constexpr size_t SMEM = sizeof(float) * ZERO_FLOATS + 3 * sizeof(TileRec) + 3 * 
 // without these values load a harmless word and ignore it).  With the packed
 // x faces xf of x (and L.cxf), an x face reads the neighbour's packed plane.
 template <typename VT>
-__device__ __forceinline__ void halo_load(const LevelView& L, const VT* __restrict__ x,
-                                          const VT* __restrict__ xf, const FaceRes& r, int dir,
-                                          int side, int a, int b, VT& xv, float& cv,
-                                          int zeroStart = 0) {
+__device__ __forceinline__ void halo_load(const LevelView& L, const VT* x, const VT* xf,
+                                          const FaceRes& r, int dir, int side, int a, int b,
+                                          VT& xv, float& cv, int zeroStart = 0) {
   const float* cd = dir == 0 ? L.cx : dir == 1 ? L.cy : L.cz;
   const VT* px = x;
   const float* pc = cd;
@@ -102,7 +101,7 @@ __device__ __forceinline__ void halo_load(const LevelView& L, const VT* __restri
     px = x + r.nOff + plane_idx(r.nts, dir, side ? 0 : r.nts - 1, r.oa + (a >> 1), r.ob + (b >> 1));
     pc = L.ifc + r.ifOwn + a + TS * b;
   }
-  xv = __ldg(px);
+  xv = *px;  // (not __ldg: the kernels before write x, see pdl_wait)
   cv = __ldg(pc);
 }
 
@@ -167,9 +166,8 @@ __device__ __forceinline__ VT* sraw_b(float* st) {
 // own, since a runtime test in the halo loads costs every sweep 2 %).
 template <typename VT, int NTH, bool ZERO>
 __global__ void __launch_bounds__(NTH, 1)
-    k_smooth_pipe16(LevelView L, int tileBase, int count, VT* __restrict__ x,
-                    const VT* __restrict__ b, int inner, int reverse, int* __restrict__ err,
-                    VT* __restrict__ xf, int zeroFlags) {
+    k_smooth_pipe16(LevelView L, int tileBase, int count, VT* x, const VT* b, int inner,
+                    int reverse, int* __restrict__ err, VT* xf, int zeroFlags) {
   using namespace pipe;
   const int zeroStart = ZERO ? zeroFlags : 0;
   static_assert(NTH == 1024, "the z-pair thread map covers a 16^3 tile with 1024 threads");
@@ -511,11 +509,9 @@ enum { APPLY_MATVEC = 0, APPLY_RESIDUAL = 1 };
 
 template <int MODE, typename VT, typename VC, int NTH>
 __global__ void __launch_bounds__(NTH, 1)
-    k_apply_pipe16(LevelView L, int tileBase, int count, const VT* __restrict__ x,
-                   const VT* __restrict__ b, VT* __restrict__ y,
-                   VC* __restrict__ bc, const int64_t* __restrict__ coarseOff,
-                   double* __restrict__ partial, int* __restrict__ err,
-                   const VT* __restrict__ xf) {
+    k_apply_pipe16(LevelView L, int tileBase, int count, const VT* x, const VT* b, VT* y,
+                   VC* bc, const int64_t* __restrict__ coarseOff, double* partial,
+                   int* __restrict__ err, const VT* xf) {
   using namespace pipe;
   constexpr int ZC = TS / (NTH / (TS * TS));  // cells of a thread's z column
   constexpr int NHALO = 6 * TS * TS;

@@ -49,7 +49,7 @@ enum {
 
 // Deterministic second stage: fixed-order sum of the CTA partials, then the
 // scalar step of PCG that depends on it.
-static __global__ void __launch_bounds__(1024) k_finalize(const double* __restrict__ partial, int n,
+static __global__ void __launch_bounds__(1024) k_finalize(const double* partial, int n,
                                                    Scalars* s, int what) {
   pdl_go();
   pdl_wait();
@@ -119,9 +119,9 @@ constexpr int VEC_GRID = 148 * 4, VEC_BLOCK = 512;
 inline bool vectors_dependent(int64_t n) { return n <= (8 << 20); }
 
 template <typename VA, typename VB>
-__global__ void __launch_bounds__(VEC_BLOCK) k_dot(const VA* __restrict__ a,
-                                                   const VB* __restrict__ b, int64_t n,
-                                                   double* __restrict__ partial) {
+__global__ void __launch_bounds__(VEC_BLOCK) k_dot(const VA* a,
+                                                   const VB* b, int64_t n,
+                                                   double* partial) {
   pdl_go();
   pdl_wait();
   double acc = 0;
@@ -136,11 +136,11 @@ __global__ void __launch_bounds__(VEC_BLOCK) k_dot(const VA* __restrict__ a,
 
 // x += alpha d; r -= alpha q; partial |r|^2.  Skipped (norm only) after a breakdown.
 template <typename VT>
-__global__ void __launch_bounds__(VEC_BLOCK) k_axpy_norm(VT* __restrict__ x, VT* __restrict__ r,
-                                                         const VT* __restrict__ d,
-                                                         const VT* __restrict__ q, int64_t n,
-                                                         const Scalars* __restrict__ s,
-                                                         double* __restrict__ partial) {
+__global__ void __launch_bounds__(VEC_BLOCK) k_axpy_norm(VT* x, VT* r,
+                                                         const VT* d,
+                                                         const VT* q, int64_t n,
+                                                         const Scalars* s,
+                                                         double* partial) {
   pdl_go();
   pdl_wait();
   const bool ok = s->status == 0;
@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(VEC_BLOCK) k_axpy_norm(VT* __restrict__ x, VT*
 
 // d = z + beta d
 template <typename VT>
-__global__ void __launch_bounds__(VEC_BLOCK) k_update_d(VT* __restrict__ d,
-                                                        const VT* __restrict__ z, int64_t n,
-                                                        const Scalars* __restrict__ s) {
+__global__ void __launch_bounds__(VEC_BLOCK) k_update_d(VT* d,
+                                                        const VT* z, int64_t n,
+                                                        const Scalars* s) {
   pdl_go();
   pdl_wait();
   if (s->status) return;
@@ -221,7 +221,7 @@ struct TileGeo {
 // Coupling times neighbour of face cell (a, b) of face (dir, side), as ghost_sum.
 template <int TS, typename VT>
 __device__ __forceinline__ float halo_term(const LevelView& L, const TileRec& r, int ti,
-                                           const VT* __restrict__ x, int dir, int side, int a,
+                                           const VT* x, int dir, int side, int a,
                                            int b, int zeroStart) {
   const FaceRes& F = r.f[2 * dir + side];
   const int kind = F.kind;
@@ -264,7 +264,7 @@ struct TileCells {
     }
   }
   __device__ __forceinline__ void load_x(const LevelView& L, const TileRec& r, int ti,
-                                         const VT* __restrict__ x, float* xs, int zeroStart = 0) {
+                                         const VT* x, float* xs, int zeroStart = 0) {
     const int t = threadIdx.x;
 #pragma unroll
     for (int q = 0; q < G::PER; q++) {
@@ -296,9 +296,9 @@ struct TileCells {
 // q = A d on tiles tileBase.., partial d.q per CTA.
 template <int TS, typename VT>
 __global__ void __launch_bounds__(TileGeo<TS>::NT) k_matvec_dot(LevelView L, int tileBase,
-                                                                const VT* __restrict__ d,
-                                                                VT* __restrict__ q,
-                                                                double* __restrict__ partial) {
+                                                                const VT* d,
+                                                                VT* q,
+                                                                double* partial) {
   using G = TileGeo<TS>;
   __shared__ float xs[G::P * G::P * G::P];
   const int ti = tileBase + blockIdx.x, t = threadIdx.x;
@@ -331,8 +331,8 @@ __global__ void __launch_bounds__(TileGeo<TS>::NT) k_matvec_dot(LevelView L, int
 // P^T) into the coarse right-hand side bc (vectors VT, coarse vectors VC).
 template <int TS, typename VT, typename VC>
 __global__ void __launch_bounds__(TileGeo<TS>::NT)
-    k_residual_restrict(LevelView L, int tileBase, const VT* __restrict__ x,
-                        const VT* __restrict__ b, VC* __restrict__ bc,
+    k_residual_restrict(LevelView L, int tileBase, const VT* x,
+                        const VT* b, VC* bc,
                         const int64_t* __restrict__ coarseOff) {
   using G = TileGeo<TS>;
   __shared__ float xs[G::P * G::P * G::P];
@@ -399,10 +399,10 @@ __global__ void __launch_bounds__(TS* TS) k_pack_cx_plane(const int64_t* __restr
 // 16^3 tiles the packed x faces xf (if given) are written too.
 template <int TS, typename VT, typename VC>
 __global__ void __launch_bounds__(TS* TS) k_prolong(LevelView L, const int* __restrict__ tiles,
-                                                    VT* __restrict__ x,
-                                                    const VC* __restrict__ xc,
+                                                    VT* x,
+                                                    const VC* xc,
                                                     const int64_t* __restrict__ coarseOff,
-                                                    float scale, VT* __restrict__ xf) {
+                                                    float scale, VT* xf) {
   constexpr int N = TS * TS * TS, NT = TS * TS;
   pdl_go();
   const int ti = tiles[blockIdx.x];
@@ -462,8 +462,8 @@ __global__ void __launch_bounds__(TS* TS) k_prolong(LevelView L, const int* __re
 // reverse=1: black then red (the adjoint order).  zeroStart: see pressure_kernels.cuh.
 template <int TS, typename VT>
 __global__ void __launch_bounds__(TileGeo<TS>::NT) k_smooth(LevelView L, int tileBase,
-                                                            VT* __restrict__ x,
-                                                            const VT* __restrict__ b, int inner,
+                                                            VT* x,
+                                                            const VT* b, int inner,
                                                             int reverse, int zeroStart) {
   using G = TileGeo<TS>;
   __shared__ float xs[G::P * G::P * G::P];
@@ -511,7 +511,7 @@ constexpr int COARSE_ROWS = 16, COARSE_PARTS = 32;
 template <typename VT>
 __global__ void __launch_bounds__(COARSE_ROWS* COARSE_PARTS)
     k_coarse_solve(const double* __restrict__ Ainv, int n, const int64_t* __restrict__ cells,
-                   const VT* __restrict__ b, VT* __restrict__ x) {
+                   const VT* b, VT* x) {
   __shared__ double bs[512];
   __shared__ double part[COARSE_PARTS][COARSE_ROWS];
   const int t = threadIdx.x, r = t % COARSE_ROWS, q = t / COARSE_ROWS;
