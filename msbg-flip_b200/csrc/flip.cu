@@ -125,7 +125,8 @@ __global__ void k_p2g_scatter(const msbg_flip_particle* __restrict__ p, int64_t 
 // P2G's 2.5 ms).  Here
 //   k_p2g_count  gives each particle its cell and its rank there, and counts the cells'
 //                particles and liquid ones; a particle with a finite position outside the
-//                grid reaches its boundary faces alone, and does so here;
+//                grid reaches its boundary faces alone, and does so here, as do those that a
+//                cell has beyond P2G_CELL_MAX;
 //   k_p2g_start, k_p2g_place  list the particles cell by cell (indices; the particles
 //                stay where they are);
 //   k_p2g_cells  a CTA per 8 x 8 x 4 cells, a thread per cell: a cell's particles reach 2 x 3 x
@@ -134,6 +135,10 @@ __global__ void k_p2g_scatter(const msbg_flip_particle* __restrict__ p, int64_t 
 //                offset at a time, in which no two threads meet, and from there to the
 //                grid with one float atomic per face and sum.
 // 0.73 ms for the four kernels.
+
+// A cell's particles that its thread sums: a chain of dependent loads, 0.4 us each, that its
+// CTA waits for; a clump of any size ends there.
+constexpr int P2G_CELL_MAX = 32;
 
 // The cell of a particle with a finite position; -1 outside the grid.
 __device__ __forceinline__ int64_t cell_of(const msbg_flip_particle& q, const GridF& g) {
@@ -154,8 +159,10 @@ __global__ void __launch_bounds__(256) k_p2g_count(const msbg_flip_particle* __r
     int2 at = make_int2((int)ci, 0);
     // low word particles, high word liquid ones
     if (ci >= 0) at.y = (int)atomicAdd(&cnt[ci], q.phase == 0 ? (1ull << 32) + 1 : 1ull);
+    const bool listed = ci >= 0 && (unsigned)at.y < P2G_CELL_MAX;
+    if (!listed) at.x = -1;
     place[k] = at;
-    if (finite && ci < 0) scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
+    if (finite && !listed) scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
   }
 }
 
@@ -170,7 +177,7 @@ __global__ void __launch_bounds__(1024) k_p2g_start(int64_t n,
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t c = blockIdx.x * (int64_t)1024 + threadIdx.x;
   const unsigned long long u = c < n ? cnt[c] : 0ull;
-  const int v = (int)(unsigned)u;
+  const int all = (int)(unsigned)u, v = min(all, P2G_CELL_MAX);
   int x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -192,7 +199,7 @@ __global__ void __launch_bounds__(1024) k_p2g_start(int64_t n,
   __syncthreads();
   if (c >= n) return;
   start[c] = v ? base + (w ? sum[w - 1] : 0) + x - v : 0;
-  mass[c] = (float)v;
+  mass[c] = (float)all;
   liq[c] = (int)(u >> 32);
 }
 
@@ -285,7 +292,7 @@ __global__ void __launch_bounds__(SUB_T, 3) k_p2g_cells(
   const int lx = t % SUB, ly = t / SUB % SUB, lz = t / (SUB * SUB);
   const int x = bx + lx, y = by + ly, z = bz + lz;
   const int64_t ci = g.idx(x, y, z);
-  const int m = (int)(unsigned)cnt[ci];
+  const int m = (int)min((unsigned)cnt[ci], (unsigned)P2G_CELL_MAX);
   if (!__syncthreads_or(m)) return;
   const int* list = perm + start[ci];
   const int at = (lx + 1) + FACE_ROW * ((ly + 1) + FACE_ROW * (lz + 1));

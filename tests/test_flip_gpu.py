@@ -170,3 +170,53 @@ def test_many_particles_in_any_order(res, bsx, order):
         assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("count", [31, 32, 33, 100000])
+def test_crowded_cells(count):
+    """P2G sums a cell in one thread only up to a number of particles: cells around that number,
+    and a clump that holds them all, against the restatement.  The call on the clump is no
+    slower than ten of the same number of particles spread out (and 20 ms).
+
+    A face sums up to N = 8 count + 64 terms in FP32, in an order of its own on either side:
+    each is off by at most N 2^-24 of the sum of the terms' sizes, so a velocity (a quotient of
+    two sums) by 2 N 2^-24 max|v|, and the two sides differ by at most twice that; 1e-5 is what
+    the other tests allow."""
+    import time
+
+    import torch
+
+    res, bsx = 64, 16
+    p = msbg_gpu.flip_particles(res, bsx, z_liquid=0.6, ppv=8, air_ppv=2, air_band=6, seed=3)
+    rng = np.random.default_rng(4)
+    cells = rng.integers(4, res - 4, (1 if count > 1000 else 500, 3))
+    extra = np.zeros(len(cells) * count, msbg_gpu.FLIP_PARTICLE)
+    extra["pos"] = np.repeat(cells, count, 0) + rng.uniform(0.01, 0.99, (len(extra), 3))
+    extra["vel"] = rng.standard_normal((len(extra), 3))
+    extra["phase"] = rng.integers(0, 2, len(extra))
+    spread = extra.copy()
+    spread["pos"] = rng.uniform(4, res - 4, (len(extra), 3))
+    both = [np.concatenate([p, e])[rng.permutation(len(p) + len(e))] for e in (extra, spread)]
+    ctx = msbg_gpu.Context(0)
+    try:
+        ctx.set_topology(res, res, res, bsx)
+        sec = []
+        for q in both[::-1]:
+            d = torch.from_numpy(q.view(np.uint8).copy()).cuda()
+            torch.cuda.synchronize()
+            for _ in range(4):
+                t = time.perf_counter()
+                ctx.flip_p2g_device(d.data_ptr(), len(q))
+                t = time.perf_counter() - t
+            sec.append(t)
+        assert sec[1] <= 0.02 + 10 * sec[0], sec
+        vel = ctx.flip_channel(msbg_gpu.FLIP_VEL, res ** 3)
+        beta = ctx.flip_channel(msbg_gpu.FLIP_BETA, res ** 3)
+        vel_o, mass_o, beta_o, _ = oracle.flip_p2g(res, bsx, both[0])
+        assert np.array_equal(ctx.flip_channel(msbg_gpu.FLIP_MASS, res ** 3), mass_o)
+        tol = 1e-5 + 4 * (8 * count + 64) * 2.0 ** -24
+        assert np.abs(vel - vel_o).max() <= tol * max(1.0, np.abs(both[0]["vel"]).max())
+        bad = np.abs(beta - beta_o) > tol * np.maximum(1e-3, np.abs(beta_o))
+        assert bad.mean() <= 1e-4, bad.sum()
+    finally:
+        ctx.close()
