@@ -61,6 +61,7 @@ struct SplatGeom {
   int nb[3];  // blocks per axis
   int sh;     // log2(bsx)
   float lo[3], hi[3];  // domain bounds of a particle position
+  int visits;  // up to how many particles of a chunk visit their voxels (k_splat_cubes)
   float rScan, rScanBsx, toBlock, distSqMax, distSqMaxInv, rParticle, nbDist;
 };
 
@@ -270,22 +271,59 @@ __device__ __forceinline__ int splat_bin(const SplatGeom& g, const int* __restri
   return (int)(start[ns + 1] - s0);
 }
 
-// Voxels gather their nearest particle (k_splat_cubes) where a particle's reach is at most
-// 4 voxels and many particles lie around a block, else particles visit their voxels
-// (k_splat_blocks).  A visit of a particle costs some 500 voxel tests whatever lies next to
-// it; a gather costs a block its bins and each voxel a search that ends at the first
-// particles.  The line (splat_many_min) is flat: 256, 1024 or 4096 particles around a 16^3
-// block gave 14.34, 14.29 and 14.24 ms in the case below.
+// A visit of a particle costs some 500 voxel tests (reach 4) whatever lies next to it; a gather
+// costs a block the sorting of its particles and each voxel a search that ends at the first ones.
+// Where a particle's reach is at most 4 voxels, k_splat_cubes looks at what reaches a cube and
+// does the one or the other, else k_splat_blocks lets all particles visit.  Clouds on 256^3 to
+// 1024^3, blocks of 8^3, 16^3 and 32^3 (B200, ms a call: visits alone; gathers alone; both by
+// count): the demo's 4096 x 4096 particles 28.2, 12.3, 11.9; 1 M spread evenly over 512^3 8.1,
+// 13.6, 2.6; 2 M over 256^3 3.8, 2.6, 2.5, and with a reach of 1 1.2, 1.5, 1.4.
 __host__ __device__ __forceinline__ bool splat_gather(const SplatGeom& g) {
   return g.rScan <= 4.f;
 }
-template <int BSX>
-__host__ __device__ constexpr int splat_many_min() { return 4 * BSX * BSX; }
+
+// A particle's visit by a warp: the voxels of the box B0 .. B0 + N - 1 in its scan box, the lanes
+// over the (x, y) columns, each marching the z range that can lie within rScan (a bound one
+// voxel wider than the sphere's chord; the exact test decides inside it).  tile holds the FP32 bits
+// of the smallest d^2.
+template <int N>
+__device__ __forceinline__ void splat_visit(const SplatGeom& g, const float p[3], int abortIdx,
+                                            const int B0[3], int lane, uint32_t* tile) {
+  int i1[3], i2[3], c1[3], c2[3];
+  scan_box(g, p, i1, i2);
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    c1[q] = max(i1[q], B0[q]);
+    c2[q] = min(i2[q], B0[q] + N - 1);
+  }
+  const float p0[3] = {__fsub_rn(p[0], 0.5f), __fsub_rn(p[1], 0.5f), __fsub_rn(p[2], 0.5f)};
+  const int wx = c2[0] - c1[0] + 1, wy = c2[1] - c1[1] + 1;
+  const int fx = i2[0] - i1[0] + 1, fy = i2[1] - i1[1] + 1;
+  for (int t = lane; t < wx * wy; t += 32) {
+    const int ly = t / wx, ix = c1[0] + (t - ly * wx), iy = c1[1] + ly;
+    const float dx = __fsub_rn((float)ix, p0[0]), dy = __fsub_rn((float)iy, p0[1]);
+    const float zr2 = g.distSqMax - (dx * dx + dy * dy);
+    if (zr2 < -0.5f) continue;
+    const float h = sqrtf(fmaxf(zr2, 0.f)) + 1.f;
+    const int z1 = max(c1[2], (int)ceilf(p0[2] - h)), z2 = min(c2[2], (int)floorf(p0[2] + h));
+    uint32_t* col = tile + (ix - B0[0]) + N * (iy - B0[1]);
+    for (int iz = z1; iz <= z2; iz++) {
+      const float dz = __fsub_rn((float)iz, p0[2]);
+      const float distSq = splat_dist_sq(dx, dy, dz);
+      if (distSq > g.distSqMax) continue;
+      if (abortIdx != INT_MAX &&
+          ((iz - i1[2]) * fy + (iy - i1[1])) * fx + (ix - i1[0]) >= abortIdx)
+        continue;
+      uint32_t* cell = col + N * N * (iz - B0[2]);
+      const uint32_t bits = __float_as_uint(distSq);
+      if (bits < *cell) atomicMin(cell, bits);
+    }
+  }
+}
 
 // One CTA per value block: the minimum squared distance of the particles
 // binned in its 27-block neighbourhood, in shared memory, then quantised and
-// finalised (or left raw) into the channel's pool; for blocks with few particles
-// around them (splat_gather tells).  The quantisation
+// finalised (or left raw) into the channel's pool (splat_gather tells).  The quantisation
 // round(d^2 / rScan^2 * 65535) is monotonic in d^2, so quantising the minimum
 // equals the reference's minimum of quantised values; the tile holds the
 // FP32 bits of d^2 (non-negative floats order like their bit patterns), +inf
@@ -303,17 +341,6 @@ __global__ void __launch_bounds__(256, 4) k_splat_blocks(SplatGeom g, const int*
   const int bx = bid % g.nb[0], by = (bid / g.nb[0]) % g.nb[1],
             bz = bid / (g.nb[0] * g.nb[1]);
   const int B0[3] = {bx * BSX, by * BSX, bz * BSX};
-  if (splat_gather(g)) {
-    __shared__ int around;
-    if (threadIdx.x < 32) {
-      int64_t s0;
-      const int n = threadIdx.x < 27 ? splat_bin(g, slot, start, bx, by, bz, threadIdx.x, s0) : 0;
-      const int all = __reduce_add_sync(0xffffffffu, n);
-      if (threadIdx.x == 0) around = all;
-    }
-    __syncthreads();
-    if (around >= splat_many_min<BSX>()) return;  // k_splat_cubes has it
-  }
   constexpr uint32_t FAR = 0x7f800000u;  // +inf
   for (int v = threadIdx.x; v < NV; v += blockDim.x) tile[v] = FAR;
   __syncthreads();
@@ -347,40 +374,7 @@ __global__ void __launch_bounds__(256, 4) k_splat_blocks(SplatGeom g, const int*
         const float p[3] = {__shfl_sync(0xffffffffu, P.x, k), __shfl_sync(0xffffffffu, P.y, k),
                             __shfl_sync(0xffffffffu, P.z, k)};
         const int abortIdx = __float_as_int(__shfl_sync(0xffffffffu, P.w, k));
-        int i1[3], i2[3], c1[3], c2[3];
-        scan_box(g, p, i1, i2);
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-          c1[q] = max(i1[q], B0[q]);
-          c2[q] = min(i2[q], B0[q] + BSX - 1);
-        }
-        const float p0[3] = {__fsub_rn(p[0], 0.5f), __fsub_rn(p[1], 0.5f),
-                             __fsub_rn(p[2], 0.5f)};
-        const int wx = c2[0] - c1[0] + 1, wy = c2[1] - c1[1] + 1;
-        const int fx = i2[0] - i1[0] + 1, fy = i2[1] - i1[1] + 1;
-        // lanes over the (x, y) columns of the clipped box, each marching the
-        // z range that can lie within rScan (a bound one voxel wider than
-        // the sphere's chord; the exact test decides inside it)
-        for (int t = lane; t < wx * wy; t += 32) {
-          const int ly = t / wx, ix = c1[0] + (t - ly * wx), iy = c1[1] + ly;
-          const float dx = __fsub_rn((float)ix, p0[0]), dy = __fsub_rn((float)iy, p0[1]);
-          const float zr2 = g.distSqMax - (dx * dx + dy * dy);
-          if (zr2 < -0.5f) continue;
-          const float h = sqrtf(fmaxf(zr2, 0.f)) + 1.f;
-          const int z1 = max(c1[2], (int)ceilf(p0[2] - h)), z2 = min(c2[2], (int)floorf(p0[2] + h));
-          uint32_t* col = tile + (ix - B0[0]) + BSX * (iy - B0[1]);
-          for (int iz = z1; iz <= z2; iz++) {
-            const float dz = __fsub_rn((float)iz, p0[2]);
-            const float distSq = splat_dist_sq(dx, dy, dz);
-            if (distSq > g.distSqMax) continue;
-            if (abortIdx != INT_MAX &&
-                ((iz - i1[2]) * fy + (iy - i1[1])) * fx + (ix - i1[0]) >= abortIdx)
-              continue;
-            uint32_t* cell = col + BSX * BSX * (iz - B0[2]);
-            const uint32_t bits = __float_as_uint(distSq);
-            if (bits < *cell) atomicMin(cell, bits);
-          }
-        }
+        splat_visit<BSX>(g, p, abortIdx, B0, lane, tile);
       }
     }
   }
@@ -395,7 +389,7 @@ __global__ void __launch_bounds__(256, 4) k_splat_blocks(SplatGeom g, const int*
   }
 }
 
-// Blocks with many particles around them: a CTA per cube of CUBE^3 voxels (a block, or an
+// A CTA per cube of CUBE^3 voxels (a block, or an
 // eighth of a 32^3 block).  The particles of the 27 bins that reach the cube come in chunks
 // of up to CHUNK; a chunk is sorted by cell in shared memory (a cell: a voxel's unit cube;
 // W^3 of them, the cube and 4 around it), and every voxel searches the cells around it for
@@ -408,8 +402,11 @@ __global__ void __launch_bounds__(256, 4) k_splat_blocks(SplatGeom g, const int*
 // exactly (both differences are exact), so nothing that could lower the minimum is skipped.
 // The scan box and a scan that stops early matter only at the edge of the reach and for marked
 // particles; those look the particle up again.
-// The demo's 4096 x 4096 particles at 1024^3 (B200): 28.4 ms a call with particles visiting
-// voxels everywhere, 13.1 with this kernel but masks of the occupied rows alone, 10.4 when
+// A chunk of few particles (g.visits: 256 at reach 4, where half or twice as many cost up to 1.8
+// of it, and 512 at reaches up to 2) is not sorted: its particles visit their voxels, in a
+// function of its own, since the search needs all registers.
+// The demo's 4096 x 4096 particles, moved within their cells, at 1024^3 (B200): 28.4 ms a call
+// with particles visiting voxels everywhere, 13.1 with this kernel but masks of the occupied rows alone, 10.4 when
 // only the voxels with a cell in reach are searched, 10.0 when the warps share those as they go.
 constexpr int CUBE_T = 512, CHUNK = 2048;
 
@@ -439,6 +436,21 @@ __device__ __noinline__ bool splat_in_scan(const SplatGeom& g, const float4* __r
   return ((vz - i1[2]) * fy + (vy - i1[1])) * fx + (vx - i1[0]) < end;
 }
 
+// The n particles of a chunk visit their voxels, a warp each.
+template <int CUBE>
+__device__ __noinline__ void splat_visits(const SplatGeom& g, const float4* buf, int n,
+                                          const float4* __restrict__ sorted, int x0, int y0, int z0,
+                                          float* best) {
+  const int C0[3] = {x0, y0, z0};
+  for (int i = threadIdx.x >> 5; i < n; i += CUBE_T / 32) {
+    const float4 q = buf[i];
+    const float p[3] = {q.x, q.y, q.z};
+    const int j = __float_as_int(q.w);  // marked: its scan stops early
+    splat_visit<CUBE>(g, p, j >= 0 ? INT_MAX : __float_as_int(sorted[j & 0x7fffffff].w), C0,
+                      threadIdx.x & 31, reinterpret_cast<uint32_t*>(best));
+  }
+}
+
 template <int BSX, int CUBE>
 __global__ void __launch_bounds__(CUBE_T, 2)
     k_splat_cubes(SplatGeom g, const int* __restrict__ slot, const int* __restrict__ vbid,
@@ -448,7 +460,7 @@ __global__ void __launch_bounds__(CUBE_T, 2)
   constexpr int W = C::W, SUBS = BSX / CUBE, NV = BSX * BSX * BSX;
   extern __shared__ __align__(16) unsigned char smem[];
   float4* buf = reinterpret_cast<float4*>(smem);                   // p - 1/2, index of the particle
-  float* best = reinterpret_cast<float*>(buf + CHUNK);             // [VOX] each its thread's own
+  float* best = reinterpret_cast<float*>(buf + CHUNK);             // [VOX]
   // bit x: particles within reach of a voxel's x in cell row (y, z); in the rows within
   // reach of its y; in the planes within reach of its z
   uint32_t* inRow = reinterpret_cast<uint32_t*>(best + C::VOX);    // [W z][W y]
@@ -470,7 +482,6 @@ __global__ void __launch_bounds__(CUBE_T, 2)
   if (w == 0) {
     int64_t s0 = 0;
     const int n = lane < 27 ? splat_bin(g, slot, start, bx, by, bz, lane, s0) : 0;
-    const int all = __reduce_add_sync(0xffffffffu, n);
     // (bins out of a sub-cube's reach are left out)
     const int d[3] = {lane % 3 - 1, lane / 3 % 3 - 1, lane / 9 - 1};
     bool near = true;
@@ -488,19 +499,24 @@ __global__ void __launch_bounds__(CUBE_T, 2)
       binEnd[lane] = x;
     }
     if (lane == 31) {
-      total = all >= splat_many_min<BSX>() ? x : -1;
+      total = x;
       nBuf = 0;
     }
   }
   __syncthreads();
-  if (total < 0) return;  // k_splat_blocks has it
   const float none = __uint_as_float(__float_as_uint(g.distSqMax) + 1u);
   // nearer than this a voxel is inside the scan box whatever the rounding of its bounds
   const float in = fmaxf(g.rScan - (1e-4f + 2e-6f * (float)max(g.s[0], max(g.s[1], g.s[2]))), 0.f);
   const float edge = in * in;
   for (int v = tid; v < C::VOX; v += CUBE_T) best[v] = none;
+  __syncthreads();
 
   auto flush = [&](int n) {
+    if (n <= g.visits) {
+      splat_visits<CUBE>(g, buf, n, sorted, C0[0], C0[1], C0[2], best);
+      __syncthreads();  // the chunk is read
+      return;
+    }
     for (int i = tid; i < (C::CELLS + 2) / 2; i += CUBE_T) cnt[i] = 0u;
     for (int i = tid; i < W * W; i += CUBE_T) inRow[i] = 0u;
     if (tid == 0) nReached = nTaken = 0;
@@ -682,19 +698,21 @@ template <int BSX>
 cudaError_t launch_blocks(const SplatGeom& g, const int* slot, const int* vbid,
                           const int64_t* start, const float4* sorted, uint16_t* pool,
                           int64_t nValue, int raw, cudaStream_t st) {
-  const size_t smem = sizeof(uint32_t) * BSX * BSX * BSX;
-  cudaError_t e = cudaFuncSetAttribute(k_splat_blocks<BSX>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_splat_blocks<BSX><<<(unsigned)nValue, 256, smem, st>>>(g, slot, vbid, start, sorted, pool,
-                                                           raw);
   if (splat_gather(g)) {
     constexpr int CUBE = BSX < 16 ? BSX : 16, SUBS = BSX / CUBE;
-    e = cudaFuncSetAttribute(k_splat_cubes<BSX, CUBE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SplatCube<CUBE>::SMEM);
+    const cudaError_t e = cudaFuncSetAttribute(k_splat_cubes<BSX, CUBE>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)SplatCube<CUBE>::SMEM);
     if (e != cudaSuccess) return e;
     k_splat_cubes<BSX, CUBE><<<(unsigned)nValue * SUBS * SUBS * SUBS, CUBE_T,
                                SplatCube<CUBE>::SMEM, st>>>(g, slot, vbid, start, sorted, pool, raw);
+  } else {
+    const size_t smem = sizeof(uint32_t) * BSX * BSX * BSX;
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_splat_blocks<BSX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_splat_blocks<BSX><<<(unsigned)nValue, 256, smem, st>>>(g, slot, vbid, start, sorted, pool,
+                                                             raw);
   }
   return cudaGetLastError();
 }
@@ -776,6 +794,7 @@ int splat_run(msbg_gpu_ctx* ctx, int chan, const float* pos, int64_t n,
   g.toBlock = 1.0f / (float)bsx;
   g.distSqMax = g.rScan * g.rScan;
   g.distSqMaxInv = 1.0f / g.distSqMax;
+  g.visits = (int)std::min(512.f, 1024.f / g.rScan);
 
   const float* dpos = pos;
   if (!onDevice && n > 0) {

@@ -202,3 +202,16 @@ def test_gpu_dense_clumps_and_reaches(bsx, r_particle, nb_dist):
     kind[rng.choice(drop, len(drop) // 5, replace=False)] = 2
     _, fin = gpu_splat(res3, bsx, pos, kind=kind, **kw)
     assert np.array_equal(fin, oracle.splat(res3, bsx, kind, pos, r_particle, nb_dist))
+
+
+@pytest.mark.parametrize("bsx", [8, 16, 32])
+@pytest.mark.parametrize("count", [0, 1, 60])
+def test_gpu_few_particles_among_value_blocks(bsx, count):
+    """Blocks with a few particles around them, and with none: most of a grid whose blocks all
+    hold values."""
+    res3 = (64, 96, 128)
+    rng = np.random.default_rng(23)
+    pos = (rng.uniform(0, 1, (count, 3)) * np.array(res3) * 0.999).astype(np.float32)
+    kind = np.ones((64 // bsx) * (96 // bsx) * (128 // bsx), np.int8)
+    _, fin = gpu_splat(res3, bsx, pos, kind=kind)
+    assert np.array_equal(fin, oracle.splat(res3, bsx, kind, pos, 2.0, 2.0))
