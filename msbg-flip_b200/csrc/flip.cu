@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(256) k_pair_channels(const float* __restrict__
 }
 
 // (vel, velOld) of component d at a position, trilinear.  The index of the block
-// layout is a sum of one term per axis; a corner outside the grid reads 0.
+// layout is a sum of one term per axis; a corner outside the grid counts as 0.
 template <bool PAIR>
 __device__ __forceinline__ void interp_comp(const GridF& g, const float* __restrict__ vel,
                                             const float* __restrict__ velOld,
@@ -461,10 +461,16 @@ __device__ __forceinline__ void interp_comp(const GridF& g, const float* __restr
 #pragma unroll
   for (int c = 0; c < 8; c++) {
     const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
+    const bool in = vx[dx] && vy[dy] && vz[dz];
     float2 v = make_float2(0.f, 0.f);
-    if (vx[dx] && vy[dy] && vz[dz]) {
-      const int64_t i = 3 * (ox[dx] + oy[dy] + oz[dz]) + d;
-      v = PAIR ? pair[i] : make_float2(vel[i], velOld[i]);
+    if (PAIR) {
+      if (in) v = pair[3 * (ox[dx] + oy[dy] + oz[dz]) + d];
+    } else {
+      // no branch around the loads, so that all are in flight together (4 M particles in no order
+      // on 128^3 cells: 0.69 -> 0.59 ms); pairs are faster with it
+      const int64_t i = in ? 3 * (ox[dx] + oy[dy] + oz[dz]) + d : 0;
+      v = make_float2(vel[i], velOld[i]);
+      if (!in) v = make_float2(0.f, 0.f);
     }
     const float w = __fmul_rn(__fmul_rn(dx ? fx : ex, dy ? fy : ey), dz ? fz : ez);
     pic = __fadd_rn(pic, __fmul_rn(w, v.x));
@@ -539,10 +545,14 @@ int state_of(msbg_gpu_ctx* ctx, FlipState** out, GridF& g) {
 
 int grid_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 32); }
 
-// From how many particles on P2G goes cell by cell and G2P orders them (below, the extra
-// launches cost more than they save), and from how many particles per voxel on G2P lays
-// the channels side by side first (48 bytes per voxel against half the loads).
-constexpr int64_t FLIP_MANY = 1 << 16, FLIP_PAIR_RATIO = 2;
+// From how many particles on P2G goes cell by cell (below, the extra launches cost more than they
+// save).
+constexpr int64_t FLIP_MANY = 1 << 16;
+// From how many particles on G2P looks whether it should order them (five launches, 10 us, where
+// it should not), and lays the channels side by side first (48 bytes per voxel against half the
+// loads), if there is at least one particle per G2P_PAIR_VOXELS voxels: 4 M particles on 128^3
+// cells take 0.16 ms either way in cell order, 0.39 against 0.59 ms in none.
+constexpr int64_t G2P_ORDER_MANY = 1 << 19, G2P_PAIR_MANY = 1 << 16, G2P_PAIR_VOXELS = 2;
 
 }  // namespace
 
@@ -653,13 +663,13 @@ int flip_g2p(msbg_gpu_ctx* ctx, msbg_flip_particle* particles, int64_t np, float
     dp = S->parts.as<msbg_flip_particle>();
   }
   BinsOrder order;
-  if (np >= FLIP_MANY)
+  if (np >= G2P_ORDER_MANY)
     MSBG_CUDA_TRY(ctx, bins_build(S->lists, dp, np, BinsGrid{g.sx, g.sy, g.sz, g.sh, g.nbx, g.nby},
-                                  ctx->nb(), st, order));
+                                  ctx->nb(), 24.0 * (double)(S->n / ctx->nb()), st, order));
   const float* vel = S->vel.as<float>();
   const float* velOld = S->velOld.as<float>();
   float2* pair = nullptr;
-  if (np >= FLIP_MANY && np * FLIP_PAIR_RATIO >= S->n) {
+  if (np >= G2P_PAIR_MANY && np * G2P_PAIR_VOXELS >= S->n) {
     if (S->acc.ensure(24 * (size_t)S->n) == cudaSuccess) {
       pair = S->acc.as<float2>();
       k_pair_channels<<<grid_blocks(3 * S->n), 256, 0, st>>>(vel, velOld, 3 * S->n, pair);

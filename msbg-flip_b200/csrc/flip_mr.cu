@@ -458,9 +458,9 @@ __global__ void __launch_bounds__(256)
 
 int grid_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 32); }
 
-// From how many particles on G2P orders them: below, the four launches cost more than
-// a gather out of order does.
-constexpr int64_t MR_BINS_MIN = 1 << 16;
+// From how many particles on G2P looks whether it should order them.  As they come and ordered
+// (512^3, 3 levels, 16^3 blocks, in no order, B200): 1 M 193 and 206 us, 4 M 658 and 575.
+constexpr int64_t MR_BINS_MIN = 1 << 21;
 
 // One of the two interleaved channels: into it (get = 0) or out of it.
 __global__ void __launch_bounds__(256) k_mr_channel(float2* __restrict__ vel, int which,
@@ -645,7 +645,7 @@ int flip_g2p_mr(msbg_gpu_ctx* ctx, msbg_flip_particle* particles, int64_t np, fl
   BinsOrder order;
   if (np >= MR_BINS_MIN)
     MSBG_CUDA_TRY(ctx, bins_build(S->scratch, dp, np, BinsGrid{g.sx, g.sy, g.sz, g.sh0, g.nbx, g.nby},
-                                  ctx->nb(), st, order));
+                                  ctx->nb(), 26.0 * (double)S->n / (double)ctx->nb(), st, order));
   k_g2p_mr<<<grid_blocks(2 * np), 256, 0, st>>>(dp, np, g, S->vel.as<float2>(), order, flipAlpha,
                                             (double)la, (double)lb);
   MSBG_CUDA_TRY(ctx, cudaGetLastError());

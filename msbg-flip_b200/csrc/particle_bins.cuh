@@ -3,10 +3,11 @@
 //
 // A gather from a grid of a few hundred MB reads about 20 sectors per particle.  Particles
 // that a program keeps near block order find them in L1 and L2; particles in no order pull
-// each of them from DRAM.  The particles themselves are not moved: `perm` lists their indices
-// block by block, built per call from their positions.
+// each of them from DRAM, if the blocks that they lie in exceed L2.  The particles themselves
+// are not moved: `perm` lists their indices block by block, built per call from their positions.
 //   k_bins_sample  looks at up to 4096 groups of 32 consecutive particles; where most groups
-//                  lie in more than 8 blocks the particles count as scattered
+//                  lie in more than 8 blocks, and all of them in more blocks than L2 holds, the
+//                  particles count as scattered
 //   k_bins_count, k_bins_start, k_bins_place  a counting sort by block (the bins in no
 //                  order of their own); they return at once when the particles are not
 //                  scattered, and the gather then takes them as they come
@@ -14,8 +15,9 @@
 #pragma once
 
 // Scratch of an order: [np] rank of a particle in its block, [np] perm, [nb] particles per
-// block, then their first entries in perm, [2] scattered groups, cursor of the bins.
-inline size_t bins_bytes(int64_t np, int64_t nb) { return 4 * (size_t)(2 * np + nb + 2); }
+// block, then their first entries in perm, [nb] blocks seen in the sample, [3] scattered groups,
+// cursor of the bins, number of blocks seen.
+inline size_t bins_bytes(int64_t np, int64_t nb) { return 4 * (size_t)(2 * np + 2 * nb + 3); }
 
 constexpr int BINS_GROUPS = 4096;
 
@@ -30,35 +32,43 @@ struct BinsGrid {
   }
 };
 
-__device__ __forceinline__ bool bins_scattered(const int* flag, int groups) {
-  return flag[0] * 2 > groups;
+// What the sample has to show: of how many groups more than half lie in many blocks, and how
+// many blocks are more than L2 holds.
+struct BinsRule {
+  int groups, blocks;
+};
+__device__ __forceinline__ bool bins_scattered(const int* flag, BinsRule r) {
+  return flag[0] * 2 > r.groups && flag[2] >= r.blocks;
 }
 
 __global__ void __launch_bounds__(256) k_bins_sample(const msbg_flip_particle* __restrict__ p,
                                                      int64_t np, BinsGrid g, int groups,
-                                                     int* __restrict__ flag) {
+                                                     int* seen, int* flag) {
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= groups) return;
   const msbg_flip_particle& q = p[(np / 32) * w / groups * 32 + lane];
-  const unsigned peers = __match_any_sync(0xffffffffu, g.block(q.pos[0], q.pos[1], q.pos[2]));
-  const unsigned first = __ballot_sync(0xffffffffu, __ffs(peers) - 1 == lane);
-  if (lane == 0 && __popc(first) > 8) atomicAdd(flag, 1);
+  const int b = g.block(q.pos[0], q.pos[1], q.pos[2]);
+  const unsigned peers = __match_any_sync(0xffffffffu, b);
+  const bool mine = __ffs(peers) - 1 == lane;
+  const unsigned first = __ballot_sync(0xffffffffu, mine);
+  if (lane == 0 && __popc(first) > 8) atomicAdd(&flag[0], 1);
+  if (mine && !seen[b] && !atomicExch(&seen[b], 1)) atomicAdd(&flag[2], 1);
 }
 
 __global__ void __launch_bounds__(256) k_bins_count(const msbg_flip_particle* __restrict__ p,
-                                                    int64_t np, BinsGrid g, int groups,
+                                                    int64_t np, BinsGrid g, BinsRule rule,
                                                     const int* __restrict__ flag,
                                                     int* __restrict__ cnt, int* __restrict__ rank) {
-  if (!bins_scattered(flag, groups)) return;
+  if (!bins_scattered(flag, rule)) return;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
        k += (int64_t)gridDim.x * blockDim.x)
     rank[k] = atomicAdd(&cnt[g.block(p[k].pos[0], p[k].pos[1], p[k].pos[2])], 1);
 }
 
 // Counts to first entries: a CTA's 1024 blocks back to back, the CTAs in any order.
-__global__ void __launch_bounds__(1024) k_bins_start(int64_t nb, int groups, int* __restrict__ flag,
+__global__ void __launch_bounds__(1024) k_bins_start(int64_t nb, BinsRule rule, int* __restrict__ flag,
                                                      int* __restrict__ cnt) {
-  if (!bins_scattered(flag, groups)) return;
+  if (!bins_scattered(flag, rule)) return;
   __shared__ int sum[32], base;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t b = blockIdx.x * (int64_t)1024 + threadIdx.x;
@@ -86,12 +96,12 @@ __global__ void __launch_bounds__(1024) k_bins_start(int64_t nb, int groups, int
 }
 
 __global__ void __launch_bounds__(256) k_bins_place(const msbg_flip_particle* __restrict__ p,
-                                                    int64_t np, BinsGrid g, int groups,
+                                                    int64_t np, BinsGrid g, BinsRule rule,
                                                     const int* __restrict__ flag,
                                                     const int* __restrict__ start,
                                                     const int* __restrict__ rank,
                                                     int* __restrict__ perm) {
-  if (!bins_scattered(flag, groups)) return;
+  if (!bins_scattered(flag, rule)) return;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
        k += (int64_t)gridDim.x * blockDim.x)
     perm[start[g.block(p[k].pos[0], p[k].pos[1], p[k].pos[2])] + rank[k]] = (int)k;
@@ -101,19 +111,30 @@ __global__ void __launch_bounds__(256) k_bins_place(const msbg_flip_particle* __
 struct BinsOrder {
   const int* perm = nullptr;
   const int* flag = nullptr;
-  int groups = 0;
+  BinsRule rule{0, 0};
   __device__ __forceinline__ const int* get() const {
-    return perm && bins_scattered(flag, groups) ? perm : nullptr;
+    return perm && bins_scattered(flag, rule) ? perm : nullptr;
   }
 };
 
+// From how many bytes of the blocks in use on an order pays.  B200 (126 MB of L2), G2P of 4 M
+// particles in no order, as they come and ordered: on 160^3 cells (98 MB) 0.43 and 0.76 ms, on
+// 192^3 (170 MB) 0.59 and 0.69, on 256^3 (403 MB) 1.47 and 0.63; of 0.5 M in few of the cells of
+// 256^3 0.20 and 0.10, of 4 M in an eighth of them 0.51 and 1.43.
+constexpr double BINS_BYTES = 300e6;
+
 // Builds the order of np device particles on stream st, in scratch memory that the gather
-// reads.  Without enough device memory the particles are taken as they come.
+// reads; blockBytes: what a gather reads of a block, on average.  Without enough device memory
+// the particles are taken as they come.
 inline cudaError_t bins_build(DeviceBuffer& scratch, const msbg_flip_particle* p, int64_t np,
-                              const BinsGrid& g, int64_t nb, cudaStream_t st, BinsOrder& out) {
+                              const BinsGrid& g, int64_t nb, double blockBytes, cudaStream_t st,
+                              BinsOrder& out) {
   out = BinsOrder();
   const int groups = (int)std::min<int64_t>(np / 32, BINS_GROUPS);
-  if (groups < 1 || np > INT_MAX || nb > INT_MAX) return cudaSuccess;
+  if (groups < 1 || np > INT_MAX || nb > INT_MAX || (double)nb * blockBytes < BINS_BYTES)
+    return cudaSuccess;
+  // (no more blocks than the sample can see)
+  const BinsRule rule{groups, (int)std::min(BINS_BYTES / blockBytes, 8.0 * groups)};
   if (scratch.ensure(bins_bytes(np, nb)) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
@@ -121,16 +142,18 @@ inline cudaError_t bins_build(DeviceBuffer& scratch, const msbg_flip_particle* p
   int* rank = scratch.as<int>();
   int* perm = rank + np;
   int* cnt = perm + np;
-  int* flag = cnt + nb;
-  const cudaError_t e = cudaMemsetAsync(cnt, 0, 4 * (size_t)(nb + 2), st);
+  int* seen = cnt + nb;
+  int* flag = seen + nb;
+  const cudaError_t e = cudaMemsetAsync(cnt, 0, 4 * (size_t)(2 * nb + 3), st);
   if (e != cudaSuccess) return e;
-  const int grid = (int)std::min<int64_t>((np + 255) / 256, 148 * 32);
-  k_bins_sample<<<(groups * 32 + 255) / 256, 256, 0, st>>>(p, np, g, groups, flag);
-  k_bins_count<<<grid, 256, 0, st>>>(p, np, g, groups, flag, cnt, rank);
-  k_bins_start<<<(unsigned)((nb + 1023) / 1024), 1024, 0, st>>>(nb, groups, flag, cnt);
-  k_bins_place<<<grid, 256, 0, st>>>(p, np, g, groups, flag, cnt, rank, perm);
+  // (few CTAs at the smaller sizes: where there is no order to make, they start to return at once)
+  const int grid = (int)std::min<int64_t>((np + 2047) / 2048, 148 * 32);
+  k_bins_sample<<<(groups * 32 + 255) / 256, 256, 0, st>>>(p, np, g, groups, seen, flag);
+  k_bins_count<<<grid, 256, 0, st>>>(p, np, g, rule, flag, cnt, rank);
+  k_bins_start<<<(unsigned)((nb + 1023) / 1024), 1024, 0, st>>>(nb, rule, flag, cnt);
+  k_bins_place<<<grid, 256, 0, st>>>(p, np, g, rule, flag, cnt, rank, perm);
   out.perm = perm;
   out.flag = flag;
-  out.groups = groups;
+  out.rule = rule;
   return cudaGetLastError();
 }

@@ -220,3 +220,31 @@ def test_crowded_cells(count):
         assert bad.mean() <= 1e-4, bad.sum()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("where", ["everywhere", "one corner"])
+def test_many_particles_on_a_large_grid(where):
+    """Enough particles for G2P to look at their order, on a grid beyond L2: spread over it, in no
+    order, they are ordered, in a corner of it they are not.  The bits of smaller batches, which
+    are taken as they come."""
+    res, bsx, count = 256, 16, (1 << 19) + 77
+    n = res ** 3
+    rng = np.random.default_rng(12)
+    p = np.zeros(count, msbg_gpu.FLIP_PARTICLE)
+    p["pos"] = rng.uniform(-1.0, (res if where == "everywhere" else 40) + 1.0, (count, 3))
+    p["pos"][5:9, 0] = np.nan
+    p["vel"] = rng.standard_normal((count, 3))
+    ctx = msbg_gpu.Context(0)
+    try:
+        ctx.set_topology(res, res, res, bsx)
+        for w in (msbg_gpu.FLIP_VEL, msbg_gpu.FLIP_VEL_OLD):
+            ctx.flip_channel(w, n, rng.standard_normal(3 * n, np.float32))
+        q, r = p.copy(), p.copy()
+        ctx.flip_g2p(q, 0.95)
+        for i in range(0, count, 1 << 18):
+            part = r[i:i + (1 << 18)].copy()
+            ctx.flip_g2p(part, 0.95)
+            r[i:i + (1 << 18)] = part
+        assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
+    finally:
+        ctx.close()

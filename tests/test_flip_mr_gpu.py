@@ -257,3 +257,33 @@ def test_few_particles_and_a_ragged_last_warp(count):
         assert np.array_equal(q["vel"][-count:].view(np.uint32), r["vel"].view(np.uint32))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("order", ["blocks", "random"])
+def test_many_particles_on_a_large_grid(order):
+    """Enough particles for G2P to look at their order, on a grid beyond L2: the bits of smaller
+    batches, which are taken as they come."""
+    res, bsx, nl, count = 320, 16, 2, (1 << 21) + 5
+    nb = res // bsx
+    lev = np.where(np.arange(nb ** 3) // (nb * nb) < nb * 3 // 8, 0, 1).astype(np.int32)
+    n = msbg_gpu.packed_voxels(bsx, lev)
+    assert 26 * n > 300e6
+    vel, old = _channels(n, 15)
+    p = particles_for(res, count, 19)
+    if order == "blocks":
+        c = np.clip(np.nan_to_num(p["pos"]), 0, res - 1).astype(np.int64) // bsx
+        p = p[np.argsort(c[:, 0] + nb * (c[:, 1] + nb * c[:, 2]), kind="stable")]
+    ctx = msbg_gpu.Context(0)
+    try:
+        ctx.set_topology(res, res, res, bsx, nl, lev)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL, vel)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL_OLD, old)
+        q, r = p.copy(), p.copy()
+        ctx.flip_g2p_mr(q, ALPHA)
+        for i in range(0, count, 1 << 20):
+            part = r[i:i + (1 << 20)].copy()
+            ctx.flip_g2p_mr(part, ALPHA)
+            r[i:i + (1 << 20)] = part
+        assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
+    finally:
+        ctx.close()
