@@ -36,10 +36,9 @@ struct FlipState {
   int sx = 0, sy = 0, sz = 0, bsx = 0;
   int64_t n = 0;
   DeviceBuffer vel, velOld, beta, mass, liq, acc, active, parts;
-  // P2G cell by cell: counts per cell (particles, liquid ones) and first entries in the
-  // list, cursor; the particles' ranks and the list itself, and G2P's visiting order.
+  // P2G cell by cell: the particles' ranks and the list; G2P's visiting order.
   // (acc also takes G2P's side-by-side copy of vel and velOld.)
-  DeviceBuffer cells, lists;
+  DeviceBuffer lists;
 };
 
 std::map<msbg_gpu_ctx*, std::unique_ptr<FlipState>>& states() {
@@ -120,108 +119,154 @@ __global__ void k_p2g_scatter(const msbg_flip_particle* __restrict__ p, int64_t 
   }
 }
 
-// Many particles: cell by cell.  Scattering them one by one costs 72 float atomics each,
-// at 400 G atomics/s the bound of the pass (13.3 M particles on 160^3 cells, B200: 2.2 of
-// P2G's 2.5 ms).  Here
-//   k_p2g_count  gives each particle its cell and its rank there, and counts the cells'
-//                particles and liquid ones; a particle with a finite position outside the
-//                grid reaches its boundary faces alone, and does so here, as do those that a
-//                cell has beyond P2G_CELL_MAX;
-//   k_p2g_start, k_p2g_place  list the particles cell by cell (indices; the particles
-//                stay where they are);
-//   k_p2g_cells  a CTA per 8 x 8 x 4 cells, a thread per cell: a cell's particles reach 2 x 3 x
+// Many particles, where they lie close: cell by cell.  Scattering them one by one costs 72 float
+// atomics each, at 400 G atomics/s the bound of the pass (13.3 M particles on 160^3 cells, B200:
+// 2.2 of P2G's 2.5 ms).  Here, for boxes of 8 x 8 x 4 cells,
+//   k_p2g_sample counts one particle of 32 of each box and lists the boxes that count as
+//                crowded;
+//   k_p2g_count  gives each particle of a crowded box its cell and its rank there, and counts the
+//                cells' particles.  The others are scattered here: particles of other boxes,
+//                those that a cell has beyond P2G_CELL_MAX, and those outside the grid, which
+//                reach its boundary faces alone;
+//   k_p2g_start, k_p2g_place  list the particles of crowded boxes cell by cell (indices; the
+//                particles stay where they are);
+//   k_p2g_cells  a CTA per crowded box, a thread per cell: a cell's particles reach 2 x 3 x
 //                3 faces per direction, whose three sums the thread keeps in registers;
 //                they go to the CTA's faces in shared memory one neighbour
 //                offset at a time, in which no two threads meet, and from there to the
-//                grid with one float atomic per face and sum.
-// 0.73 ms for the four kernels.
+//                grid with one float atomic per face and sum.  A box whose particles lie in
+//                few of its cells is scattered after all.
+constexpr int SUB = 8, SUB_Z = 4, SUB_T = SUB * SUB * SUB_Z;
+
+// A box counts as crowded from P2G_CROWDED sampled particles on.
+constexpr int P2G_SAMPLE = 32, P2G_CROWDED = 8;
+
+// Scattering a box's particles takes 27 ns each of an SM's share of the atomics; summing them
+// takes its CTA, one of three on the SM, 54 barriers (5 us) and 1.2 us for each particle of
+// its fullest cell.
+__device__ __forceinline__ bool box_pays(int particles, int fullest) {
+  return particles >= 64 + 16 * fullest;
+}
 
 // A cell's particles that its thread sums: a chain of dependent loads, 0.4 us each, that its
 // CTA waits for; a clump of any size ends there.
 constexpr int P2G_CELL_MAX = 32;
 
-// The cell of a particle with a finite position; -1 outside the grid.
-__device__ __forceinline__ int64_t cell_of(const msbg_flip_particle& q, const GridF& g) {
-  return g.idx((int)floorf(q.pos[0]), (int)floorf(q.pos[1]), (int)floorf(q.pos[2]));
+// The cell of a particle with a finite position, -1 outside the grid, and its box.
+__device__ __forceinline__ int64_t cell_of(const msbg_flip_particle& q, const GridF& g, int& box) {
+  const int x = (int)floorf(q.pos[0]), y = (int)floorf(q.pos[1]), z = (int)floorf(q.pos[2]);
+  const int64_t ci = g.idx(x, y, z);
+  box = ci < 0 ? 0 : x / SUB + g.sx / SUB * (y / SUB + g.sy / SUB * (z / SUB_Z));
+  return ci;
 }
 
+struct P2GBoxes {
+  int* cnt;      // [boxes] sampled particles
+  int* n;        // crowded boxes, then the cursor of the particles' list
+  int* crowded;  // [boxes] their ids
+  int* start;    // [n] first entry of a cell of a crowded box
+};
+
+__global__ void __launch_bounds__(256) k_p2g_sample(const msbg_flip_particle* __restrict__ p,
+                                                    int64_t np, GridF g, P2GBoxes B) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np / P2G_SAMPLE;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    // one of 32, no fixed one: programs lay particles out with strides of their own
+    const msbg_flip_particle& q = p[i * P2G_SAMPLE + (((unsigned)i * 0x9e3779b1u) >> 27)];
+    if (!finite_pos(q)) continue;
+    int box;
+    if (cell_of(q, g, box) >= 0 && atomicAdd(&B.cnt[box], 1) == P2G_CROWDED - 1)
+      B.crowded[atomicAdd(&B.n[0], 1)] = box;
+  }
+}
+
+// mass counts in float where a box is not crowded, in int where it is; liq leaves the listed
+// particles to k_p2g_cells, which turns mass into floats too.
 __global__ void __launch_bounds__(256) k_p2g_count(const msbg_flip_particle* __restrict__ p,
                                                    int64_t np, GridF g, int64_t n, float rhoL,
-                                                   float rhoG,
-                                                   unsigned long long* __restrict__ cnt,
-                                                   int2* __restrict__ place,
+                                                   float rhoG, P2GBoxes B, float* __restrict__ mass,
+                                                   int* __restrict__ liq, int2* __restrict__ place,
                                                    float* __restrict__ acc) {
+  const bool any = B.n[0] > 0;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
        k += (int64_t)gridDim.x * blockDim.x) {
     const msbg_flip_particle& q = p[k];
     const bool finite = finite_pos(q);
-    const int64_t ci = finite ? cell_of(q, g) : -1;
-    int2 at = make_int2((int)ci, 0);
-    // low word particles, high word liquid ones
-    if (ci >= 0) at.y = (int)atomicAdd(&cnt[ci], q.phase == 0 ? (1ull << 32) + 1 : 1ull);
-    const bool listed = ci >= 0 && (unsigned)at.y < P2G_CELL_MAX;
-    if (!listed) at.x = -1;
-    place[k] = at;
-    if (finite && !listed) scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
+    int box = 0;
+    const int64_t ci = finite ? cell_of(q, g, box) : -1;
+    int2 at = make_int2(-1, 0);
+    if (ci >= 0) {
+      if (B.cnt[box] >= P2G_CROWDED) {
+        at.y = atomicAdd(reinterpret_cast<int*>(mass) + ci, 1);
+        if ((unsigned)at.y < P2G_CELL_MAX) at.x = (int)ci;
+      } else {
+        atomicAdd(&mass[ci], 1.f);
+      }
+      if (q.phase == 0 && at.x < 0) atomicAdd(&liq[ci], 1);
+    }
+    if (any) place[k] = at;
+    if (finite && at.x < 0) scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
   }
 }
 
-// First entries of the cells in perm (a CTA's 1024 cells back to back, the CTAs in any
-// order); the cells' mass and liquid count.
-__global__ void __launch_bounds__(1024) k_p2g_start(int64_t n,
-                                                    const unsigned long long* __restrict__ cnt,
-                                                    int* __restrict__ start,
-                                                    float* __restrict__ mass,
-                                                    int* __restrict__ liq, int* __restrict__ cursor) {
-  __shared__ int sum[32], base;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t c = blockIdx.x * (int64_t)1024 + threadIdx.x;
-  const unsigned long long u = c < n ? cnt[c] : 0ull;
-  const int all = (int)(unsigned)u, v = min(all, P2G_CELL_MAX);
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) sum[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    int s = sum[lane];
+// Cell of thread t in a box, and its place in the block layout.
+__device__ __forceinline__ int64_t box_cell(const GridF& g, int box, int t, int& bx, int& by, int& bz,
+                                            int& x, int& y, int& z) {
+  const int nsx = g.sx / SUB, nsy = g.sy / SUB;
+  bx = box % nsx * SUB;
+  by = box / nsx % nsy * SUB;
+  bz = box / (nsx * nsy) * SUB_Z;
+  x = bx + t % SUB;
+  y = by + t / SUB % SUB;
+  z = bz + t / (SUB * SUB);
+  return g.idx(x, y, z);
+}
+
+// First entries of the cells of the crowded boxes in perm, box by box in any order.
+__global__ void __launch_bounds__(SUB_T) k_p2g_start(GridF g, P2GBoxes B,
+                                                     const float* __restrict__ mass) {
+  __shared__ int sum[SUB_T / 32], base;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  for (int i = blockIdx.x; i < B.n[0]; i += gridDim.x) {
+    int bx, by, bz, x, y, z;
+    const int64_t c = box_cell(g, B.crowded[i], t, bx, by, bz, x, y, z);
+    const int v = min(reinterpret_cast<const int*>(mass)[c], P2G_CELL_MAX);
+    int s = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += y;
+      const int u = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += u;
     }
-    sum[lane] = s;
-    if (lane == 31 && s) base = atomicAdd(cursor, s);
+    if (lane == 31) sum[w] = s;
+    __syncthreads();
+    int before = 0;
+    for (int k = 0; k < w; k++) before += sum[k];
+    if (t == SUB_T - 1) base = atomicAdd(&B.n[1], before + s);
+    __syncthreads();
+    B.start[c] = base + before + s - v;
+    __syncthreads();  // sum and base are read
   }
-  __syncthreads();
-  if (c >= n) return;
-  start[c] = v ? base + (w ? sum[w - 1] : 0) + x - v : 0;
-  mass[c] = (float)all;
-  liq[c] = (int)(u >> 32);
 }
 
 __global__ void __launch_bounds__(256) k_p2g_place(int64_t np, const int2* __restrict__ place,
-                                                   const int* __restrict__ start,
-                                                   int* __restrict__ perm) {
+                                                   P2GBoxes B, int* __restrict__ perm) {
+  if (B.n[0] == 0) return;  // place is not written
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < np;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int2 at = place[k];
-    if (at.x >= 0) perm[start[at.x] + at.y] = (int)k;
+    if (at.x >= 0) perm[B.start[at.x] + at.y] = (int)k;
   }
 }
 
-// Cells of a CTA along x and y, and along z.  A thread needs 54 sums and so close to 80
-// registers: three CTAs of this size share an SM, of 8^3 cells it holds one, which waits out
-// its loads and barriers alone (0.66 ms; 0.56 this way).
-constexpr int SUB = 8, SUB_Z = 4, SUB_T = SUB * SUB * SUB_Z;
+// A thread needs 54 sums and so close to 80 registers: three CTAs of this size share an SM, of
+// 8^3 cells it holds one, which waits out its loads and barriers alone (0.66 ms for 13.3 M
+// particles on 160^3 cells; 0.56 this way).
 constexpr int FACE_ROW = SUB + 2, FACES = FACE_ROW * FACE_ROW * (SUB_Z + 2);
 
 // Direction D: faces of cell (x, y, z) at offset 0, 1 along D and -1, 0, 1 along the others.
+// Returns the number of liquid particles.
 template <int D>
-__device__ __forceinline__ void p2g_direction(const msbg_flip_particle* __restrict__ p,
+__device__ __forceinline__ int p2g_direction(const msbg_flip_particle* __restrict__ p,
                                               const int* __restrict__ list, int cnt, int x, int y,
                                               int z, int at, float rhoL, float rhoG,
                                               float (*sums)[FACES]) {
@@ -230,8 +275,10 @@ __device__ __forceinline__ void p2g_direction(const msbg_flip_particle* __restri
   float v[NX * NY * NZ], w[NX * NY * NZ], r[NX * NY * NZ];
 #pragma unroll
   for (int i = 0; i < NX * NY * NZ; i++) v[i] = w[i] = r[i] = 0.f;
+  int liquid = 0;
   for (int m = 0; m < cnt; m++) {
     const msbg_flip_particle& q = p[list[m]];
+    liquid += q.phase == 0;
     const float mp = q.phase == 0 ? rhoL : rhoG, u = q.vel[D];
     // the weights along an axis: of the particle's two faces, 0 for a third
     auto axis = [](float pos, float off, int cell, int i0, int ni, float* out) -> int {
@@ -278,45 +325,67 @@ __device__ __forceinline__ void p2g_direction(const msbg_flip_particle* __restri
         }
         __syncthreads();
       }
+  return liquid;
 }
 
 __global__ void __launch_bounds__(SUB_T, 3) k_p2g_cells(
-    const msbg_flip_particle* __restrict__ p, GridF g, int64_t n, float rhoL, float rhoG,
-    const unsigned long long* __restrict__ cnt, const int* __restrict__ start,
-    const int* __restrict__ perm, float* __restrict__ acc) {
+    const msbg_flip_particle* __restrict__ p, GridF g, int64_t n, float rhoL, float rhoG, P2GBoxes B,
+    float* __restrict__ mass, int* __restrict__ liq, const int* __restrict__ perm,
+    float* __restrict__ acc) {
   __shared__ float sums[3][FACES];
+  __shared__ int total, fullest, first;
   const int t = threadIdx.x;
-  const int nsx = g.sx / SUB, nsy = g.sy / SUB;
-  const int bx = blockIdx.x % nsx * SUB, by = blockIdx.x / nsx % nsy * SUB,
-            bz = blockIdx.x / (nsx * nsy) * SUB_Z;
-  const int lx = t % SUB, ly = t / SUB % SUB, lz = t / (SUB * SUB);
-  const int x = bx + lx, y = by + ly, z = bz + lz;
-  const int64_t ci = g.idx(x, y, z);
-  const int m = (int)min((unsigned)cnt[ci], (unsigned)P2G_CELL_MAX);
-  if (!__syncthreads_or(m)) return;
-  const int* list = perm + start[ci];
-  const int at = (lx + 1) + FACE_ROW * ((ly + 1) + FACE_ROW * (lz + 1));
-  auto direction = [&](auto dd) {
-    constexpr int D = decltype(dd)::value;
-    for (int i = t; i < 3 * FACES; i += SUB_T) sums[i / FACES][i % FACES] = 0.f;
-    __syncthreads();
-    p2g_direction<D>(p, list, m, x, y, z, at, rhoL, rhoG, sums);
-    for (int i = t; i < FACES; i += SUB_T) {
-      const float w = sums[1][i];
-      const float v = sums[0][i], r = sums[2][i];
-      if (w == 0.f && v == 0.f && r == 0.f) continue;
-      const int64_t f = g.idx(bx + i % FACE_ROW - 1, by + i / FACE_ROW % FACE_ROW - 1,
-                              bz + i / (FACE_ROW * FACE_ROW) - 1);
-      if (f < 0) continue;
-      atomicAdd(&acc[(size_t)D * n + f], v);
-      atomicAdd(&acc[(size_t)(3 + D) * n + f], w);
-      atomicAdd(&acc[(size_t)(6 + D) * n + f], r);
+  for (int i = blockIdx.x; i < B.n[0]; i += gridDim.x) {
+    int bx, by, bz, x, y, z;
+    const int64_t ci = box_cell(g, B.crowded[i], t, bx, by, bz, x, y, z);
+    const int all = reinterpret_cast<const int*>(mass)[ci], m = min(all, P2G_CELL_MAX);
+    mass[ci] = (float)all;
+    if (t == 0) {
+      total = fullest = 0;
+      first = B.start[ci];
     }
     __syncthreads();
-  };
-  direction(std::integral_constant<int, 0>{});
-  direction(std::integral_constant<int, 1>{});
-  direction(std::integral_constant<int, 2>{});
+    const int wm = __reduce_max_sync(0xffffffffu, m), ws = __reduce_add_sync(0xffffffffu, m);
+    if ((t & 31) == 0) {
+      atomicAdd(&total, ws);
+      atomicMax(&fullest, wm);
+    }
+    __syncthreads();
+    if (!box_pays(total, fullest)) {  // its particles, one after the other in perm
+      for (int k = t; k < total; k += SUB_T) {
+        const msbg_flip_particle& q = p[perm[first + k]];
+        int box;
+        if (q.phase == 0) atomicAdd(&liq[cell_of(q, g, box)], 1);
+        scatter_faces(q, g, n, q.phase == 0 ? rhoL : rhoG, acc);
+      }
+      __syncthreads();  // total is read
+      continue;
+    }
+    const int* list = perm + B.start[ci];
+    const int at = (x - bx + 1) + FACE_ROW * ((y - by + 1) + FACE_ROW * (z - bz + 1));
+    auto direction = [&](auto dd) {
+      constexpr int D = decltype(dd)::value;
+      for (int q = t; q < 3 * FACES; q += SUB_T) sums[q / FACES][q % FACES] = 0.f;
+      __syncthreads();
+      const int liquid = p2g_direction<D>(p, list, m, x, y, z, at, rhoL, rhoG, sums);
+      if (D == 0 && liquid) liq[ci] += liquid;
+      for (int q = t; q < FACES; q += SUB_T) {
+        const float w = sums[1][q];
+        const float v = sums[0][q], r = sums[2][q];
+        if (w == 0.f && v == 0.f && r == 0.f) continue;
+        const int64_t f = g.idx(bx + q % FACE_ROW - 1, by + q / FACE_ROW % FACE_ROW - 1,
+                                bz + q / (FACE_ROW * FACE_ROW) - 1);
+        if (f < 0) continue;
+        atomicAdd(&acc[(size_t)D * n + f], v);
+        atomicAdd(&acc[(size_t)(3 + D) * n + f], w);
+        atomicAdd(&acc[(size_t)(6 + D) * n + f], r);
+      }
+      __syncthreads();
+    };
+    direction(std::integral_constant<int, 0>{});
+    direction(std::integral_constant<int, 1>{});
+    direction(std::integral_constant<int, 2>{});
+  }
 }
 
 struct P2GConst {
@@ -545,9 +614,10 @@ int state_of(msbg_gpu_ctx* ctx, FlipState** out, GridF& g) {
 
 int grid_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 32); }
 
-// From how many particles on P2G goes cell by cell (below, the extra launches cost more than they
-// save).
-constexpr int64_t FLIP_MANY = 1 << 16;
+// From how many particles on P2G looks for crowded boxes: four launches more, 10 to 15 us, which
+// 0.5 M particles on 64^3 to 256^3 cells give back where they lie 8 (127 against 193 us on 64^3,
+// B200) or 2 to a cell (138 against 130), and 0.25 M do not.
+constexpr int64_t P2G_MANY = 1 << 19;
 // From how many particles on G2P looks whether it should order them (five launches, 10 us, where
 // it should not), and lays the channels side by side first (48 bytes per voxel against half the
 // loads), if there is at least one particle per G2P_PAIR_VOXELS voxels: 4 M particles on 128^3
@@ -588,34 +658,37 @@ int flip_p2g(msbg_gpu_ctx* ctx, const msbg_flip_particle* particles, int64_t np,
                                        cudaMemcpyHostToDevice, st));
     dp = S->parts.as<msbg_flip_particle>();
   }
-  bool cells = np >= FLIP_MANY && np <= INT_MAX && n <= INT_MAX;
-  if (cells && (S->cells.ensure(12 * (size_t)n + 8) != cudaSuccess ||
-                S->lists.ensure(std::max<size_t>(12 * (size_t)np, bins_bytes(np, ctx->nb()))) !=
-                    cudaSuccess)) {
+  bool cells = np >= P2G_MANY && np <= INT_MAX && n <= INT_MAX;
+  if (cells && S->lists.ensure(12 * (size_t)np) != cudaSuccess) {
     cudaGetLastError();  // no room for the lists: particle by particle
     cells = false;
   }
+  MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S->mass.p, 0, 4 * (size_t)n, st));
+  MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S->liq.p, 0, 4 * (size_t)n, st));
   if (cells) {
-    auto* cnt = S->cells.as<unsigned long long>();  // [n], the cursor, then the starts [n]
-    int* cursor = reinterpret_cast<int*>(cnt + n);
-    int* start = cursor + 2;
+    // beta, which k_p2g_finish writes in full, holds the boxes and the cells' entries until then
+    const int boxes = (int)(n / SUB_T);
+    P2GBoxes B;
+    B.cnt = S->beta.as<int>();
+    B.n = B.cnt + boxes;
+    B.crowded = B.n + 2;
+    B.start = B.crowded + boxes;
     int2* place = S->lists.as<int2>();  // cell (-1: none) and rank in it of a particle
     int* perm = reinterpret_cast<int*>(place + np);
-    MSBG_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, 8 * (size_t)(n + 1), st));
-    k_p2g_count<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, n, prm->rhoL, prm->rhoG, cnt, place,
+    MSBG_CUDA_TRY(ctx, cudaMemsetAsync(B.cnt, 0, 4 * (size_t)(boxes + 2), st));
+    k_p2g_sample<<<grid_blocks(np / P2G_SAMPLE), 256, 0, st>>>(dp, np, g, B);
+    k_p2g_count<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, n, prm->rhoL, prm->rhoG, B,
+                                                 S->mass.as<float>(), S->liq.as<int>(), place,
                                                  S->acc.as<float>());
-    k_p2g_start<<<(unsigned)((n + 1023) / 1024), 1024, 0, st>>>(
-        n, cnt, start, S->mass.as<float>(), S->liq.as<int>(), cursor);
-    k_p2g_place<<<grid_blocks(np), 256, 0, st>>>(np, place, start, perm);
-    k_p2g_cells<<<(unsigned)(n / SUB_T), SUB_T, 0, st>>>(
-        dp, g, n, prm->rhoL, prm->rhoG, cnt, start, perm, S->acc.as<float>());
-  } else {
-    MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S->mass.p, 0, 4 * (size_t)n, st));
-    MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S->liq.p, 0, 4 * (size_t)n, st));
-    if (np)
-      k_p2g_scatter<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, n, prm->rhoL, prm->rhoG,
-                                                     S->acc.as<float>(), S->mass.as<float>(),
-                                                     S->liq.as<int>());
+    k_p2g_start<<<std::min(boxes, 148 * 8), SUB_T, 0, st>>>(g, B, S->mass.as<float>());
+    k_p2g_place<<<grid_blocks(np), 256, 0, st>>>(np, place, B, perm);
+    k_p2g_cells<<<std::min(boxes, 148 * 3), SUB_T, 0, st>>>(dp, g, n, prm->rhoL, prm->rhoG, B,
+                                                            S->mass.as<float>(), S->liq.as<int>(),
+                                                            perm, S->acc.as<float>());
+  } else if (np) {
+    k_p2g_scatter<<<grid_blocks(np), 256, 0, st>>>(dp, np, g, n, prm->rhoL, prm->rhoG,
+                                                   S->acc.as<float>(), S->mass.as<float>(),
+                                                   S->liq.as<int>());
   }
   P2GConst c;
   c.massEps = prm->massEps;

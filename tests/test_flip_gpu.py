@@ -222,6 +222,56 @@ def test_crowded_cells(count):
         ctx.close()
 
 
+@pytest.mark.parametrize("bsx", [8, 16, 32])
+def test_boxes_of_every_kind(bsx):
+    """Enough particles for P2G to look for crowded boxes, which it sums, and others, which it
+    scatters: cells with 8, 2, 1 and no particles, clumps of 40 (in a box of their own and beside
+    full cells), particles outside the grid, on its faces and without a finite position; laid out
+    cell by cell, in no order and as 32 interleaved streams (the sample takes one in 32).
+    Bounds as in test_crowded_cells, of the fullest cells here."""
+    res = 64
+    rng = np.random.default_rng(21)
+
+    def fill(cells, per):
+        return np.repeat(cells, per, 0) + rng.uniform(0.0, 1.0, (len(cells) * per, 3))
+
+    cells = np.stack(np.meshgrid(*[np.arange(res)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    x = cells[:, 0]
+    some = cells[x >= 48]
+    pos = [fill(cells[x < 16], 8), fill(cells[(x >= 16) & (x < 24)], 2),
+           fill(cells[(x >= 24) & (x < 32)], 1),
+           fill(some[rng.choice(len(some), 500, replace=False)], 40),
+           fill(cells[x < 8][::997], 40), rng.uniform(-1.5, res + 1.5, (3000, 3))]
+    pos = np.concatenate(pos).astype(np.float32)
+    pos[::50] = np.round(pos[::50] * 2) / 2
+    pos[7:20, 1] = np.nan
+    pos[30:33, 2] = np.inf
+    p = np.zeros(len(pos), msbg_gpu.FLIP_PARTICLE)
+    assert len(p) > 1 << 19
+    p["pos"] = pos
+    p["vel"] = rng.standard_normal((len(p), 3))
+    p["phase"] = rng.integers(0, 2, len(p))
+    n = res ** 3
+    vel_o, mass_o, beta_o, act_o = oracle.flip_p2g(res, bsx, p)
+    tol = 1e-5 + 4 * (8 * 56 + 64) * 2.0 ** -24
+    m = len(p) // 32 * 32
+    streams = np.concatenate([np.arange(m).reshape(32, -1).T.reshape(-1), np.arange(m, len(p))])
+    ctx = msbg_gpu.Context(0)
+    try:
+        ctx.set_topology(res, res, res, bsx)
+        for order in (np.arange(len(p)), rng.permutation(len(p)), streams):
+            act = ctx.flip_p2g(p[order])
+            vel = ctx.flip_channel(msbg_gpu.FLIP_VEL, n)
+            beta = ctx.flip_channel(msbg_gpu.FLIP_BETA, n)
+            assert np.array_equal(ctx.flip_channel(msbg_gpu.FLIP_MASS, n), mass_o)
+            assert np.array_equal(np.sort(act), np.nonzero(act_o)[0])
+            assert np.abs(vel - vel_o).max() <= tol * max(1.0, np.abs(p["vel"]).max())
+            bad = np.abs(beta - beta_o) > tol * np.maximum(1e-3, np.abs(beta_o))
+            assert bad.mean() <= 1e-4, bad.sum()
+    finally:
+        ctx.close()
+
+
 @pytest.mark.parametrize("where", ["everywhere", "one corner"])
 def test_many_particles_on_a_large_grid(where):
     """Enough particles for G2P to look at their order, on a grid beyond L2: spread over it, in no
