@@ -49,7 +49,7 @@ struct MrState {
   bool distBuilt = false;
   DeviceBuffer level, off, fc, kind, key, dist, parts;
   DeviceBuffer vel;      // [3n] (vel, velOld) side by side: a gather reads both in one load
-  DeviceBuffer scratch;  // one channel on its way in or out; the visiting order of G2P
+  DeviceBuffer scratch;  // pieces of a channel on its way in or out; the visiting order of G2P
   DeviceBuffer dsOffA, dsOffB, dsFlags, dsSrc, dsDst;  // downsampleVelocity
 };
 
@@ -462,6 +462,9 @@ int grid_blocks(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 
 // (512^3, 3 levels, 16^3 blocks, in no order, B200): 1 M 193 and 206 us, 4 M 658 and 575.
 constexpr int64_t MR_BINS_MIN = 1 << 21;
 
+// Floats of a channel that are on the device at a time on their way in or out (16 MB).
+constexpr int64_t MR_PIECE = 4 << 20;
+
 // One of the two interleaved channels: into it (get = 0) or out of it.
 __global__ void __launch_bounds__(256) k_mr_channel(float2* __restrict__ vel, int which,
                                                     float* __restrict__ data, int64_t n, int get) {
@@ -604,17 +607,27 @@ extern "C" int msbg_gpu_flip_mr_channel(msbg_gpu_ctx* ctx, int which, float* dat
   if (n != 3 * S->n)
     return set_error(ctx, MSBG_EINVARG, "mixed-resolution channel holds %lld floats, not %lld",
                      (long long)(3 * S->n), (long long)n);
-  MSBG_CUDA_TRY(ctx, S->scratch.ensure(sizeof(float) * n));
   const int w = which == MSBG_FLIP_VEL ? 0 : 1;
-  if (!get)
-    MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(S->scratch.p, data, sizeof(float) * n,
-                                       cudaMemcpyHostToDevice, ctx->stream));
-  k_mr_channel<<<grid_blocks(n), 256, 0, ctx->stream>>>(S->vel.as<float2>(), w,
-                                                        S->scratch.as<float>(), n, get);
-  MSBG_CUDA_TRY(ctx, cudaGetLastError());
-  if (get)
-    MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(data, S->scratch.p, sizeof(float) * n,
-                                       cudaMemcpyDeviceToHost, ctx->stream));
+  cudaStream_t st = ctx->stream;
+  if (S->scratch.ensure(sizeof(float) * std::min(n, MR_PIECE)) != cudaSuccess) {
+    cudaGetLastError();  // no room for a piece: value by value
+    float* v = S->vel.as<float>() + w;
+    MSBG_CUDA_TRY(ctx, get ? cudaMemcpy2DAsync(data, 4, v, 8, 4, n, cudaMemcpyDeviceToHost, st)
+                           : cudaMemcpy2DAsync(v, 8, data, 4, 4, n, cudaMemcpyHostToDevice, st));
+    return msbg_gpu_sync(ctx);
+  }
+  float* piece = S->scratch.as<float>();
+  for (int64_t o = 0; o < n; o += MR_PIECE) {
+    const int64_t m = std::min(n - o, MR_PIECE);
+    if (!get)
+      MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(piece, data + o, sizeof(float) * m,
+                                         cudaMemcpyHostToDevice, st));
+    k_mr_channel<<<grid_blocks(m), 256, 0, st>>>(S->vel.as<float2>() + o, w, piece, m, get);
+    MSBG_CUDA_TRY(ctx, cudaGetLastError());
+    if (get)
+      MSBG_CUDA_TRY(ctx, cudaMemcpyAsync(data + o, piece, sizeof(float) * m,
+                                         cudaMemcpyDeviceToHost, st));
+  }
   return msbg_gpu_sync(ctx);
 }
 

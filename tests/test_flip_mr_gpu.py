@@ -287,3 +287,32 @@ def test_many_particles_on_a_large_grid(order):
         assert np.array_equal(q["vel"].view(np.uint32), r["vel"].view(np.uint32))
     finally:
         ctx.close()
+
+
+def test_channels_need_no_scratch_of_their_size():
+    """Channels come and go in pieces: beside the two channels and the distances a context keeps
+    little, however large its grid, and the values of all pieces are in their places."""
+    import torch
+
+    res, bsx, nl = 256, 16, 2
+    nb = res // bsx
+    lev = np.where(np.arange(nb ** 3) // (nb * nb) < nb * 3 // 8, 0, 1).astype(np.int32)
+    n = msbg_gpu.packed_voxels(bsx, lev)
+    vel, old = _channels(n, 25)
+    ctx = msbg_gpu.Context(0)
+    try:
+        ctx.set_topology(res, res, res, bsx, nl, lev)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL, vel[:3 * n])
+        ctx.close()
+        ctx = msbg_gpu.Context(0)
+        ctx.set_topology(res, res, res, bsx, nl, lev)
+        free = torch.cuda.mem_get_info()[0]
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL, vel)
+        ctx.flip_mr_channel(msbg_gpu.FLIP_VEL_OLD, old)
+        used = free - torch.cuda.mem_get_info()[0]
+        assert used <= 26 * n + 32 * nb ** 3 + (48 << 20), (used, n)
+        assert 3 * n > 4 * (4 << 20)  # several pieces, the last not full
+        assert np.array_equal(ctx.flip_mr_channel(msbg_gpu.FLIP_VEL), vel)
+        assert np.array_equal(ctx.flip_mr_channel(msbg_gpu.FLIP_VEL_OLD), old)
+    finally:
+        ctx.close()
