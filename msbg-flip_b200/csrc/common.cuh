@@ -73,32 +73,57 @@ enum : int {
 
 // Device blocks on their way from one owner to the next.  While a PoolScope is open on a
 // thread, buffers that it releases there go to the scope's pool, and buffers that need memory
-// look there first (a block of at most 1/4 more than asked for); what is left is freed when
-// the scope closes, or before an allocation fails.  For work on one stream: a block may still
-// be read by what its last owner has issued there.
+// look there first; what is left is freed when the scope closes, or before an allocation fails.
+// For work on one stream: a block may still be read by what its last owner has issued there.
+// A block may be up to 1/4 larger than asked for, and its new owner keeps what is too much.  That
+// comes to 1/64 of the memory that was free when the scope opened, and to nothing but the rest
+// of a 2 MB page (which cudaMalloc keeps as well) where less than a quarter of the card was: what
+// fits without a pool is not to be refused with one.
 class DevicePool {
  public:
+  DevicePool() {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) == cudaSuccess && free >= total / 4) allowed_ = free / 64;
+  }
   ~DevicePool() { clear(); }
+  DevicePool(const DevicePool&) = delete;
+  DevicePool& operator=(const DevicePool&) = delete;
   void clear() {
     for (auto& b : blocks_) cudaFree(b.second);
     blocks_.clear();
   }
-  void give(void* p, size_t cap) { blocks_.emplace(cap, p); }
+  void give(void* p, size_t cap) noexcept {
+    try {
+      blocks_.emplace(cap, p);
+    } catch (...) {  // no memory for the entry
+      cudaFree(p);
+    }
+  }
   void* take(size_t n, size_t& cap) {
     auto it = blocks_.lower_bound(n);
     if (it == blocks_.end() || it->first > n + n / 4 + 4096) return nullptr;
+    const size_t more = it->first - n;
+    if (n < PAGE || (n + PAGE - 1) / PAGE != (it->first + PAGE - 1) / PAGE) {
+      if (more > allowed_) return nullptr;
+      allowed_ -= more;
+      wasted_ += more;
+    }
     void* p = it->second;
     cap = it->first;
     blocks_.erase(it);
     return p;
   }
+  // What the owners of this pool's blocks have too much.
+  size_t wasted() const { return wasted_; }
   static DevicePool*& current() {
     static thread_local DevicePool* c = nullptr;
     return c;
   }
 
  private:
+  static constexpr size_t PAGE = 2 << 20;
   std::multimap<size_t, void*> blocks_;
+  size_t allowed_ = 0, wasted_ = 0;
 };
 class PoolScope {
  public:
@@ -106,6 +131,7 @@ class PoolScope {
   ~PoolScope() { DevicePool::current() = before_; }
   PoolScope(const PoolScope&) = delete;
   PoolScope& operator=(const PoolScope&) = delete;
+  size_t wasted() const { return pool_.wasted(); }
 
  private:
   DevicePool* before_;

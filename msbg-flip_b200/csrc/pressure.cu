@@ -210,24 +210,47 @@ extern "C" int msbg_gpu_pressure_prepare(msbg_gpu_ctx* ctx, const msbg_topo_desc
   return msbg::ps::pressure_prepare(ctx, topo, cb, nullptr);
 }
 
+namespace {
+int prepare_problem(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
+                    const msbg_pressure_callbacks* cb, const ArrayInput* arr);
+}
+
 int msbg::ps::pressure_prepare(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
                                const msbg_pressure_callbacks* cb, const ArrayInput* arr) {
   int rc = msbg_gpu_sync_topology(ctx, topo);
   if (rc) return rc;
   cudaSetDevice(ctx->device);
   auto& sp = solver_of(ctx);
-  // The next problem of a simulation has nearly the sizes of the last one: its buffers take
-  // over the last one's device blocks (cudaFree and cudaMalloc of some hundred buffers were
-  // 12 of a prepare's 31 ms at 320^3).
-  PoolScope pool;
-  Scalars* hScal = nullptr;
   if (sp) {
+    // The next problem of a simulation has nearly the sizes of the last one: its buffers take
+    // over the last one's device blocks (cudaFree and cudaMalloc of some hundred buffers were
+    // 12 of a prepare's 31 ms at 320^3).
+    PoolScope pool;
     cudaStreamSynchronize(ctx->stream);
+    Scalars* hScal = nullptr;
     std::swap(hScal, sp->hScal);
+    sp.reset(new Solver());
+    sp->hScal = hScal;
+    rc = prepare_problem(ctx, topo, cb, arr);
+    if (rc == MSBG_OK) return rc;
+    sp.reset();
+    if (rc != MSBG_ENOMEM || !pool.wasted()) return rc;
+    cudaGetLastError();  // out of memory with blocks that are too large: once more without
   }
   sp.reset(new Solver());
+  rc = prepare_problem(ctx, topo, cb, arr);
+  if (rc) sp.reset();
+  return rc;
+}
+
+namespace {
+
+// The problem into the context's new Solver.
+int prepare_problem(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
+                    const msbg_pressure_callbacks* cb, const ArrayInput* arr) {
+  auto& sp = solver_of(ctx);
   Solver& S = *sp;
-  S.hScal = hScal;
+  int rc = MSBG_OK;
   std::string err;
   auto tp0 = std::chrono::steady_clock::now();
   // per-cell arrays: the per-cell work of the build runs on the GPU (set
@@ -396,8 +419,6 @@ int msbg::ps::pressure_prepare(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
       std::chrono::duration<double>(std::chrono::steady_clock::now() - tp0).count();
   return MSBG_OK;
 }
-
-namespace {
 
 struct PcgResult {
   int iters = 0;
