@@ -138,6 +138,18 @@ class PoolScope {
   DevicePool pool_;
 };
 
+// No pool while a caller's code runs: what it releases is of another owner, stream or device.
+class PoolPause {
+ public:
+  PoolPause() : before_(DevicePool::current()) { DevicePool::current() = nullptr; }
+  ~PoolPause() { DevicePool::current() = before_; }
+  PoolPause(const PoolPause&) = delete;
+  PoolPause& operator=(const PoolPause&) = delete;
+
+ private:
+  DevicePool* before_;
+};
+
 struct DeviceBuffer {
   void* p = nullptr;
   size_t bytes = 0;  // asked for

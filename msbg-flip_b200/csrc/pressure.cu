@@ -269,9 +269,11 @@ int prepare_problem(msbg_gpu_ctx* ctx, const msbg_topo_desc* topo,
       err.clear();
     }
   }
-  if (!onDevice)
+  if (!onDevice) {
+    PoolPause callbacks;
     rc = build_hierarchy(S.H, topo->sx, topo->sy, topo->sz, topo->bsx0, topo->nLevels,
                          topo->blockLevel, topo->domainBc, cb, 512, &err, arr);
+  }
   S.buildSeconds =
       std::chrono::duration<double>(std::chrono::steady_clock::now() - tp0).count();
   if (rc) {

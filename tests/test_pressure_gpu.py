@@ -232,3 +232,37 @@ def test_prepare_over_another_problem(first, second):
     assert out[0][0] == 0
     for o in out[1:]:
         assert o[:2] == out[0][:2] and np.array_equal(o[2], out[0][2])
+
+
+def test_buffers_released_in_a_callback_are_freed(gpu_ctx):
+    """A prepare over an earlier problem keeps that problem's device blocks for its own buffers;
+    what the caller releases inside a callback is not its, and is freed there."""
+    import ctypes as C
+    import threading
+
+    import torch
+
+    import refgrid
+
+    pool = refgrid.OpenPool()
+    gpu_ctx.pressure_prepare(pool)
+    other = msbg_gpu.Context(0)
+    other.set_topology(128, 128, 128, 16)
+    other.flip_gravity(-9.8, 0.01)  # allocates its channels, over 80 MB
+    freed = []
+    main = threading.get_ident()
+
+    def cell_type(u, x, y, z):
+        if not freed and threading.get_ident() == main:
+            before = torch.cuda.mem_get_info()[0]
+            other.close()
+            freed.append(torch.cuda.mem_get_info()[0] - before)
+        return 0 if z < 12 else 0x1000
+
+    fn = msbg_gpu.CELL_TYPE_FN(cell_type)
+    cb = pool.callbacks()
+    pool._cb = msbg_gpu.PressureCallbacks(C.cast(fn, C.c_void_p).value, cb.sampleFaceCoeff,
+                                          cb.sampleRhs, None)
+    gpu_ctx.pressure_prepare(pool)
+    assert freed and freed[0] >= 80 << 20, freed
+    assert gpu_ctx.pressure_solve(tol=1e-6).status == 0
