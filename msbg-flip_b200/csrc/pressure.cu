@@ -1320,9 +1320,11 @@ int profile_typed(msbg_gpu_ctx* ctx, Solver& S, int what, int reps, int innerIte
       const double n = (double)S.H.levels[m].nCells;
       const double vs = m == 0 ? v : 4.0;
       const double sm = m == 0 ? smooth0 : smoothC;
-      // zero x, sweeps, residual (x, b, operator, 1/8 restricted write),
-      // prolongation (a_ii mask, x read + write, 1/8 coarse read)
-      s += n * (vs + (R.nPre + R.nPost) * sm + (16.0 + 2 * vs + 0.5) + (4.0 + 2 * vs + 0.5));
+      // sweeps (the first starts from x = 0 without reading it; without pre-sweeps x is
+      // cleared), residual (x, b, operator, 1/8 restricted write), prolongation (a_ii mask, x
+      // read + write, 1/8 coarse read)
+      s += n * ((R.nPre > 0 ? -vs : vs) + (R.nPre + R.nPost) * sm + (16.0 + 2 * vs + 0.5) +
+                (4.0 + 2 * vs + 0.5));
     }
     return s;
   };

@@ -266,3 +266,18 @@ def test_buffers_released_in_a_callback_are_freed(gpu_ctx):
     gpu_ctx.pressure_prepare(pool)
     assert freed and freed[0] >= 80 << 20, freed
     assert gpu_ctx.pressure_solve(tol=1e-6).status == 0
+
+
+def test_vcycle_bytes_of_the_profile(gpu_ctx):
+    """The bytes that the profile states for a V-cycle are those that it cannot do without: four
+    sweeps of 28 bytes per cell, of which the first does not read x, the residual and the
+    prolongation.  64^3 cells in 16^3 tiles on MG levels 0, 1 and 2 (of 64^3, 32^3, 16^3)."""
+    import refgrid
+
+    flags, faces, rhs = refgrid.box_problem(64, 16, 60)
+    gpu_ctx.pressure_prepare_arrays(64, 16, 1, np.zeros(64, np.int32), flags, faces, rhs)
+    cells = 64 ** 3 + 32 ** 3 + 16 ** 3
+    _, sweep = gpu_ctx.pressure_profile(0, 1, 3)
+    _, vcycle = gpu_ctx.pressure_profile(2, 1, 3)
+    assert sweep == 28 * 64 ** 3
+    assert vcycle == cells * (4 * 28 - 4 + (16 + 8 + 0.5) + (4 + 8 + 0.5))
