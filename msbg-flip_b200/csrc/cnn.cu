@@ -638,12 +638,13 @@ int cnn_error(msbg_cnn* n, int code, const char* fmt, ...) {
                        "%s: %s (%s:%d)", #expr, cudaGetErrorString(_e), __FILE__, __LINE__); \
   } while (0)
 
-void set_attrs() {
-  static bool done = false;
-  if (done) return;
-  cudaFuncSetAttribute(k_conv3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
-  cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
-  done = true;
+// The limits are attributes of the kernels on the current device: set for every network.
+cudaError_t set_attrs() {
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_conv3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(
+                                k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
 }
 
 const __nv_bfloat16* image(msbg_cnn* net, int layer, bool backward) {
@@ -741,7 +742,10 @@ extern "C" int msbg_cnn_create(int device, msbg_cnn** out) {
   auto* net = new msbg_cnn();
   net->device = device;
   cudaDeviceGetAttribute(&net->numSMs, cudaDevAttrMultiProcessorCount, device);
-  set_attrs();
+  if (set_attrs() != cudaSuccess) {
+    delete net;
+    return MSBG_ERROR;
+  }
   if (cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) != cudaSuccess ||
       net->w.ensure(NPARAM * sizeof(float)) != cudaSuccess ||
       net->m.ensure(NPARAM * sizeof(float)) != cudaSuccess ||
