@@ -1391,23 +1391,30 @@ namespace {
 // Copy a level-0 vector (tile layout) into the reference's packed block layout.
 // The reference's block layout (packed): per block in bid order,
 // (bsx0 >> level)^3 values, vid = x + y*bs + z*bs*bs.  A tile lies inside one
-// block, so its cell (i, j, k) lands at base + i + bs*(j + bs*k).
+// block, so its cell (i, j, k) lands at base + i + bs*(j + bs*k); except that on a grid of
+// 8^3 blocks that are all at level 0 a tile of 16^3 holds eight blocks.
 struct PackTile {
   int64_t base;  // packed index of the tile's first cell
-  int bs, ts;
+  int bs, ts, ox, oy, oz;
 };
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_to_packed(const T* __restrict__ v,
                                                    const int64_t* __restrict__ tileOff,
-                                                   const PackTile* __restrict__ pt,
+                                                   const PackTile* __restrict__ pt, int nbx, int nby,
                                                    T* __restrict__ out) {
   const PackTile P = pt[blockIdx.x];
   const int64_t off = tileOff[blockIdx.x];
-  const int n = P.ts * P.ts * P.ts;
+  const int n = P.ts * P.ts * P.ts, bs = P.bs;
   for (int e = threadIdx.x; e < n; e += blockDim.x) {
     const int i = e % P.ts, j = (e / P.ts) % P.ts, k = e / (P.ts * P.ts);
-    out[P.base + i + (int64_t)P.bs * (j + (int64_t)P.bs * k)] = v[off + e];
+    int64_t to = P.base + i + (int64_t)bs * (j + (int64_t)bs * k);
+    if (P.ts > bs) {  // all blocks hold bs^3 cells
+      const int x = P.ox + i, y = P.oy + j, z = P.oz + k;
+      const int64_t blk = x / bs + (int64_t)nbx * (y / bs + (int64_t)nby * (z / bs));
+      to = blk * bs * bs * bs + x % bs + bs * (y % bs + bs * (z % bs));
+    }
+    out[to] = v[off + e];
   }
 }
 
@@ -1444,6 +1451,9 @@ int to_packed(msbg_gpu_ctx* ctx, Solver& S, const T* dvec, T* packed, int64_t n)
       pt[ti].base = boff[blk] + (t.ox % bs) + (int64_t)bs * ((t.oy % bs) + (int64_t)bs * (t.oz % bs));
       pt[ti].bs = bs;
       pt[ti].ts = t.ts;
+      pt[ti].ox = t.ox;
+      pt[ti].oy = t.oy;
+      pt[ti].oz = t.oz;
     }
     MSBG_CUDA_TRY(ctx, upload(S.packTiles, pt, st));
     MSBG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
@@ -1452,7 +1462,8 @@ int to_packed(msbg_gpu_ctx* ctx, Solver& S, const T* dvec, T* packed, int64_t n)
   MSBG_CUDA_TRY(ctx, cudaMemsetAsync(S.packBuf.p, 0, sizeof(T) * need, st));
   if (!L.tiles.empty())
     k_to_packed<T><<<(unsigned)L.tiles.size(), 256, 0, st>>>(
-        dvec, S.dev[0]->tileOff.as<int64_t>(), S.packTiles.as<PackTile>(), S.packBuf.as<T>());
+        dvec, S.dev[0]->tileOff.as<int64_t>(), S.packTiles.as<PackTile>(), S.nbx, S.nby,
+        S.packBuf.as<T>());
   MSBG_CUDA_TRY(ctx, cudaGetLastError());
   MSBG_CUDA_TRY(ctx, copy_d2h(packed, S.packBuf.p, sizeof(T) * need, st));
   return MSBG_OK;

@@ -61,16 +61,23 @@ struct Ctx {
     return boff[b] + ((x & m) >> l) + ((int64_t)((y & m) >> l) << lsh) +
            ((int64_t)((z & m) >> l) << (2 * lsh));
   }
-  // packed array cell of the first cell of tile t (a tile lies in one block),
-  // and the block's edge in cells of the tile's level
-  int64_t tile_cell0(const Tile& t, int& bs) const {
-    const int l = t.level;
-    const int64_t b = ((t.ox << l) >> sh0) +
-                      (int64_t)H.nb1x * (((t.oy << l) >> sh0) + (int64_t)H.nb1y * ((t.oz << l) >> sh0));
-    bs = H.bsx0 >> l;
-    const int m = bs - 1;
-    return boff[b] + (t.ox & m) + (int64_t)bs * ((t.oy & m) + (int64_t)bs * (t.oz & m));
-  }
+  // Packed array cells of a tile.  A tile lies in one block, except that on a grid of 8^3
+  // blocks that are all at level 0 a tile of 16^3 holds eight.
+  struct TileCells {
+    const Ctx& C;
+    const Tile& t;
+    int64_t c0 = 0;  // the first cell
+    int bs;          // edge of a block in cells of the tile's level
+    int run;         // cells along x that follow each other from a multiple of it on
+    TileCells(const Ctx& c, const Tile& tile)
+        : C(c), t(tile), bs(c.H.bsx0 >> tile.level), run(std::min(tile.ts, bs)) {
+      if (C.arr) c0 = C.cell(t.ox << t.level, t.oy << t.level, t.oz << t.level);
+    }
+    int64_t at(int i, int j, int k) const {
+      if (t.ts <= bs) return c0 + i + (int64_t)bs * (j + (int64_t)bs * k);
+      return C.cell((t.ox + i) << t.level, (t.oy + j) << t.level, (t.oz + k) << t.level);
+    }
+  };
   // The scene at fine voxel (x, y, z): from the callbacks, or from the arrays
   // (outside the domain: solid, no face, no right-hand side).
   uint16_t cell_type(int x, int y, int z) const {
@@ -406,14 +413,13 @@ void sample_level0(const Ctx& C, Level& L, std::vector<uint8_t>& fluid) {
     thread_local std::vector<double> low;  // reused across this thread's tiles
     if (low.size() < 3 * n3) low.resize(3 * n3);
     // with arrays, a lower face inside the tile is the cell's own entry
-    int pbs = 0;
-    const int64_t pc0 = C.arr ? C.tile_cell0(t, pbs) : 0;
+    const Ctx::TileCells cells(C, t);
     const float* const* af = C.arr ? C.arr->face : nullptr;
     for (int k = 0; k < ts; k++)
       for (int j = 0; j < ts; j++)
         for (int i = 0; i < ts; i++) {
           const int64_t ci = i + (int64_t)ts * (j + (int64_t)ts * k);
-          const int64_t pc = pc0 + i + (int64_t)pbs * (j + (int64_t)pbs * k);
+          const int64_t pc = af ? cells.at(i, j, k) : 0;
           const int loc[3] = {i, j, k};
           for (int dir = 0; dir < 3; dir++) {
             if (af && loc[dir] > 0) {
@@ -441,8 +447,7 @@ void sample_level0(const Ctx& C, Level& L, std::vector<uint8_t>& fluid) {
             const int X = t.ox + i, Y = t.oy + j, Z = t.oz + k;
             L.diag[t.off + ci] = (float)diag;
             const double r =
-                C.arr ? (C.arr->rhs ? C.arr->rhs[pc0 + i + (int64_t)pbs * (j + (int64_t)pbs * k)]
-                                    : 0.f)
+                C.arr ? (C.arr->rhs ? C.arr->rhs[cells.at(i, j, k)] : 0.f)
                       : C.rhs(X << l, Y << l, Z << l);
             L.rhs[t.off + ci] = (float)(r * h * h * h);
           }
@@ -879,12 +884,11 @@ int build_hierarchy(Hierarchy& H, int sx, int sy, int sz, int bsx0, int nLevels,
     for (int64_t i = 0; i < (int64_t)cand.size(); i++) {
       const Tile& t = cand[i];
       bool any = false;
-      int pbs = 0;
-      const int64_t pc0 = arr ? C.tile_cell0(t, pbs) : 0;
+      const Ctx::TileCells cells(C, t);
       for (int k = 0; k < t.ts && !any; k++)
         for (int j = 0; j < t.ts && !any; j++)
           for (int ii = 0; ii < t.ts; ii++) {
-            uint16_t ct = arr ? arr->flags[pc0 + ii + (int64_t)pbs * (j + (int64_t)pbs * k)]
+            uint16_t ct = arr ? arr->flags[cells.at(ii, j, k)]
                               : C.cell_type((t.ox + ii) << t.level, (t.oy + j) << t.level,
                                             (t.oz + k) << t.level);
             if (!(ct & CELL_NONFLUID)) {
@@ -904,12 +908,11 @@ int build_hierarchy(Hierarchy& H, int sx, int sy, int sz, int bsx0, int nLevels,
 #pragma omp parallel for schedule(dynamic, 4)
     for (int64_t ti = 0; ti < (int64_t)L.tiles.size(); ti++) {
       const Tile& t = L.tiles[ti];
-      int pbs = 0;
-      const int64_t pc0 = arr ? C.tile_cell0(t, pbs) : 0;
+      const Ctx::TileCells cells(C, t);
       for (int k = 0; k < t.ts; k++)
         for (int j = 0; j < t.ts; j++)
           for (int i = 0; i < t.ts; i++) {
-            uint16_t ct = arr ? arr->flags[pc0 + i + (int64_t)pbs * (j + (int64_t)pbs * k)]
+            uint16_t ct = arr ? arr->flags[cells.at(i, j, k)]
                               : C.cell_type((t.ox + i) << t.level, (t.oy + j) << t.level,
                                             (t.oz + k) << t.level);
             const int64_t c = t.off + i + (int64_t)t.ts * (j + (int64_t)t.ts * k);
@@ -1192,18 +1195,18 @@ int build_hierarchy_device(Hierarchy& H, std::vector<std::unique_ptr<LevelDev>>&
 #pragma omp parallel for schedule(dynamic, 16)
     for (int64_t i = 0; i < (int64_t)cand.size(); i++) {
       const Tile& t = cand[i];
-      int pbs = 0;
-      const int64_t pc0 = C.tile_cell0(t, pbs);
+      const Ctx::TileCells cells(C, t);
       bool any = false;
       for (int k = 0; k < t.ts && !any; k++)
-        for (int j = 0; j < t.ts && !any; j++) {
-          const uint16_t* f = arr.flags + pc0 + (int64_t)pbs * (j + (int64_t)pbs * k);
-          for (int ii = 0; ii < t.ts; ii++)
-            if (!(f[ii] & CELL_NONFLUID)) {
-              any = true;
-              break;
-            }
-        }
+        for (int j = 0; j < t.ts && !any; j++)
+          for (int i0 = 0; i0 < t.ts && !any; i0 += cells.run) {
+            const uint16_t* f = arr.flags + cells.at(i0, j, k);
+            for (int ii = 0; ii < cells.run; ii++)
+              if (!(f[ii] & CELL_NONFLUID)) {
+                any = true;
+                break;
+              }
+          }
       keep[i] = any;
     }
     std::vector<Tile> tiles;
@@ -1295,21 +1298,22 @@ int build_hierarchy_device(Hierarchy& H, std::vector<std::unique_ptr<LevelDev>>&
     for (int ti = t0; ti < t1; ti++) {
       const Tile& t = L.tiles[ti];
       const int ts = t.ts, l = t.level;
-      int pbs = 0;
-      const int64_t pc0 = C.tile_cell0(t, pbs);
+      const Ctx::TileCells cells(C, t);
+      const int run = cells.run;
       const int64_t d0 = t.off - c0;
       for (int kk = 0; kk < ts; kk++)
-        for (int j = 0; j < ts; j++) {
-          const int64_t s0 = pc0 + (int64_t)pbs * (j + (int64_t)pbs * kk);
-          const int64_t dd = d0 + (int64_t)ts * (j + (int64_t)ts * kk);
-          std::memcpy(hf + dd, arr.flags + s0, sizeof(uint16_t) * ts);
-          for (int w = 0; w < 4; w++) {
-            if (src[w])
-              std::memcpy(hx[w] + dd, src[w] + s0, sizeof(float) * ts);
-            else
-              std::memset(hx[w] + dd, 0, sizeof(float) * ts);
+        for (int j = 0; j < ts; j++)
+          for (int i0 = 0; i0 < ts; i0 += run) {
+            const int64_t s0 = cells.at(i0, j, kk);
+            const int64_t dd = d0 + i0 + (int64_t)ts * (j + (int64_t)ts * kk);
+            std::memcpy(hf + dd, arr.flags + s0, sizeof(uint16_t) * run);
+            for (int w = 0; w < 4; w++) {
+              if (src[w])
+                std::memcpy(hx[w] + dd, src[w] + s0, sizeof(float) * run);
+              else
+                std::memset(hx[w] + dd, 0, sizeof(float) * run);
+            }
           }
-        }
       // couplings of the upper tile faces inside the domain
       double* pl = hp + (size_t)(ti - t0) * 3 * TS_MAX * TS_MAX;
       for (int dir = 0; dir < 3; dir++) {

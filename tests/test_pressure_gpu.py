@@ -281,3 +281,26 @@ def test_vcycle_bytes_of_the_profile(gpu_ctx):
     _, vcycle = gpu_ctx.pressure_profile(2, 1, 3)
     assert sweep == 28 * 64 ** 3
     assert vcycle == cells * (4 * 28 - 4 + (16 + 8 + 0.5) + (4 + 8 + 0.5))
+
+
+@pytest.mark.parametrize("storage", [msbg_gpu.F32, msbg_gpu.F16, msbg_gpu.BF16])
+@pytest.mark.parametrize("arrays", [False, True])
+def test_blocks_smaller_than_a_tile(gpu_ctx, storage, arrays):
+    """A grid of 8^3 blocks that are all at level 0, where a tile of 16^3 cells holds eight: the
+    right-hand side and the solution come out in the block layout, from callbacks and from
+    arrays, which are in it.  Bounds of test_mgpcg_converges_to_oracle."""
+    s = msbg_gpu.PressureScene(64, 8, 1, band=1e4, seed=7)
+    if arrays:
+        flags, face, rhs = s.arrays()
+        gpu_ctx.pressure_prepare_arrays(64, 8, 1, s.block_levels, flags, face, rhs)
+    else:
+        gpu_ctx.pressure_prepare(s)
+    xo, bo, it, rr = oracle.pressure_oracle(s, tol=1e-12)
+    b = gpu_ctx.pressure_download(rhs=True)
+    assert np.abs(b - bo).max() <= 1e-6 * np.abs(bo).max()
+    info = gpu_ctx.pressure_solve(tol=1e-6, maxRefine=30, storage=storage)
+    assert info.status == 0 and info.relResidual <= 1e-6
+    x = gpu_ctx.pressure_download()
+    assert rel_err(x, xo) <= 1e-5, rel_err(x, xo)
+    x64 = gpu_ctx.pressure_download(fp64=True)
+    assert np.abs(x64 - x).max() <= 1e-6 * np.abs(x).max()

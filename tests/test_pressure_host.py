@@ -170,3 +170,30 @@ def test_galerkin_levels_of_a_three_level_grid_are_exact():
     _, nmg, _, gerr = host_check(s, x)
     assert nmg >= 5
     assert gerr.max() < 1e-6, gerr
+
+
+@pytest.mark.parametrize("res,bsx0,nl", [(32, 8, 1), (48, 8, 1), (32, 8, 2), (40, 8, 1)])
+def test_array_build_on_blocks_smaller_than_a_tile(res, bsx0, nl):
+    """On a grid of 8^3 blocks that are all at level 0 a tile of 16^3 holds eight blocks, and its
+    cells come from all of them: the arrays build the callbacks' operator and liquid cells.  (40:
+    tiles of 8^3 cells.)"""
+    s = msbg_gpu.PressureScene(res, bsx0, nl, band=1e4, seed=6)
+    assert (s.block_levels == 0).all()
+    flags, face, rhs = s.arrays()
+    x = np.random.default_rng(3).standard_normal(s.packed_size()).astype(np.float32)
+    y_cb, nm_cb, fl_cb, _ = host_check(s, x)
+    L = msbg_gpu.lib()
+    fn = L.msbg_gpu_pressure_host_check_arrays
+    fn.restype = C.c_int
+    bl = np.ascontiguousarray(s.block_levels, np.int32)
+    d = msbg_gpu.TopoDesc(res, res, res, bsx0, nl, bl.ctypes.data_as(C.POINTER(C.c_int)))
+    P = lambda a, t: a.ctypes.data_as(C.POINTER(t))
+    y = np.zeros(len(x))
+    nm = C.c_int()
+    fluid = np.zeros(32, np.int64)
+    rc = fn(C.byref(d), P(flags, C.c_uint16), P(face[0], C.c_float), P(face[1], C.c_float),
+            P(face[2], C.c_float), P(rhs, C.c_float), P(x, C.c_float), P(y, C.c_double),
+            C.byref(nm), P(fluid, C.c_int64), None)
+    assert rc == 0
+    assert nm.value == nm_cb and (fluid[:nm.value] == fl_cb).all()
+    assert np.array_equal(y, y_cb)
