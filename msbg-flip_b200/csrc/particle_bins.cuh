@@ -128,12 +128,13 @@ struct BinsOrder {
 };
 
 // From how many bytes on an order pays: of a group's box, and of the blocks in use.  G2P (B200, 126
-// MB of L2), as the particles come and ordered.  4 M in no order on 160^3 cells (98 MB) 0.43 and
-// 0.76 ms, on 192^3 (170 MB) 0.59 and 0.69, on 256^3 (403 MB) 1.46 and 0.72; in an eighth of them
-// 0.51 and 1.43; in order on 256^3, but shuffled among 262 144 neighbours, 0.68 and 0.73, among
-// 8192 0.57 and 0.57.  16 M on 512^3 with three levels in no order 2.50 and 2.03, shuffled among
-// 262 144 1.80 and 2.10.
-constexpr double BINS_BYTES = 250e6;
+// MB of L2), as the particles come and ordered.  4 M in no order on 160^3 cells (98 MB; the box
+// around 32 of them holds 0.83 of the grid) 0.43 and 0.76 ms, on 192^3 (170 MB) 0.56 and 0.70, on
+// 208^3 (216 MB) 1.04 and 0.68, on 256^3 (403 MB) 1.46 and 0.72; in an eighth of 256^3 0.51 and
+// 1.43; in order, but shuffled among 262 144 neighbours, 0.68 and 0.73, among 8192 0.57 and 0.57.
+// 16 M on 512^3 with three levels, 222 to 484 MB, 2.25 to 2.35 and 2.29 to 2.31; with 630 MB 2.50
+// and 2.03, shuffled among 262 144 1.80 and 2.10.
+constexpr double BINS_BYTES = 160e6;
 
 // Builds the order of np device particles on stream st, in scratch memory that the gather
 // reads; blockBytes: what a gather reads of a block, on average.  Without enough device memory
