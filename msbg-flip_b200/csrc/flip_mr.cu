@@ -65,16 +65,6 @@ struct MrGrid {
   const int8_t* __restrict__ kind;  // [nl][nb]: 0 empty, 1 value, 2 full
   const uint16_t* __restrict__ dist;
   const uint64_t* __restrict__ key;  // level, kinds and offset of a block
-  // packed index of voxel (x, y, z) of level lv, or -1 (outside the level's
-  // grid, or in a block of another level)
-  __device__ __forceinline__ int64_t idx(int lv, int x, int y, int z) const {
-    if (x < 0 || y < 0 || z < 0 || x >= (sx >> lv) || y >= (sy >> lv) || z >= (sz >> lv))
-      return -1;
-    const int sh = sh0 - lv, m = (1 << sh) - 1;
-    const int b = (x >> sh) + nbx * ((y >> sh) + nby * (z >> sh));
-    if (level[b] != lv) return -1;
-    return off[b] + ((x & m) + ((y & m) << sh) + ((z & m) << (2 * sh)));
-  }
 };
 
 // BLK_FINE_COARSE per block: a block of a coarser level among its 26

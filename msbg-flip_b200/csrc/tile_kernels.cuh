@@ -113,9 +113,10 @@ static __global__ void __launch_bounds__(1024) k_finalize(const double* partial,
 // ---------------------------------------------------------------------------
 constexpr int VEC_GRID = 148 * 4, VEC_BLOCK = 512;
 // Dependent launches (common.cuh) of the vector kernels and their scalar steps: where they
-// are short.  On long vectors an early start of the next kernel takes from the running one:
-// a solve of 167 M cells took 148.9 ms with them, 145.9 without (B200); one of 64^3, whose
-// kernels take 2-4 us, 1.48 against 1.78 ms.
+// are short.  On long vectors an early start of the next kernel takes from the running one.
+// Plain FP32 solves with them and without (B200, kernel by kernel; in a CUDA graph the small ones
+// take the same either way): 64^3 cells 1.09 and 1.18 ms, 192^3 4.42 and 4.52, 256^3 6.58 and 6.61,
+// 320^3 9.79 and 9.56, 512^3 41.6 and 40.8.
 inline bool vectors_dependent(int64_t n) { return n <= (8 << 20); }
 
 template <typename VA, typename VB>
